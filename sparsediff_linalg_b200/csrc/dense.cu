@@ -9,7 +9,7 @@
 // warp computes whole output columns with its lanes on the block's rows, reading
 // the block's columns contiguously from a transposed copy, and each output is
 // summed in exactly that order (__dmul_rn / __dadd_rn: no FMA, as the upstream
-// build has none). The kernel is bound by the writes of C.
+// build has none).
 #include <algorithm>
 #include <climits>
 #include <map>
@@ -29,38 +29,257 @@ int grid_cap(long long work_items, int per_block, int cap)
 
 constexpr int BC_THREADS = 256;
 
-__global__ void k_gather_vals(const int *__restrict__ pos, const double *__restrict__ Sx, long long n,
-                              double *__restrict__ vals)
-{
-    for (long long d = blockIdx.x * (long long)blockDim.x + threadIdx.x; d < n;
-         d += (long long)gridDim.x * blockDim.x)
-        vals[d] = Sx[pos[d]];
-}
-
-// BT = the source blocks transposed (each n0 x m0 row-major), so that one column of
-// a block is contiguous.
-__global__ void k_transpose_blocks(const BlkDesc *__restrict__ descs, int nblk, const double *__restrict__ B,
-                                   double *__restrict__ BT)
+// What a fill lays out before its products, in one launch (the two halves do not depend
+// on each other): the first `gather_ctas` CTAs gather S.x into compact order, the others
+// take a 32 x 32 tile each of the transposed copies BT of the source blocks (n0 x m0
+// row-major, so that one column of a block is contiguous).
+__global__ void __launch_bounds__(BC_THREADS) k_blocks_csr_inputs(
+    const int *__restrict__ pos, const double *__restrict__ Sx, long long n, double *__restrict__ vals,
+    int gather_ctas, const BlkDesc *__restrict__ descs, int tr_x, int tr_y, const double *__restrict__ B,
+    double *__restrict__ BT)
 {
     __shared__ double t[32][33];
-    const BlkDesc D = descs[blockIdx.z];
-    const int i0 = blockIdx.y * 32, r0 = blockIdx.x * 32;
+    if ((int)blockIdx.x < gather_ctas)
+    {
+        for (long long d = blockIdx.x * (long long)blockDim.x + threadIdx.x; d < n;
+             d += (long long)gather_ctas * blockDim.x)
+            vals[d] = Sx[pos[d]];
+        return;
+    }
+    const int q = blockIdx.x - gather_ctas;
+    const BlkDesc D = descs[q / (tr_x * tr_y)];
+    const int i0 = q / tr_x % tr_y * 32, r0 = q % tr_x * 32;
     if (i0 >= D.m0 || r0 >= D.n0_B) return;
     const double *src = B + D.b_off;
     double *dst = BT + D.b_off;
-    for (int y = threadIdx.y; y < 32; y += blockDim.y)
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int y = ty; y < 32; y += BC_THREADS / 32)
     {
-        const int i = i0 + y, r = r0 + threadIdx.x;
-        if (i < D.m0 && r < D.n0_B) t[y][threadIdx.x] = src[(long long)i * D.n0_B + r];
+        const int i = i0 + y, r = r0 + tx;
+        if (i < D.m0 && r < D.n0_B) t[y][tx] = src[(long long)i * D.n0_B + r];
     }
     __syncthreads();
-    for (int y = threadIdx.y; y < 32; y += blockDim.y)
+    for (int y = ty; y < 32; y += BC_THREADS / 32)
     {
-        const int r = r0 + y, i = i0 + threadIdx.x;
-        if (r < D.n0_B && i < D.m0) dst[(long long)r * D.m0 + i] = t[threadIdx.x][y];
+        const int r = r0 + y, i = i0 + tx;
+        if (r < D.n0_B && i < D.m0) dst[(long long)r * D.m0 + i] = t[tx][y];
     }
 }
 
+// ------------------------------------------------------------------ resident slabs
+// A CTA keeps a slab of its block (up to 64 rows by n0 columns, at most 128 KB,
+// transposed) in shared memory, and its warps take units of 16 output columns one after
+// the other, with no barrier between them.
+//
+// What bounds it: every output and term takes 8 bytes of the block from shared memory
+// (64 blocks of 64 x 256 times 256 x 100000 with 6 per column: 19.7 GB, 0.53 ms at 128
+// bytes a clock and SM; 0.68 ms measured without the stores), and C is written at 4.5
+// TB/s (0.73 ms without the sums). So
+// * the reads are conflict-free 16-byte ones: four lanes (p = lane & 3) share a column
+//   and read 64 bytes of it, two columns at a time use the two halves of a 128-byte
+//   line (odd columns take the halves in the other order), and a term's {value, column}
+//   record is one read for all 16 Q rows;
+// * the sums leave from registers, eight columns of four rows at a time, as whole 32-byte
+//   sectors of C: a lane's rows are those with row % 4 == p, so they share an alignment
+//   in C whatever n0_C is, and the lane's columns start up to 3 early to meet it. With
+//   the segments where they fell, rows of odd length took 1.5 times as long (5 blocks of
+//   50 x 256 times 256 x 99991 with 5 per column: 115 -> 80 us).
+// The fill above: 1.93 -> 1.07 ms against k_blocks_csr (32 x 64 tiles through shared
+// memory, the block read from L1). Through a warp-private 32 x 16 tile instead of
+// registers it took 1.15 ms, with 32 rows a pass 1.11-1.16 ms.
+// Blocks of more than RS_N0_MAX columns stay with k_blocks_csr: slabs of only 16 rows
+// spread a record's read too thin (8 blocks of 64 x 1000 with 40 per column: 711 against
+// 601 us; with slabs of 32 rows, n0 = 512 and 6 per column, 96 against 143 us).
+constexpr int RS_WARPS = 16; // warps of a CTA
+constexpr int RS_COLS = 16;  // output columns of a unit
+constexpr int RS_SHIFT = 3;  // columns a unit may start early, to meet C's 32-byte sectors
+constexpr int RS_REC = 128;  // records a warp stages at once
+constexpr int RS_SLAB_BYTES = 128 * 1024;
+constexpr int RS_N0_MAX = RS_SLAB_BYTES / (32 * 8);
+constexpr int RS_WARP_BYTES = 2 * RS_REC * 16; // two units' records
+
+// One term of NQ 16-row groups: acc[4 k + 2 h + b] is row 16 k + 8 (h ^ sw) + 4 b + p.
+template <int NQ>
+__device__ __forceinline__ void rs_term(const char *col, int sw64, double v, double (&acc)[4 * NQ])
+{
+#pragma unroll
+    for (int k = 0; k < NQ; ++k)
+    {
+        const double2 b0 = *reinterpret_cast<const double2 *>(col + 128 * k + sw64);
+        const double2 b1 = *reinterpret_cast<const double2 *>(col + 128 * k + (sw64 ^ 64));
+        acc[4 * k] = __dadd_rn(acc[4 * k], __dmul_rn(b0.x, v));
+        acc[4 * k + 1] = __dadd_rn(acc[4 * k + 1], __dmul_rn(b0.y, v));
+        acc[4 * k + 2] = __dadd_rn(acc[4 * k + 2], __dmul_rn(b1.x, v));
+        acc[4 * k + 3] = __dadd_rn(acc[4 * k + 3], __dmul_rn(b1.y, v));
+    }
+}
+
+// Starts copying the records of entries [d0, d1) (at most RS_REC) into `recs`: the
+// value in the first 8 bytes, the block column in the next 4.
+__device__ __forceinline__ void rs_stage(int4 *recs, int d0, int d1, const int *__restrict__ rows,
+                                         const double *__restrict__ vals)
+{
+    for (int d = d0 + lane_id(); d < d1; d += 32)
+    {
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(recs + (d - d0));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(vals + d) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 8), "l"(rows + d) : "memory");
+    }
+}
+
+// One unit: the columns from c0 + shift on, 16 of them, of a slab of NQ 16-row groups.
+// `off`: lane j holds the first entry of column c0 - RS_SHIFT + j. `recs` holds the
+// unit's records when `whole`; else they are staged eight columns at a time, and read
+// from rows / vals where even those exceed RS_REC.
+template <int NQ>
+__device__ __forceinline__ void rs_unit(const char *Bq, int4 *recs, bool whole, int off, int shift, int c0, int n0_C,
+                                        const int *__restrict__ rows, const double *__restrict__ vals,
+                                        double *__restrict__ C, int nr)
+{
+    constexpr int row_bytes = 16 * NQ * 8;
+    const int lane = lane_id(), p = lane & 3, cl = lane >> 2, sw64 = (cl & 1) * 64;
+    const int d0 = __shfl_sync(FULL_MASK, off, 0);
+#pragma unroll
+    for (int g = 0; g < RS_COLS / 8; ++g)
+    {
+        const int j = 8 * g + cl + RS_SHIFT + shift, c = c0 - RS_SHIFT + j;
+        const int s = __shfl_sync(FULL_MASK, off, j);
+        const int e = __shfl_sync(FULL_MASK, off, j + 1);
+        int base = d0;
+        bool staged = whole;
+        if (!whole)
+        {
+            base = __shfl_sync(FULL_MASK, off, 8 * g);
+            const int ge = __shfl_sync(FULL_MASK, off, 8 * g + 8 + RS_SHIFT);
+            staged = ge - base <= RS_REC;
+            __syncwarp();
+            if (staged)
+            {
+                rs_stage(recs, base, ge, rows, vals);
+                asm volatile("cp.async.wait_all;" ::: "memory");
+            }
+            __syncwarp();
+        }
+        double acc[4 * NQ];
+#pragma unroll
+        for (int k = 0; k < 4 * NQ; ++k) acc[k] = 0.0;
+        if (staged)
+        {
+#pragma unroll 2
+            for (int d = s; d < e; ++d)
+            {
+                const int4 r = recs[d - base];
+                rs_term<NQ>(Bq + r.z * row_bytes, sw64, __hiloint2double(r.y, r.x), acc);
+            }
+        }
+        else
+            for (int d = s; d < e; ++d) rs_term<NQ>(Bq + rows[d] * row_bytes, sw64, vals[d], acc);
+        if (c >= 0 && c < n0_C)
+        {
+            double *o = C + c + (long long)p * n0_C;
+#pragma unroll
+            for (int q = 0; q < 4 * NQ; ++q, o += 4 * (long long)n0_C)
+            {
+                // even columns hold rows 0-7 of a group first, odd columns rows 8-15
+                const double x = sw64 ? acc[q ^ 2] : acc[q];
+                if (4 * q + p < nr) __stcs(o, x);
+            }
+        }
+    }
+}
+
+// Slabs of 16 * (Q - 1) + 1 .. 16 * Q rows.
+template <int Q>
+__global__ void __launch_bounds__(RS_WARPS * 32, Q <= 2 ? 2 : 1) k_blocks_csr_slabs(
+    const BlkSlab *__restrict__ slabs, const int *__restrict__ first_slab, long long units, int slab_smem,
+    const int *__restrict__ cp_all, const int *__restrict__ rows_all,
+    const double *__restrict__ vals_all, const double *__restrict__ BT_vals, double *__restrict__ C_vals)
+{
+    extern __shared__ __align__(16) unsigned char rs_smem[];
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    double *Bs = reinterpret_cast<double *>(rs_smem);
+    int4 *recs = reinterpret_cast<int4 *>(rs_smem + slab_smem + warp * RS_WARP_BYTES);
+    // this CTA's even share of the units, contiguous: it loads few slabs
+    long long u = units * blockIdx.x / gridDim.x;
+    const long long u_end = units * (blockIdx.x + 1) / gridDim.x;
+    for (int si = first_slab[blockIdx.x]; u < u_end; ++si)
+    {
+        const BlkSlab sl = slabs[si];
+        const BlkDesc &D = sl.D;
+        constexpr int ld = 16 * Q;
+        const int n_units = (int)(min(sl.unit_end, u_end) - u);
+        const int u_first = (int)(u - sl.unit_begin);
+        const int *cp = cp_all + D.cp_off;
+        const int *rows = rows_all + D.d_off;
+        const double *vals = vals_all + D.d_off;
+        // column offsets of the warp's unit k: lane j holds the first entry of column j - RS_SHIFT
+        const auto offs = [&](int k) {
+            const int c = (u_first + k) * RS_COLS - RS_SHIFT + lane;
+            return k < n_units ? cp[max(0, min(c, D.n0_C))] : 0;
+        };
+        int off = offs(warp), off_next = offs(warp + RS_WARPS), buf = 0;
+        // the slab, transposed and padded with zero rows to whole 16-row groups
+        __syncthreads();
+        const double *src = BT_vals + D.b_off + sl.i0;
+        for (int x0 = threadIdx.x; x0 < D.n0_B * ld; x0 += 8 * RS_WARPS * 32)
+        {
+            double v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+            {
+                const int x = x0 + j * RS_WARPS * 32, r = x / ld, y = x - r * ld;
+                const int i = (y & ~7) | ((y & 1) << 2) | ((y >> 1) & 3); // rows i and i + 4 side by side
+                v[j] = r < D.n0_B && i < sl.nrow ? src[(long long)r * D.m0 + i] : 0.0;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+            {
+                const int x = x0 + j * RS_WARPS * 32;
+                if (x < D.n0_B * ld) Bs[x] = v[j];
+            }
+        }
+        __syncthreads();
+        const char *Bl = reinterpret_cast<const char *>(Bs) + (lane & 3) * 16;
+        double *Cs = C_vals + D.c_off + (long long)sl.i0 * D.n0_C;
+        // the rows of a lane (i mod 4 alike) have the same alignment in C: its columns start
+        // 0 .. RS_SHIFT early, so that every 8 columns of a row are two whole 32-byte sectors
+        const int shift = -(int)((((uintptr_t)Cs >> 3) + (unsigned long long)(lane & 3) * D.n0_C) & 3);
+        // a unit's records are copied in while the unit before it is computed, and its
+        // column offsets are read one unit earlier still
+        const auto stage = [&](int off, int4 *to) {
+            const int d0 = __shfl_sync(FULL_MASK, off, 0), d1 = __shfl_sync(FULL_MASK, off, RS_COLS + RS_SHIFT);
+            const bool whole = d1 - d0 <= RS_REC;
+            if (whole) rs_stage(to, d0, d1, rows, vals);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            return whole;
+        };
+        bool whole = stage(off, recs);
+        for (int k = warp; k < n_units; k += RS_WARPS)
+        {
+            __syncwarp(); // the other buffer's unit is done with it
+            const bool whole_next = stage(off_next, recs + (buf ^ RS_REC));
+            const int off_after = offs(k + 2 * RS_WARPS);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            rs_unit<Q>(Bl, recs + buf, whole, off, shift, (u_first + k) * RS_COLS, D.n0_C, rows, vals, Cs, sl.nrow);
+            off = off_next;
+            off_next = off_after;
+            whole = whole_next;
+            buf ^= RS_REC;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        u += n_units;
+    }
+}
+
+using SlabKernel = void (*)(const BlkSlab *, const int *, long long, int, const int *, const int *, const double *,
+                            const double *, double *);
+SlabKernel slab_kernel(int q)
+{
+    return q == 1 ? k_blocks_csr_slabs<1> : q == 2 ? k_blocks_csr_slabs<2> : q == 3 ? k_blocks_csr_slabs<3> : k_blocks_csr_slabs<4>;
+}
+
+// ------------------------------------------------------------------ wider blocks
 #ifndef SDL_BC_COLS
 #define SDL_BC_COLS 32
 #endif
@@ -214,6 +433,7 @@ std::unique_ptr<BlocksCsrPlan> blocks_csr_build(int n_src, const int *m0, const 
     // output blocks and their work tiles
     std::vector<BlkDesc> descs;
     std::vector<BlkTile> tiles;
+    std::vector<BlkSlab> slabs[SLAB_Q];
     long long b_off = 0;
     for (int k = 0; k < n_src; ++k)
     {
@@ -232,7 +452,24 @@ std::unique_ptr<BlocksCsrPlan> blocks_csr_build(int n_src, const int *m0, const 
             D.n0_B = n0[k];
             D.n0_C = n0C;
             const int blk = (int)descs.size();
-            for (int c0 = 0; c0 < n0C && m0[k] > 0; c0 += BC_COLS) tiles.push_back(BlkTile{blk, c0});
+            if (n0[k] > RS_N0_MAX)
+                for (int c0 = 0; c0 < n0C && m0[k] > 0; c0 += BC_COLS) tiles.push_back(BlkTile{blk, c0});
+            else if (n0C > 0 && m0[k] > 0)
+            {
+                // slabs of at most 64 rows and RS_SLAB_BYTES, rows shared out evenly
+                const int qmax = std::max(1, std::min(SLAB_Q, RS_SLAB_BYTES / (16 * 8 * std::max(1, n0[k]))));
+                const int ns = (m0[k] + 16 * qmax - 1) / (16 * qmax);
+                const int per = (m0[k] + ns - 1) / ns;
+                for (int i0 = 0; i0 < m0[k]; i0 += per)
+                {
+                    const int nrow = std::min(per, m0[k] - i0), q = (nrow + 15) / 16;
+                    auto &cls = P->slab_cls[q - 1];
+                    const long long u0 = cls.units;
+                    cls.units += (n0C + RS_SHIFT + RS_COLS - 1) / RS_COLS;
+                    slabs[q - 1].push_back(BlkSlab{D, i0, nrow, u0, cls.units});
+                    cls.smem = std::max(cls.smem, n0[k] * q * 16 * 8);
+                }
+            }
             descs.push_back(D);
             P->src.push_back(k);
             P->col_perm.push_back(cc.col_perm_C);
@@ -256,7 +493,34 @@ std::unique_ptr<BlocksCsrPlan> blocks_csr_build(int n_src, const int *m0, const 
         P->tr_y = std::max(P->tr_y, (descs[q].m0 + 31) / 32);
     }
     P->desc = upload(descs.data(), std::max<size_t>(1, descs.size()), s);
-    P->tiles = upload(tiles.data(), std::max<size_t>(1, tiles.size()), s);
+    P->tiles = upload(tiles.data(), tiles.size(), s);
+    for (int q = 0; q < SLAB_Q; ++q)
+        if (!slabs[q].empty())
+        {
+            auto &cls = P->slab_cls[q];
+            cls.n = (int)slabs[q].size();
+            cls.slabs = upload(slabs[q].data(), slabs[q].size(), s);
+            // a persistent grid: the CTAs that fit, but no more than give every warp a unit,
+            // or one per SM where the units are few
+            const int smem = cls.smem + RS_WARPS * RS_WARP_BYTES;
+            const auto kern = slab_kernel(q + 1);
+            SDL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          RS_SLAB_BYTES + RS_WARPS * RS_WARP_BYTES));
+            int per_sm = 1;
+            SDL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RS_WARPS * 32, smem));
+            cls.grid = (int)std::max<long long>(
+                1, std::min<long long>((long long)runtime().num_sms * std::max(1, per_sm),
+                                       std::max((cls.units + RS_WARPS - 1) / RS_WARPS,
+                                                std::min<long long>(cls.units, runtime().num_sms))));
+            std::vector<int> first((size_t)cls.grid);
+            for (int b = 0, si = 0; b < cls.grid; ++b)
+            {
+                while (slabs[q][si].unit_end <= cls.units * b / cls.grid) ++si;
+                first[b] = si;
+            }
+            cls.first = upload(first.data(), first.size(), s);
+            SDL_CUDA(cudaStreamSynchronize(s)); // `first` leaves
+        }
     SDL_CUDA(cudaStreamSynchronize(s));
     return P;
 }
@@ -264,17 +528,24 @@ std::unique_ptr<BlocksCsrPlan> blocks_csr_build(int n_src, const int *m0, const 
 void blocks_csr_fill(const BlocksCsrPlan &P, const double *B_vals, const double *S_x, double *C_vals,
                      cudaStream_t s)
 {
-    if (P.ntiles == 0) return;
-    Runtime &rt = runtime();
-    if (P.d_total > 0)
-        SDL_LAUNCH(k_gather_vals, grid_cap(P.d_total, 256, rt.num_sms * 8), 256, 0, s, P.pos.get(), S_x,
-                   P.d_total, P.vals.get());
-    // the output blocks' sources, transposed (a source feeding two outputs is
-    // transposed twice: outputs and sources are one to one here)
-    const dim3 tg(std::max(1, P.tr_x), std::max(1, P.tr_y), (unsigned)P.src.size());
-    SDL_LAUNCH(k_transpose_blocks, tg, dim3(32, 8), 0, s, P.desc.get(), (int)P.src.size(), B_vals, P.BT.get());
-    SDL_LAUNCH(k_blocks_csr, P.ntiles, BC_THREADS, 0, s, P.tiles.get(), P.desc.get(), P.cp.get(),
-               P.rows.get(), P.vals.get(), P.BT.get(), C_vals);
+    if (P.c_total == 0) return;
+    // (a source feeding two outputs would be transposed twice: they are one to one here)
+    const int gather = P.d_total > 0 ? grid_cap(P.d_total, BC_THREADS, runtime().num_sms * 8) : 0;
+    const long long tiles = (long long)P.tr_x * P.tr_y * (long long)P.src.size();
+    if (gather + tiles > INT_MAX) fail(SDL_ERR_OVERFLOW, "blocks x CSR: too many blocks");
+    SDL_LAUNCH(k_blocks_csr_inputs, (unsigned)(gather + tiles), BC_THREADS, 0, s, P.pos.get(), S_x, P.d_total,
+               P.vals.get(), gather, P.desc.get(), P.tr_x, P.tr_y, B_vals, P.BT.get());
+    for (int q = 0; q < SLAB_Q; ++q)
+    {
+        const auto &c = P.slab_cls[q];
+        if (c.n)
+            SDL_LAUNCH(slab_kernel(q + 1), c.grid, RS_WARPS * 32, c.smem + RS_WARPS * RS_WARP_BYTES, s, c.slabs.get(),
+                       c.first.get(), c.units, c.smem, P.cp.get(), P.rows.get(), P.vals.get(), P.BT.get(),
+                       C_vals);
+    }
+    if (P.ntiles)
+        SDL_LAUNCH(k_blocks_csr, P.ntiles, BC_THREADS, 0, s, P.tiles.get(), P.desc.get(), P.cp.get(),
+                   P.rows.get(), P.vals.get(), P.BT.get(), C_vals);
 }
 
 } // namespace sdl

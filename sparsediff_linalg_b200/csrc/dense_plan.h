@@ -27,6 +27,17 @@ struct BlkTile
     int blk, c0;
 };
 
+// Rows [i0, i0 + nrow) of an output block, kept in shared memory while the block's
+// units of output columns (unit_begin .. unit_end, counted over all slabs of the class)
+// are computed.
+constexpr int SLAB_Q = 4; // 16-row groups of a slab at most
+struct BlkSlab
+{
+    BlkDesc D;
+    int i0, nrow;
+    long long unit_begin, unit_end;
+};
+
 struct BlocksCsrPlan
 {
     int S_m = 0, S_n = 0, S_nnz = 0;
@@ -46,6 +57,15 @@ struct BlocksCsrPlan
     DevBuf<BlkDesc> desc;
     DevBuf<BlkTile> tiles;
     int ntiles = 0;
+    // slabs by their 16-row groups: class q holds slabs of 16 q + 1 .. 16 (q + 1) rows
+    struct SlabClass
+    {
+        DevBuf<BlkSlab> slabs;
+        DevBuf<int> first; // the slab each CTA starts in
+        int n = 0, smem = 0, grid = 0; // smem: the largest slab's bytes
+        long long units = 0;
+    };
+    SlabClass slab_cls[SLAB_Q];
 };
 
 // Builds the plan of C_k = B_k S[col_perm_k, :] for n_src source blocks of shape

@@ -1,0 +1,56 @@
+"""Kernels at the sizes where their tiling can go wrong (edges of tiles, remainders,
+smallest and largest of each dispatch class), against the CPU oracle. Every comparison
+here is bit for bit: the kernels keep upstream's order of roundings."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def bits(a):
+    return np.ascontiguousarray(a, np.float64).view(np.int64)
+
+
+def T(a, dtype=None):
+    import torch
+    return torch.as_tensor(np.ascontiguousarray(a), device="cuda", dtype=dtype)
+
+
+# ---------------------------------------------------------------- dense blocks x CSR
+# rows: one 16-row group and its edges, a full 64-row slab, several slabs; columns: the
+# limits of 64 / 48 / 32-row slabs (256, 341, 512) and one beyond them;
+# S columns: one unit of 16 and its edges; entries per column up to every row of S, so
+# that a unit's entries (and eight columns' entries) exceed the staged records
+@pytest.mark.parametrize("m0,n0,S_n,dens", [
+    (1, 1, 1, 1.0), (15, 5, 16, 0.5), (16, 7, 17, 0.9), (17, 64, 15, 0.1), (33, 256, 33, 0.03),
+    (64, 256, 100, 0.02), (64, 257, 50, 0.3), (65, 341, 40, 1.0), (48, 342, 31, 0.05), (130, 512, 20, 0.2),
+    (31, 513, 18, 0.02), (20, 1024, 19, 0.6), (70, 1025, 34, 0.1)])
+def test_blocks_csr_slab_edges_bit_exact(sdl, orc, m0, n0, S_n, dens):
+    import torch
+    from sparsediff_linalg_b200.device import BlocksCsr
+    rng = np.random.default_rng(m0 * 7919 + n0)
+    D = rng.random((n0, S_n)) < dens
+    D[n0 // 2, S_n // 2] = True
+    Sp = np.concatenate([[0], np.cumsum(D.sum(1))]).astype(np.int32)
+    Si = np.nonzero(D)[1].astype(np.int32)
+    Sx = rng.standard_normal(len(Si))
+    Sx[::5] = -0.0
+    # the block of these sizes, a smaller one (another slab class) on a subset of the
+    # rows, and the first once more
+    half = np.sort(rng.permutation(n0)[:max(1, n0 // 2)]).astype(np.int32)
+    full = np.arange(n0, dtype=np.int32)
+    blocks = [(rng.standard_normal((m0, n0)), full), (rng.standard_normal(((m0 + 1) // 2, len(half))), half),
+              (rng.standard_normal((m0, n0)), full)]
+    P = BlocksCsr([X.shape[0] for X, _ in blocks], [X.shape[1] for X, _ in blocks], [c for _, c in blocks], Sp, Si,
+                  n0, S_n)
+    Cv = torch.full((max(1, P.c_values),), float("nan"), dtype=torch.float64, device="cuda")
+    P.fill(T(np.concatenate([X.ravel() for X, _ in blocks])), T(Sx), Cv)
+    got = Cv.cpu().numpy()
+    want = orc.blocks_csr(blocks, Sp, Si, Sx, S_n)
+    at = 0
+    for src, mk, nk, perm in P.blocks:
+        cols, Cw = want[src]
+        assert np.array_equal(perm, cols) and Cw.shape == (mk, nk)
+        assert np.array_equal(bits(got[at:at + mk * nk]), bits(Cw.ravel()))
+        at += mk * nk
+    assert at == P.c_values
