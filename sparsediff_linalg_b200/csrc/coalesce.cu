@@ -1,5 +1,5 @@
 // COO coalescing (and the matrix sums built on it): the plan sorts the triplets
-// once, stably, by column and then by row, so they sit in (row, column, triplet)
+// once, stably, by (row, column), so they sit in (row, column, triplet)
 // order; the first triplet of each distinct (row, column) opens an output, which
 // gives the coalesced CSR structure and, in the same order, the triplet-to-output
 // permutation. A value refill is then a gather in output order: one thread per
@@ -12,9 +12,6 @@
 #include "sdl_internal.h"
 
 namespace sdl {
-
-void radix_sort_pairs(unsigned *keys, uint2 *vals, unsigned *keys_tmp, uint2 *vals_tmp, int n, int key_bits,
-                      cudaStream_t s);
 
 namespace {
 
@@ -71,54 +68,106 @@ __global__ void k_coal_fill(const int *__restrict__ ostart, const int *__restric
     }
 }
 
-// Structure and refill plan of a coalescing in one sort: the triplets are stably
-// radix-sorted by column, then by row, so they end up in (row, column, triplet)
-// order; the first triplet of every distinct (row, column) opens an output, in
-// CSR order; k_coal_fill refills from it.
-__global__ void k_cs_init(const int *__restrict__ rows, const int *__restrict__ cols, int n,
-                          unsigned *__restrict__ keys, uint2 *__restrict__ vals)
+// Structure and refill plan of a coalescing in one sort: the triplets stably
+// radix-sorted by (row, column); the first triplet of every distinct (row, column)
+// opens an output, in CSR order. The sorted triplets are the refill's permutation.
+constexpr int CS_TILE = 2048; // triplets of a CTA, eight consecutive ones per thread
+constexpr int CS_ITEMS = 8;
+
+// The tile's keys into shared memory (with the key before it first), and the number of
+// outputs that this thread's triplets open.
+__device__ __forceinline__ int cs_tile_heads(const unsigned long long *__restrict__ keys, int n, long long base,
+                                             unsigned long long *sk, unsigned &heads)
 {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
+    for (int k = threadIdx.x; k <= CS_TILE; k += CS_TILE / CS_ITEMS)
     {
-        keys[t] = (unsigned)cols[t];
-        vals[t] = make_uint2((unsigned)t, (unsigned)rows[t]);
+        const long long q = base - 1 + k;
+        if (q < n) sk[k] = q < 0 ? 0 : keys[q];
+    }
+    __syncthreads();
+    heads = 0;
+#pragma unroll
+    for (int j = 0; j < CS_ITEMS; ++j)
+    {
+        const int k = threadIdx.x * CS_ITEMS + j;
+        if (base + k < n && (base + k == 0 || sk[k + 1] != sk[k])) heads |= 1u << j;
+    }
+    return __popc(heads);
+}
+
+// Outputs that each tile's triplets open.
+__global__ void __launch_bounds__(CS_TILE / CS_ITEMS) k_cs_count(const unsigned long long *__restrict__ keys, int n,
+                                                                 int *__restrict__ tile_outs)
+{
+    __shared__ int part[CS_TILE / CS_ITEMS / 32];
+    const long long q0 = (long long)blockIdx.x * CS_TILE + threadIdx.x;
+    int c = 0;
+#pragma unroll
+    for (int j = 0; j < CS_ITEMS; ++j)
+    {
+        const long long q = q0 + j * (CS_TILE / CS_ITEMS);
+        c += q < n && (q == 0 || keys[q] != keys[q - 1]);
+    }
+    c = __reduce_add_sync(FULL_MASK, c);
+    if (lane_id() == 0) part[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        for (int k = 1; k < CS_TILE / CS_ITEMS / 32; ++k) c += part[k];
+        tile_outs[blockIdx.x] = c;
     }
 }
 
-// Column-sorted {column | triplet, row} -> row keys with {triplet, column}.
-__global__ void k_cs_rekey(const unsigned *__restrict__ keys1, const uint2 *__restrict__ vals1, int n,
-                           unsigned *__restrict__ keys2, uint2 *__restrict__ vals2)
+// Column and first triplet of every output, and the row offsets: the first output of a
+// row closes the rows between the previous output's row and its own (a warp shares the
+// long gaps), the last triplet the rows after it.
+__global__ void __launch_bounds__(CS_TILE / CS_ITEMS) k_cs_emit(const unsigned long long *__restrict__ keys, int n,
+                                                                int m, int col_bits,
+                                                                const int *__restrict__ tile_first,
+                                                                int *__restrict__ ostart, int *__restrict__ Ci,
+                                                                int *__restrict__ Cp)
 {
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
+    __shared__ unsigned long long sk[CS_TILE + 1];
+    __shared__ int scr[32];
+    const long long base = (long long)blockIdx.x * CS_TILE;
+    unsigned heads;
+    const int c = cs_tile_heads(keys, n, base, sk, heads);
+    int o = tile_first[blockIdx.x] + block_incl_scan_int(c, scr) - c;
+    const unsigned long long cmask = (1ull << col_bits) - 1;
+    const int lane = lane_id();
+    for (int j = 0; j < CS_ITEMS; ++j)
     {
-        const uint2 v = vals1[q];
-        keys2[q] = v.y;
-        vals2[q] = make_uint2(v.x, keys1[q]);
-    }
-}
-
-__global__ void k_cs_flags(const unsigned *__restrict__ row, const uint2 *__restrict__ vals, int n, int *__restrict__ flag)
-{
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-        flag[q] = (q == 0 || row[q] != row[q - 1] || vals[q].y != vals[q - 1].y) ? 1 : 0;
-}
-
-__global__ void k_cs_emit(const unsigned *__restrict__ row, const uint2 *__restrict__ vals, const int *__restrict__ flag,
-                          const int *__restrict__ oid, int n, int *__restrict__ perm, int *__restrict__ ostart,
-                          int *__restrict__ Ci, int *__restrict__ rowcnt)
-{
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-    {
-        perm[q] = (int)vals[q].x;
-        if (flag[q])
+        const int k = threadIdx.x * CS_ITEMS + j;
+        int lo = 0, hi = 0, val = 0; // Cp[lo .. hi] = val
+        if ((heads >> j) & 1u)
         {
-            const int o = oid[q];
-            ostart[o] = (int)q;
-            Ci[o] = (int)vals[q].y;
-            atomicAdd(&rowcnt[row[q]], 1);
+            const unsigned long long key = sk[k + 1];
+            ostart[o] = (int)(base + k);
+            Ci[o] = (int)(key & cmask);
+            const int row = (int)(key >> col_bits);
+            lo = base + k == 0 ? 0 : (int)(sk[k] >> col_bits) + 1;
+            hi = row + 1;
+            val = o++;
+        }
+        else if (base + k == n)
+        {
+            // one past the last triplet (its tile, or a tile of its own)
+            lo = (int)(sk[k] >> col_bits) + 1;
+            hi = m + 1;
+            val = o;
+            ostart[o] = n;
+        }
+        unsigned longs = __ballot_sync(FULL_MASK, hi - lo > 8);
+        if (hi - lo <= 8)
+            for (int r = lo; r < hi; ++r) Cp[r] = val;
+        for (; longs; longs &= longs - 1)
+        {
+            const int l = __ffs(longs) - 1;
+            const int a = __shfl_sync(FULL_MASK, lo, l), b = __shfl_sync(FULL_MASK, hi, l);
+            const int v = __shfl_sync(FULL_MASK, val, l);
+            for (int r = a + lane; r < b; r += 32) Cp[r] = v;
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) ostart[oid[n]] = n;
 }
 
 } // namespace
@@ -142,29 +191,27 @@ int coalesce_sorted_build(const int *rows, const int *cols, int n, int m, int nc
         while (b < 31 && ((long long)1 << b) < (long long)v) ++b;
         return b;
     };
-    DevBuf<unsigned> ka((size_t)n), kb((size_t)n);
-    DevBuf<uint2> va((size_t)n), vb((size_t)n);
-    const int g = grid_coal(n, 256);
-    SDL_LAUNCH(k_cs_init, g, 256, 0, s, rows, cols, n, ka.get(), va.get());
-    radix_sort_pairs(ka.get(), va.get(), kb.get(), vb.get(), n, bits_of(ncols), s);
-    SDL_LAUNCH(k_cs_rekey, g, 256, 0, s, ka.get(), va.get(), n, kb.get(), vb.get());
-    radix_sort_pairs(kb.get(), vb.get(), ka.get(), va.get(), n, bits_of(m), s);
-    DevBuf<int> flag((size_t)n), oid((size_t)n + 1);
-    SDL_LAUNCH(k_cs_flags, g, 256, 0, s, kb.get(), vb.get(), n, flag.get());
-    const int nout = exclusive_scan_i32_checked(flag.get(), oid.get(), n, s);
+    const int col_bits = bits_of(ncols);
+    DevBuf<unsigned long long> ka((size_t)n), kb((size_t)n);
+    DevBuf<int> pb((size_t)n);
+    if (radix_sort_coo(rows, cols, n, bits_of(m), col_bits, ka.get(), (unsigned *)perm.get(), kb.get(),
+                       (unsigned *)pb.get(), s))
+    {
+        std::swap(ka, kb);
+        std::swap(perm, pb);
+    }
+    // tiles of the n triplets and the one position after them
+    const int ntiles = (int)((long long)n / CS_TILE + 1);
+    DevBuf<int> outs((size_t)ntiles), first((size_t)ntiles + 1);
+    SDL_LAUNCH(k_cs_count, ntiles, CS_TILE / CS_ITEMS, 0, s, ka.get(), n, outs.get());
+    const int nout = exclusive_scan_i32_checked(outs.get(), first.get(), ntiles, s);
     Ci.reset((size_t)std::max(1, nout));
     ostart.reset((size_t)nout + 1);
-    DevBuf<int> rowcnt((size_t)m + 1);
-    SDL_CUDA(cudaMemsetAsync(rowcnt.get(), 0, rowcnt.bytes(), s));
-    SDL_LAUNCH(k_cs_emit, g, 256, 0, s, kb.get(), vb.get(), flag.get(), oid.get(), n, perm.get(), ostart.get(),
-               Ci.get(), rowcnt.get());
-    const int total = exclusive_scan_i32_checked(rowcnt.get(), Cp.get(), m, s);
-    if (total != nout) fail(SDL_ERR_INTERNAL, "coalesce plan: row counts disagree with the outputs");
-    SDL_CUDA(cudaStreamSynchronize(s));
+    SDL_LAUNCH(k_cs_emit, ntiles, CS_TILE / CS_ITEMS, 0, s, ka.get(), n, m, col_bits, first.get(), ostart.get(),
+               Ci.get(), Cp.get());
+    if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "coalesce plan: the sort of the triplets did not finish");
     return nout;
 }
-
-
 
 void coalesce_order_fill(const int *ostart, const int *perm, const double *x, const double *f, int nout, double *C,
                          cudaStream_t s)

@@ -39,8 +39,6 @@ namespace sdl {
 
 void segment_sort_u64(unsigned long long *d_keys, const int *d_off, int nseg, int nkeys,
                       cudaStream_t s);
-void radix_sort_pairs(unsigned *keys, uint2 *vals, unsigned *keys_tmp, uint2 *vals_tmp, int n, int key_bits,
-                      cudaStream_t s);
 
 namespace {
 
@@ -2379,7 +2377,11 @@ void build_big_lists(const ProductDesc &d, Product &P, const long long *ub, cons
         if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "product plan: a term column is missing from its row");
         int bits = 1;
         while (bits < 32 && (1LL << bits) < O) ++bits;
-        radix_sort_pairs(keys.get(), P.bpairs.get(), keys2.get(), tmp.get(), (int)T, bits, s);
+        if (radix_sort_pairs(keys.get(), P.bpairs.get(), keys2.get(), tmp.get(), (int)T, bits, s))
+        {
+            std::swap(keys, keys2);
+            std::swap(P.bpairs, tmp);
+        }
         P.bostart.reset((size_t)O + 1);
         SDL_CUDA(cudaMemcpyAsync(P.bostart.get() + O, &hti[nbig], sizeof(int), cudaMemcpyHostToDevice, s));
         SDL_LAUNCH(k_big_starts, grid_for(T, 256, rt.num_sms * 8), 256, 0, s, keys.get(), (int)T, (int)O,

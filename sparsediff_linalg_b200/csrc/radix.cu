@@ -1,17 +1,26 @@
-// Stable LSD radix sort of (32-bit key, 8-byte payload) pairs, 8 bits per pass.
-// Used once per pattern to group the terms of the rows beyond the tile budget by
-// output: stability keeps, inside every output, the input order -- upstream's
-// visiting order.
+// Stable LSD radix sort of pairs, 8 bits per pass, used once per pattern: (32-bit
+// output, 8-byte payload) pairs group the terms of the rows beyond the tile budget by
+// output; (row << bits | column, triplet) pairs order COO triplets. Stability keeps,
+// inside every key, the input order -- upstream's visiting order.
 //
-// Per pass: a 256-bin digit histogram per tile of 4096 pairs, an exclusive scan of
-// the histograms in (digit, tile) order, then a scatter in which each warp ranks its
-// 512 pairs in order (match_any over the digit; per-warp running counts in shared
-// memory), so equal digits keep their input order across warps, tiles and passes;
-// the tile is reordered by digit in shared memory before it is written out.
+// One kernel reads the keys once for the digit counts of all passes; then each pass is
+// one kernel that reads and writes every pair once. A CTA takes the next tile (a ticket,
+// so earlier tiles are always running or done), ranks its pairs by digit -- warps rank
+// their own consecutive pairs with ballots, so equal digits keep their order -- and
+// publishes its 256 digit counts; thread d then adds up digit d's counts of the tiles
+// before it (decoupled look-back: each tile's word holds its own count, or the sum of
+// all counts up to it once known). The tile is reordered by digit in shared memory, so
+// the pairs of one digit leave for consecutive positions.
+//
+// What bounds it: instruction issue (about 150 instructions per 32 pairs, a third of
+// them the ballots, at 32 warps per SM) before the 2 x 12 bytes per pair and pass through
+// HBM. 10M (64-bit, 32-bit) pairs take 93 us a pass; with a histogram kernel, a scan of
+// all tiles' digit counts and a scatter that read the keys twice more, a pass took 210 us.
+// match_any in place of the ballots: 130 us.
 #include <algorithm>
-
 #include <mutex>
-#include <unordered_set>
+#include <set>
+#include <utility>
 
 #include "sdl_device.cuh"
 #include "sdl_internal.h"
@@ -19,152 +28,295 @@
 namespace sdl {
 namespace {
 
-constexpr int RS_THREADS = 256;
+constexpr int RS_THREADS = 256; // one per digit value
 constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_PER_WARP = 512;
-constexpr int RS_TILE = RS_WARPS * RS_PER_WARP; // 4096 pairs per tile
+// Pairs of a thread, and CTAs per SM: 12 x 4 against 16 x 3, 20 x 2, 14 x 3 and 8 x 5,
+// which took 1-8 % longer.
+constexpr int RS_ITEMS = 12;
+constexpr int RS_CTAS = 4;
+constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
+constexpr int RS_MAX_PASSES = 8;
+constexpr int RS_LOOK = 4;        // tile words read at once (1: 110 us a pass, 16: 113, 4: 101)
+constexpr int RS_POLLS = 1 << 22; // look-back reads of one tile word at most
+constexpr int RS_ERR = 4;         // device error bit: a look-back wait ran out
 
-__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned *__restrict__ keys, int n, int shift,
-                                                        int ntiles, int *__restrict__ hist)
+// Where a pass reads its pairs.
+template <class K, class V>
+struct PairSource
 {
-    __shared__ int cnt[256];
-    cnt[threadIdx.x] = 0;
-    __syncthreads();
-    const long long base = (long long)blockIdx.x * RS_TILE;
-    for (int k = threadIdx.x; k < RS_TILE; k += RS_THREADS)
+    const K *keys;
+    const V *vals;
+    __device__ K key(int i) const { return keys[i]; }
+    __device__ V val(int i) const { return vals[i]; }
+};
+// COO triplets: the key is row << bits | column, the payload the triplet.
+struct CooSource
+{
+    const int *rows, *cols;
+    int bits;
+    __device__ unsigned long long key(int i) const
     {
-        const long long i = base + k;
-        if (i < n) atomicAdd(&cnt[(keys[i] >> shift) & 255u], 1);
+        return ((unsigned long long)(unsigned)rows[i] << bits) | (unsigned)cols[i];
     }
-    __syncthreads();
-    hist[(long long)threadIdx.x * ntiles + blockIdx.x] = cnt[threadIdx.x];
+    __device__ unsigned val(int i) const { return (unsigned)i; }
+};
+
+// Byte `byte` of a key.
+__device__ __forceinline__ unsigned digit(unsigned key, int byte) { return __byte_perm(key, 0, byte) & 255u; }
+__device__ __forceinline__ unsigned digit(unsigned long long key, int byte)
+{
+    return __byte_perm((unsigned)key, (unsigned)(key >> 32), byte) & 255u;
 }
 
-// Scatter of one tile: every pair's rank among the tile's pairs of its digit (warps
-// rank their 512 pairs in order with match_any; per-warp running counts in shared
-// memory), the tile reordered by digit in shared memory, then written out in that
-// order: the pairs of one digit go to consecutive positions, so the writes of
-// neighbouring threads land next to each other.
-constexpr size_t RS_SCATTER_SMEM = (size_t)RS_TILE * (sizeof(unsigned) + sizeof(uint2)) +
-                                   (size_t)(RS_WARPS + 1) * 256 * sizeof(int);
+template <class Src>
+__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(Src src, int n, int passes, unsigned *__restrict__ hist)
+{
+    __shared__ unsigned cnt[RS_MAX_PASSES * 256];
+    for (int k = threadIdx.x; k < passes * 256; k += RS_THREADS) cnt[k] = 0;
+    __syncthreads();
+    const int lane = lane_id();
+    constexpr int U = 8; // pairs per thread whose loads are in flight together
+    for (long long base = (long long)blockIdx.x * RS_THREADS * U; base < n; base += (long long)gridDim.x * RS_THREADS * U)
+    {
+        decltype(src.key(0)) key[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+        {
+            const long long i = base + j * RS_THREADS + threadIdx.x;
+            key[j] = i < n ? src.key((int)i) : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+        {
+            const unsigned act = __ballot_sync(FULL_MASK, base + j * RS_THREADS + threadIdx.x < n);
+            for (int p = 0; p < passes; ++p)
+            {
+                // neighbours often share their high digits: one add for the warp then
+                const unsigned d = digit(key[j], p);
+                const unsigned same = __ballot_sync(FULL_MASK, d == __shfl_sync(FULL_MASK, d, 0));
+                if ((same & act) == act)
+                {
+                    if (lane == 0 && act) atomicAdd(&cnt[p * 256 + d], __popc(act));
+                }
+                else if ((act >> lane) & 1u)
+                    atomicAdd(&cnt[p * 256 + d], 1u);
+            }
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < passes * 256; k += RS_THREADS)
+        if (cnt[k]) atomicAdd(&hist[k], cnt[k]);
+}
 
-__global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned *__restrict__ keys,
-                                                           const uint2 *__restrict__ vals, int n, int shift,
-                                                           int ntiles, const int *__restrict__ offs,
-                                                           unsigned *__restrict__ okeys, uint2 *__restrict__ ovals)
+// A tile's word per digit: the two highest bits say what the others count -- 0 nothing
+// yet, 1 the tile's own pairs, 2 the pairs of all tiles up to it.
+template <class W>
+struct TileWord
+{
+    static constexpr int SHIFT = 8 * sizeof(W) - 2;
+    static constexpr W MASK = (W(1) << SHIFT) - 1;
+};
+
+// The lanes whose digit is this lane's.
+__device__ __forceinline__ unsigned warp_match8(unsigned dg)
+{
+    unsigned grp = FULL_MASK;
+#pragma unroll
+    for (int b = 0; b < 8; ++b)
+    {
+        unsigned m; // the lanes whose bit b is this lane's
+        asm volatile("{\n\t.reg .pred p;\n\tand.b32 %0, %1, %2;\n\tsetp.ne.u32 p, %0, 0;\n\t"
+                     "vote.sync.ballot.b32 %0, p, 0xffffffff;\n\t@!p not.b32 %0, %0;\n\t}"
+                     : "=r"(m)
+                     : "r"(dg), "r"(1u << b));
+        grp &= m;
+    }
+    return grp;
+}
+
+template <class K, class V>
+constexpr size_t rs_smem_bytes()
+{
+    return (size_t)RS_TILE * (sizeof(K) + sizeof(V)) + (RS_WARPS + 1) * 256 * sizeof(int);
+}
+
+template <class K, class V, class W, class Src>
+__global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(Src src, int n, int byte,
+                                                                  const unsigned *__restrict__ hist, W *words,
+                                                                  int *__restrict__ ticket, K *__restrict__ okeys,
+                                                                  V *__restrict__ ovals, int *__restrict__ err)
 {
     extern __shared__ __align__(16) unsigned char rs_smem[];
-    uint2 *sv = reinterpret_cast<uint2 *>(rs_smem);
-    unsigned *sk = reinterpret_cast<unsigned *>(sv + RS_TILE);
-    int(*wc)[256] = reinterpret_cast<int(*)[256]>(sk + RS_TILE);
-    int *tstart = &wc[RS_WARPS][0];
-    const int lane = lane_id(), w = threadIdx.x >> 5;
+    K *sk = reinterpret_cast<K *>(rs_smem);
+    V *sv = reinterpret_cast<V *>(sk + RS_TILE);
+    int(*wc)[256] = reinterpret_cast<int(*)[256]>(sv + RS_TILE);
+    int *gbase = &wc[RS_WARPS][0];
+    __shared__ int tile_sh, scr[32];
+    const int lane = lane_id(), w = threadIdx.x >> 5, d = threadIdx.x;
+    if (threadIdx.x == 0) tile_sh = atomicAdd(ticket, 1);
     for (int k = threadIdx.x; k < RS_WARPS * 256; k += RS_THREADS) (&wc[0][0])[k] = 0;
-    __syncthreads();
-    const long long tbase = (long long)blockIdx.x * RS_TILE;
-    const int tn = (int)min((long long)RS_TILE, (long long)n - tbase); // pairs of this tile
-    const long long wbase = tbase + (long long)w * RS_PER_WARP;
-    // counts per warp and digit
-    for (int r = 0; r < RS_PER_WARP; r += 32)
+    const int count = (int)hist[d];
+    const int dstart = block_incl_scan_int(count, scr) - count; // pairs of smaller digits
+    const int tile = tile_sh;
+    const long long tbase = (long long)tile * RS_TILE;
+    const int tn = (int)min((long long)RS_TILE, (long long)n - tbase);
+    // the warp's pairs, 32 consecutive ones at a time; places past the last pair count as
+    // the largest key, so they rank behind every pair of the tile
+    const int first = w * 32 * RS_ITEMS + lane; // in the tile
+    K key[RS_ITEMS];
+    V val[RS_ITEMS];
+#pragma unroll
+    for (int j = 0; j < RS_ITEMS; ++j) key[j] = first + 32 * j < tn ? src.key((int)tbase + first + 32 * j) : ~K(0);
+#pragma unroll
+    for (int j = 0; j < RS_ITEMS; ++j) val[j] = first + 32 * j < tn ? src.val((int)tbase + first + 32 * j) : V{};
+    // rank inside the warp: the pairs of the digit counted so far, and those of earlier lanes
+    int rank[RS_ITEMS];
+#pragma unroll
+    for (int j = 0; j < RS_ITEMS; ++j)
     {
-        const long long i = wbase + r + lane;
-        if (i < n) atomicAdd(&wc[w][(keys[i] >> shift) & 255u], 1);
-    }
-    __syncthreads();
-    // tile-local first position of every (warp, digit): digits in order, warps in
-    // order inside a digit
-    {
-        const int d = threadIdx.x; // RS_THREADS == 256 digits
-        int c = 0;
-        for (int ww = 0; ww < RS_WARPS; ++ww) c += wc[ww][d];
-        // exclusive scan of the digit totals over the block
-        __shared__ int scr[32];
-        const int incl = block_incl_scan_int(c, scr);
-        int run = incl - c;
-        tstart[d] = run;
-        for (int ww = 0; ww < RS_WARPS; ++ww)
-        {
-            const int cw = wc[ww][d];
-            wc[ww][d] = run;
-            run += cw;
-        }
-    }
-    __syncthreads();
-    // ranks in input order, into shared memory in digit order
-    for (int r = 0; r < RS_PER_WARP; r += 32)
-    {
-        const long long i = wbase + r + lane;
-        const bool valid = i < n;
-        const unsigned key = valid ? keys[i] : 0u;
-        const int d = valid ? (int)((key >> shift) & 255u) : 256 + lane; // invalid lanes: unique groups
-        const unsigned grp = __match_any_sync(FULL_MASK, d);
-        int pos = 0;
-        if (valid) pos = wc[w][d] + __popc(grp & lanemask_lt());
+        const unsigned dg = digit(key[j], byte);
+        int *c = &wc[w][dg];
+        const unsigned grp = warp_match8(dg);
+        rank[j] = *c + __popc(grp & lanemask_lt());
         __syncwarp();
-        if (valid)
-        {
-            sk[pos] = key;
-            sv[pos] = vals[i];
-            if (lane == 31 - __clz(grp)) wc[w][d] += __popc(grp);
-        }
+        if (lane == 31 - __clz(grp)) *c = rank[j] + 1;
         __syncwarp();
     }
     __syncthreads();
-    // out in digit order: pair j of the reordered tile goes to its digit's global
-    // start plus its place inside the digit's run
+    // digit d: the warps' counts become offsets inside the tile's run of d
+    int total = 0;
+#pragma unroll
+    for (int ww = 0; ww < RS_WARPS; ++ww)
+    {
+        const int c = wc[ww][d];
+        wc[ww][d] = total;
+        total += c;
+    }
+    if (d == 255) total -= RS_TILE - tn;
+    volatile W *word = words + (size_t)tile * 256 + d;
+    *word = (W(tile ? 1 : 2) << TileWord<W>::SHIFT) | W(total);
+    const int lstart = block_incl_scan_int(total, scr) - total; // (ends with a barrier)
+#pragma unroll
+    for (int ww = 0; ww < RS_WARPS; ++ww) wc[ww][d] += lstart;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < RS_ITEMS; ++j)
+    {
+        const int pos = wc[w][digit(key[j], byte)] + rank[j];
+        sk[pos] = key[j];
+        sv[pos] = val[j];
+    }
+    // digit d's pairs in the tiles before this one, the words of RS_LOOK tiles at a time
+    W before = 0;
+    for (int t = tile - 1; t >= 0;)
+    {
+        volatile const W *tw = words + (size_t)t * 256 + d;
+        W x[RS_LOOK];
+#pragma unroll
+        for (int j = 0; j < RS_LOOK; ++j) x[j] = tw[-256 * min(j, t)];
+        bool done = false;
+#pragma unroll
+        for (int j = 0; j < RS_LOOK; ++j)
+        {
+            if (done || j > t) continue;
+            for (int it = 0; !(x[j] >> TileWord<W>::SHIFT) && it < RS_POLLS; ++it)
+            {
+                if (it > 64) __nanosleep(32);
+                x[j] = tw[-256 * j];
+            }
+            if (!(x[j] >> TileWord<W>::SHIFT)) atomicOr(err, RS_ERR);
+            before += x[j] & TileWord<W>::MASK;
+            done = x[j] >> TileWord<W>::SHIFT != 1; // all tiles counted (or the wait ran out)
+        }
+        if (done) break;
+        t -= RS_LOOK;
+    }
+    if (tile) *word = (W(2) << TileWord<W>::SHIFT) | (before + W(total));
+    gbase[d] = dstart + (int)before - lstart;
+    __syncthreads();
     for (int j = threadIdx.x; j < tn; j += RS_THREADS)
     {
-        const unsigned key = sk[j];
-        const int d = (int)((key >> shift) & 255u);
-        const long long pos = (long long)offs[(long long)d * ntiles + blockIdx.x] + (j - tstart[d]);
-        okeys[pos] = key;
-        ovals[pos] = sv[j];
+        const K k = sk[j];
+        const unsigned pos = (unsigned)(gbase[digit(k, byte)] + j);
+        if (pos < (unsigned)n) // (always, unless a look-back wait ran out)
+        {
+            okeys[pos] = k;
+            ovals[pos] = sv[j];
+        }
     }
 }
 
-} // namespace
-
-void radix_sort_pairs(unsigned *keys, uint2 *vals, unsigned *keys_tmp, uint2 *vals_tmp, int n, int key_bits,
-                      cudaStream_t s)
+template <class K, class V, class W, class Src>
+void rs_pass(const Src &src, int n, int byte, const unsigned *hist, W *words, int *ticket, K *okeys, V *ovals,
+             int ntiles, cudaStream_t s)
 {
-    if (n <= 1) return;
+    const auto kern = k_rs_pass<K, V, W, Src>;
     {
-        // the kernel attribute is per device: set it once for each device the
-        // process sorts on (plans may be built from several host threads)
+        // the kernel attribute is per device: set it once for each device the process
+        // sorts on (plans may be built from several host threads)
         static std::mutex mu;
-        static std::unordered_set<int> done;
+        static std::set<int> done;
         int dev = 0;
         SDL_CUDA(cudaGetDevice(&dev));
         std::lock_guard<std::mutex> lk(mu);
-        if (!done.count(dev))
-        {
-            SDL_CUDA(cudaFuncSetAttribute(k_rs_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)RS_SCATTER_SMEM));
-            done.insert(dev);
-        }
+        if (done.insert(dev).second)
+            SDL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)rs_smem_bytes<K, V>()));
     }
+    SDL_CUDA(cudaMemsetAsync(words, 0, (size_t)ntiles * 256 * sizeof(W), s));
+    SDL_LAUNCH(kern, ntiles, RS_THREADS, (rs_smem_bytes<K, V>()), s, src, n, byte, hist, words, ticket, okeys, ovals,
+               runtime().d_error);
+}
+
+// Sorts the n pairs of `first` by the low `bits` bits of the key: pass 0 writes them to
+// (kb, vb), the next to (ka, va), and so on. True if they end in (kb, vb).
+template <class K, class V, class W, class Src>
+bool rs_sort(const Src &first, K *ka, V *va, K *kb, V *vb, int n, int bits, cudaStream_t s)
+{
     const int ntiles = (int)(((long long)n + RS_TILE - 1) / RS_TILE);
-    if ((long long)ntiles * 256 > INT_MAX) fail(SDL_ERR_OVERFLOW, "radix sort: too many tiles");
-    DevBuf<int> hist((size_t)ntiles * 256), offs((size_t)ntiles * 256 + 1);
-    unsigned *ka = keys, *kb = keys_tmp;
-    uint2 *va = vals, *vb = vals_tmp;
-    const int passes = (key_bits + 7) / 8;
-    for (int p = 0; p < passes; ++p)
+    const int passes = std::max(1, (bits + 7) / 8);
+    DevBuf<unsigned> hist(RS_MAX_PASSES * 256 + RS_MAX_PASSES); // the digit counts, then the passes' tickets
+    SDL_CUDA(cudaMemsetAsync(hist.get(), 0, hist.bytes(), s));
+    DevBuf<W> words((size_t)ntiles * 256);
+    const int grid = std::min(ntiles, runtime().num_sms * 8);
+    SDL_LAUNCH(k_rs_hist<Src>, grid, RS_THREADS, 0, s, first, n, passes, hist.get());
+    bool in_b = false;
+    for (int p = 0; p < passes; ++p, in_b = !in_b)
     {
-        const int shift = 8 * p;
-        SDL_LAUNCH(k_rs_hist, ntiles, RS_THREADS, 0, s, ka, n, shift, ntiles, hist.get());
-        exclusive_scan_i32_checked(hist.get(), offs.get(), ntiles * 256, s);
-        SDL_LAUNCH(k_rs_scatter, ntiles, RS_THREADS, RS_SCATTER_SMEM, s, ka, va, n, shift, ntiles, offs.get(), kb,
-                   vb);
-        std::swap(ka, kb);
-        std::swap(va, vb);
+        int *ticket = reinterpret_cast<int *>(hist.get() + RS_MAX_PASSES * 256) + p;
+        K *ok = in_b ? ka : kb;
+        V *ov = in_b ? va : vb;
+        if (p == 0)
+            rs_pass<K, V, W>(first, n, 0, hist.get(), words.get(), ticket, ok, ov, ntiles, s);
+        else
+            rs_pass<K, V, W>(PairSource<K, V>{in_b ? kb : ka, in_b ? vb : va}, n, p, hist.get() + 256 * p,
+                             words.get(), ticket, ok, ov, ntiles, s);
     }
-    if (ka != keys)
-    {
-        SDL_CUDA(cudaMemcpyAsync(keys, ka, (size_t)n * sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
-        SDL_CUDA(cudaMemcpyAsync(vals, va, (size_t)n * sizeof(uint2), cudaMemcpyDeviceToDevice, s));
-    }
-    SDL_CUDA(cudaStreamSynchronize(s)); // hist / offs are freed on return
+    return in_b;
+}
+
+constexpr int RS_WORD32_MAX = 1 << 30; // pairs that a 32-bit tile word can count
+
+} // namespace
+
+bool radix_sort_pairs(unsigned *keys, uint2 *vals, unsigned *keys_tmp, uint2 *vals_tmp, int n, int key_bits,
+                      cudaStream_t s)
+{
+    if (n <= 0) return false;
+    const PairSource<unsigned, uint2> src{keys, vals};
+    return n < RS_WORD32_MAX ? rs_sort<unsigned, uint2, unsigned>(src, keys, vals, keys_tmp, vals_tmp, n, key_bits, s)
+                             : rs_sort<unsigned, uint2, unsigned long long>(src, keys, vals, keys_tmp, vals_tmp, n,
+                                                                            key_bits, s);
+}
+
+bool radix_sort_coo(const int *rows, const int *cols, int n, int row_bits, int col_bits, unsigned long long *ka,
+                    unsigned *va, unsigned long long *kb, unsigned *vb, cudaStream_t s)
+{
+    const CooSource src{rows, cols, col_bits};
+    const int bits = row_bits + col_bits;
+    return n < RS_WORD32_MAX
+               ? rs_sort<unsigned long long, unsigned, unsigned>(src, ka, va, kb, vb, n, bits, s)
+               : rs_sort<unsigned long long, unsigned, unsigned long long>(src, ka, va, kb, vb, n, bits, s);
 }
 
 } // namespace sdl

@@ -184,6 +184,15 @@ struct CoalesceBuckets
 void coalesce_bucket_build(const int *ostart, const int *perm, int n, int nout, CoalesceBuckets &B, cudaStream_t s);
 void coalesce_bucket_fill(const CoalesceBuckets &B, const int *ostart, const double *x, const double *f, int nout,
                           double *C, cudaStream_t s);
+// Stable radix sorts (csrc/radix.cu): of (key, payload) pairs by the low key_bits bits,
+// using the second pair of buffers as scratch -- true if the result is in them; and of
+// COO triplets by (row, column), giving row << col_bits | column and the triplet, in the
+// first pair of buffers (false) or the second (true). A wait that runs out sets the
+// device error word.
+bool radix_sort_pairs(unsigned *keys, uint2 *vals, unsigned *keys_tmp, uint2 *vals_tmp, int n, int key_bits,
+                      cudaStream_t s);
+bool radix_sort_coo(const int *rows, const int *cols, int n, int row_bits, int col_bits, unsigned long long *ka,
+                    unsigned *va, unsigned long long *kb, unsigned *vb, cudaStream_t s);
 // dst[k] = src[k] (int -> long long), k < n.
 void widen_i32(const int *d_src, long long *d_dst, long long n, cudaStream_t s);
 

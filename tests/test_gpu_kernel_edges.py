@@ -54,3 +54,30 @@ def test_blocks_csr_slab_edges_bit_exact(sdl, orc, m0, n0, S_n, dens):
         assert np.array_equal(bits(got[at:at + mk * nk]), bits(Cw.ravel()))
         at += mk * nk
     assert at == P.c_values
+
+
+# ---------------------------------------------------------------- sorting triplets
+# sizes around a sort tile (3072 pairs) and a structure tile (2048); matrices whose keys
+# take one digit pass up to seven, one cell only (every key equal), rows in order, and a
+# few rows far apart (long runs of empty rows)
+@pytest.mark.parametrize("n", [1, 2, 33, 2047, 2048, 2049, 3071, 3072, 3073, 6144, 40000])
+@pytest.mark.parametrize("m,ncols,kind", [(1, 1, "random"), (9, 7, "random"), (70000, 3, "sorted"),
+                                          (5000000, 2000000000, "random"), (3000000, 50, "far")])
+def test_coalesce_sort_edges_bit_exact(sdl, orc, n, m, ncols, kind):
+    import torch
+    from sparsediff_linalg_b200.device import Coalesce
+    rng = np.random.default_rng(n + m % 1000)
+    rows = rng.integers(0, m, n)
+    if kind == "sorted":
+        rows = np.sort(rows)
+    elif kind == "far":
+        rows = rng.choice([5, 6, m // 2, m - 1], n)
+    cols = rng.integers(0, ncols, n)
+    x = rng.standard_normal(n)
+    x[::3] = -0.0
+    C = Coalesce(T(rows, torch.int32), T(cols, torch.int32), m, ncols)
+    Cx = torch.full((C.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+    C.fill(T(x), Cx)
+    wp, wi, wx = orc.coalesce(rows.astype(np.int32), cols.astype(np.int32), x, m, ncols)
+    assert np.array_equal(C.Cp.cpu().numpy(), wp) and np.array_equal(C.Ci.cpu().numpy(), wi)
+    assert np.array_equal(bits(Cx.cpu().numpy()), bits(wx))
