@@ -71,110 +71,381 @@ __global__ void k_coal_fill(const int *__restrict__ ostart, const int *__restric
 // Structure and refill plan of a coalescing in one sort: the triplets stably
 // radix-sorted by (row, column); the first triplet of every distinct (row, column)
 // opens an output, in CSR order. The sorted triplets are the refill's permutation.
-constexpr int CS_TILE = 2048; // triplets of a CTA, eight consecutive ones per thread
-constexpr int CS_ITEMS = 8;
+constexpr int CS_TILE = 2048; // triplets of a CTA
+constexpr int CS_THREADS = 256;
+constexpr int CS_ITEMS = CS_TILE / CS_THREADS;
 
-// The tile's keys into shared memory (with the key before it first), and the number of
-// outputs that this thread's triplets open.
-__device__ __forceinline__ int cs_tile_heads(const unsigned long long *__restrict__ keys, int n, long long base,
-                                             unsigned long long *sk, unsigned &heads)
+__device__ __forceinline__ bool cs_opens(const unsigned long long *__restrict__ keys, int n, long long q)
 {
-    for (int k = threadIdx.x; k <= CS_TILE; k += CS_TILE / CS_ITEMS)
-    {
-        const long long q = base - 1 + k;
-        if (q < n) sk[k] = q < 0 ? 0 : keys[q];
-    }
-    __syncthreads();
-    heads = 0;
-#pragma unroll
-    for (int j = 0; j < CS_ITEMS; ++j)
-    {
-        const int k = threadIdx.x * CS_ITEMS + j;
-        if (base + k < n && (base + k == 0 || sk[k + 1] != sk[k])) heads |= 1u << j;
-    }
-    return __popc(heads);
+    return q < n && (q == 0 || keys[q] != keys[q - 1]);
 }
 
 // Outputs that each tile's triplets open.
-__global__ void __launch_bounds__(CS_TILE / CS_ITEMS) k_cs_count(const unsigned long long *__restrict__ keys, int n,
-                                                                 int *__restrict__ tile_outs)
+__global__ void __launch_bounds__(CS_THREADS) k_cs_count(const unsigned long long *__restrict__ keys, int n,
+                                                         int *__restrict__ tile_outs)
 {
-    __shared__ int part[CS_TILE / CS_ITEMS / 32];
+    __shared__ int part[CS_THREADS / 32];
     const long long q0 = (long long)blockIdx.x * CS_TILE + threadIdx.x;
     int c = 0;
 #pragma unroll
-    for (int j = 0; j < CS_ITEMS; ++j)
-    {
-        const long long q = q0 + j * (CS_TILE / CS_ITEMS);
-        c += q < n && (q == 0 || keys[q] != keys[q - 1]);
-    }
+    for (int j = 0; j < CS_ITEMS; ++j) c += cs_opens(keys, n, q0 + j * CS_THREADS);
     c = __reduce_add_sync(FULL_MASK, c);
     if (lane_id() == 0) part[threadIdx.x >> 5] = c;
     __syncthreads();
     if (threadIdx.x == 0)
     {
-        for (int k = 1; k < CS_TILE / CS_ITEMS / 32; ++k) c += part[k];
+        for (int k = 1; k < CS_THREADS / 32; ++k) c += part[k];
         tile_outs[blockIdx.x] = c;
     }
 }
 
 // Column and first triplet of every output, and the row offsets: the first output of a
 // row closes the rows between the previous output's row and its own (a warp shares the
-// long gaps), the last triplet the rows after it.
-__global__ void __launch_bounds__(CS_TILE / CS_ITEMS) k_cs_emit(const unsigned long long *__restrict__ keys, int n,
-                                                                int m, int col_bits,
-                                                                const int *__restrict__ tile_first,
-                                                                int *__restrict__ ostart, int *__restrict__ Ci,
-                                                                int *__restrict__ Cp)
+// long gaps), one past the last triplet the rows after it. A warp takes CS_ITEMS times
+// 32 consecutive triplets, so that an output's neighbours are written beside it.
+__global__ void __launch_bounds__(CS_THREADS) k_cs_emit(const unsigned long long *__restrict__ keys, int n, int m,
+                                                        int col_bits, const int *__restrict__ tile_first,
+                                                        int *__restrict__ ostart, int *__restrict__ Ci,
+                                                        int *__restrict__ Cp)
 {
-    __shared__ unsigned long long sk[CS_TILE + 1];
-    __shared__ int scr[32];
-    const long long base = (long long)blockIdx.x * CS_TILE;
-    unsigned heads;
-    const int c = cs_tile_heads(keys, n, base, sk, heads);
-    int o = tile_first[blockIdx.x] + block_incl_scan_int(c, scr) - c;
-    const unsigned long long cmask = (1ull << col_bits) - 1;
-    const int lane = lane_id();
+    __shared__ int part[CS_THREADS / 32];
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    const long long q0 = (long long)blockIdx.x * CS_TILE + warp * (32 * CS_ITEMS) + lane;
+    unsigned long long key[CS_ITEMS], prev[CS_ITEMS];
+#pragma unroll
     for (int j = 0; j < CS_ITEMS; ++j)
     {
-        const int k = threadIdx.x * CS_ITEMS + j;
-        int lo = 0, hi = 0, val = 0; // Cp[lo .. hi] = val
-        if ((heads >> j) & 1u)
+        const long long q = q0 + 32 * j;
+        key[j] = q < n ? keys[q] : 0;
+        prev[j] = q > 0 && q <= n ? keys[q - 1] : 0;
+    }
+    unsigned heads[CS_ITEMS];
+    int c = 0;
+#pragma unroll
+    for (int j = 0; j < CS_ITEMS; ++j)
+    {
+        const long long q = q0 + 32 * j;
+        heads[j] = __ballot_sync(FULL_MASK, q < n && (q == 0 || key[j] != prev[j]));
+        c += __popc(heads[j]);
+    }
+    if (lane == 0) part[warp] = c;
+    __syncthreads();
+    int o0 = tile_first[blockIdx.x];
+    for (int k = 0; k < warp; ++k) o0 += part[k];
+    const unsigned long long cmask = (1ull << col_bits) - 1;
+#pragma unroll
+    for (int j = 0; j < CS_ITEMS; ++j)
+    {
+        const long long q = q0 + 32 * j;
+        const int o = o0 + __popc(heads[j] & lanemask_lt());
+        int lo = 0, hi = 0; // Cp[lo .. hi) = o
+        if ((heads[j] >> lane) & 1u)
         {
-            const unsigned long long key = sk[k + 1];
-            ostart[o] = (int)(base + k);
-            Ci[o] = (int)(key & cmask);
-            const int row = (int)(key >> col_bits);
-            lo = base + k == 0 ? 0 : (int)(sk[k] >> col_bits) + 1;
-            hi = row + 1;
-            val = o++;
+            ostart[o] = (int)q;
+            Ci[o] = (int)(key[j] & cmask);
+            lo = q == 0 ? 0 : (int)(prev[j] >> col_bits) + 1;
+            hi = (int)(key[j] >> col_bits) + 1;
         }
-        else if (base + k == n)
+        else if (q == n) // one past the last triplet
         {
-            // one past the last triplet (its tile, or a tile of its own)
-            lo = (int)(sk[k] >> col_bits) + 1;
-            hi = m + 1;
-            val = o;
             ostart[o] = n;
+            lo = (int)(prev[j] >> col_bits) + 1;
+            hi = m + 1;
         }
         unsigned longs = __ballot_sync(FULL_MASK, hi - lo > 8);
         if (hi - lo <= 8)
-            for (int r = lo; r < hi; ++r) Cp[r] = val;
+            for (int r = lo; r < hi; ++r) Cp[r] = o;
         for (; longs; longs &= longs - 1)
         {
             const int l = __ffs(longs) - 1;
-            const int a = __shfl_sync(FULL_MASK, lo, l), b = __shfl_sync(FULL_MASK, hi, l);
-            const int v = __shfl_sync(FULL_MASK, val, l);
-            for (int r = a + lane; r < b; r += 32) Cp[r] = v;
+            const int x = __shfl_sync(FULL_MASK, lo, l), y = __shfl_sync(FULL_MASK, hi, l);
+            const int v = __shfl_sync(FULL_MASK, o, l);
+            for (int r = x + lane; r < y; r += 32) Cp[r] = v;
+        }
+        o0 += __popc(heads[j]);
+    }
+}
+
+// ------------------------------------------------------------------ bucketed refill
+// For large inputs the one-pass refill gathers every triplet value at random from an
+// array larger than L2, so DRAM moves whole sectors for 8 useful bytes. The bucketed
+// refill takes two passes. The sorted triplets are cut, at outputs, into buckets of
+// about CB_SPAN, whose values lie together in buf, ordered by input chunk:
+//  1. a CTA per input chunk reads its values (times their factors, when given) into
+//     shared memory and writes them out bucket by bucket, so a bucket's values of one
+//     chunk leave as one run;
+//  2. a CTA per bucket reads its values into shared memory and sums every output from
+//     there, in ascending triplet order from +0.0: the one-pass refill's sums.
+// A bucket beyond CB_CAP values (an output of over a thousand triplets) keeps its
+// values in sorted order and is summed from global memory.
+// What bounds it: HBM, 8 + 6 + 8 bytes per triplet in pass 1, 8 + 2 in pass 2 and 4 + 8
+// per output (2.0 GB for 50M triplets of 35M outputs), both passes at two thirds of the
+// copy bandwidth: 580 -> 445 us there. Before, buckets of 2^20 outputs were gathered from
+// L2, at 8 useful bytes a sector: 194 us for pass 1, 377 for pass 2.
+// The sizes: long runs matter more than a second CTA per SM to overlap the phases (chunks
+// of 8192 / 12288 / 14336 / 26624: 553 / 492 / 482 / 445 us; buckets of 10752, two CTAs:
+// 471), since a run's two ends are partial sectors. Values sent to buf straight from
+// registers, one sector a lane, took 643 us for pass 1 alone.
+constexpr int CB_CAP = 22528;  // values of a bucket in shared memory, with 2 bytes of order each
+constexpr int CB_SPAN = 21504; // triplets after which the next output opens a bucket
+constexpr int CB_THREADS = 1024;
+constexpr size_t CB_SMEM = (size_t)(CB_CAP + 2) * sizeof(double) + (CB_CAP + 16) * sizeof(short);
+constexpr int CB_CHUNK = 26624; // triplets of a chunk
+constexpr int CB_CHUNK_THREADS = 1024;
+constexpr size_t CB_CHUNK_SMEM = (size_t)CB_CHUNK * sizeof(double);
+constexpr int CB_RANGES = 8192;   // input ranges (whole chunks) that a bucket keeps in order
+constexpr int CB_BINS = 8192;     // ranges of buf that a chunk is written in the order of
+constexpr size_t CB_ORDER_SMEM = (size_t)CB_CHUNK * (sizeof(int) + sizeof(short)) + CB_BINS * sizeof(int);
+
+// First output of every bucket: the one that opens at or after b * CB_SPAN.
+__global__ void k_cb_begin(const int *__restrict__ ostart, int nout, int nb, int *__restrict__ begin)
+{
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b > nb) return;
+    const long long q = (long long)b * CB_SPAN;
+    begin[b] = b == nb || q > INT_MAX ? nout : lower_bound_dev(ostart, nout, (int)q);
+}
+
+// Exclusive prefix sums of cnt[0 .. N) in place, by the whole block.
+template <int N, int THREADS>
+__device__ __forceinline__ void cb_prefix(int *cnt, int *scr)
+{
+    constexpr int PER = N / THREADS;
+    int c[PER], sum = 0;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+    {
+        c[k] = cnt[threadIdx.x * PER + k];
+        sum += c[k];
+    }
+    int run = block_incl_scan_int(sum, scr) - sum;
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+    {
+        cnt[threadIdx.x * PER + k] = run;
+        run += c[k];
+    }
+    __syncthreads();
+}
+
+// A CTA per bucket: the place of each of its triplets in buf, counted out by input range
+// in shared memory -- pos of the triplet, and of every sorted triplet its place inside
+// the bucket.
+__global__ void __launch_bounds__(CB_THREADS) k_cb_plan(const int *__restrict__ perm, const int *__restrict__ begin,
+                                                        const int *__restrict__ ostart, int range,
+                                                        int *__restrict__ pos, unsigned short *__restrict__ local)
+{
+    __shared__ int at[CB_RANGES];
+    __shared__ int scr[32];
+    const int q0 = ostart[begin[blockIdx.x]], q1 = ostart[begin[blockIdx.x + 1]];
+    if (q1 - q0 > CB_CAP)
+    {
+        for (int q = q0 + threadIdx.x; q < q1; q += CB_THREADS) pos[perm[q]] = q;
+        return;
+    }
+    for (int k = threadIdx.x; k < CB_RANGES; k += CB_THREADS) at[k] = 0;
+    __syncthreads();
+    for (int q = q0 + threadIdx.x; q < q1; q += CB_THREADS) atomicAdd(&at[perm[q] / range], 1);
+    cb_prefix<CB_RANGES, CB_THREADS>(at, scr);
+    for (int q = q0 + threadIdx.x; q < q1; q += CB_THREADS)
+    {
+        const int t = perm[q];
+        const int l = atomicAdd(&at[t / range], 1);
+        local[q] = (unsigned short)l;
+        pos[t] = q0 + l;
+    }
+}
+
+// A CTA per chunk: its triplets in the order of their places in buf (to ranges of
+// 2^shift places): which triplet of the chunk, and its place (over pos).
+__global__ void __launch_bounds__(CB_CHUNK_THREADS) k_cb_order(int *__restrict__ pos, int n, int shift,
+                                                               unsigned short *__restrict__ from)
+{
+    extern __shared__ int cb_order_smem[];
+    int *sp = cb_order_smem;
+    unsigned short *sf = reinterpret_cast<unsigned short *>(sp + CB_CHUNK);
+    int *at = reinterpret_cast<int *>(sf + CB_CHUNK);
+    __shared__ int scr[32];
+    const long long t0 = (long long)blockIdx.x * CB_CHUNK;
+    const int cnt = (int)min((long long)CB_CHUNK, n - t0);
+    constexpr int PER = CB_CHUNK / CB_CHUNK_THREADS;
+    int p[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+    {
+        const int i = threadIdx.x + j * CB_CHUNK_THREADS;
+        p[j] = i < cnt ? pos[t0 + i] : -1;
+    }
+    for (int k = threadIdx.x; k < CB_BINS; k += CB_CHUNK_THREADS) at[k] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+        if (p[j] >= 0) atomicAdd(&at[p[j] >> shift], 1);
+    cb_prefix<CB_BINS, CB_CHUNK_THREADS>(at, scr);
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+        if (p[j] >= 0)
+        {
+            const int k = atomicAdd(&at[p[j] >> shift], 1);
+            sp[k] = p[j];
+            sf[k] = (unsigned short)(threadIdx.x + j * CB_CHUNK_THREADS);
+        }
+    __syncthreads();
+    for (int i = threadIdx.x; i < cnt; i += CB_CHUNK_THREADS)
+    {
+        pos[t0 + i] = sp[i];
+        from[t0 + i] = sf[i];
+    }
+}
+
+// Pass 1: a CTA per chunk.
+__global__ void __launch_bounds__(CB_CHUNK_THREADS) k_cb_scatter(const double *__restrict__ x,
+                                                                 const double *__restrict__ f, int n,
+                                                                 const unsigned short *__restrict__ from,
+                                                                 const int *__restrict__ to, double *__restrict__ buf)
+{
+    extern __shared__ __align__(16) double cb_smem[];
+    const long long t0 = (long long)blockIdx.x * CB_CHUNK;
+    const int cnt = (int)min((long long)CB_CHUNK, n - t0);
+    if (f)
+        for (int i = threadIdx.x; i < cnt; i += CB_CHUNK_THREADS)
+            cb_smem[i] = __dmul_rn(__ldcs(f + t0 + i), __ldcs(x + t0 + i));
+    else
+    {
+        // 16 bytes at a time where the values are aligned to them
+        const int w = ((uintptr_t)x & 15) == 0 ? cnt & ~1 : 0;
+        for (int i = 2 * threadIdx.x; i < w; i += 2 * CB_CHUNK_THREADS)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(cb_smem + i)),
+                         "l"(x + t0 + i)
+                         : "memory");
+        for (int i = w + threadIdx.x; i < cnt; i += CB_CHUNK_THREADS)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(cb_smem + i)),
+                         "l"(x + t0 + i)
+                         : "memory");
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    __syncthreads();
+    constexpr int U = 4;
+    for (int i0 = threadIdx.x; i0 < cnt; i0 += U * CB_CHUNK_THREADS)
+    {
+        int fr[U], p[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+        {
+            const int i = i0 + j * CB_CHUNK_THREADS;
+            if (i < cnt)
+            {
+                fr[j] = __ldcs(from + t0 + i);
+                p[j] = __ldcs(to + t0 + i);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            if (i0 + j * CB_CHUNK_THREADS < cnt) buf[p[j]] = cb_smem[fr[j]];
+    }
+}
+
+// Starts reading the 16-byte words of [first, last) into L2.
+__device__ __forceinline__ void cb_prefetch(const int *first, const int *last)
+{
+    const uintptr_t a = (uintptr_t)first & ~(uintptr_t)15, b = ((uintptr_t)last + 15) & ~(uintptr_t)15;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(b - a)) : "memory");
+}
+
+// Pass 2: a CTA per bucket, a thread per output, four outputs at a time so that their
+// loads are in flight together (the first ones beside the bucket's copy).
+__global__ void __launch_bounds__(CB_THREADS) k_cb_sum(const int *__restrict__ begin, const int *__restrict__ ostart,
+                                                       const unsigned short *__restrict__ local,
+                                                       const double *__restrict__ buf, double *__restrict__ C)
+{
+    extern __shared__ __align__(16) double cb_smem[];
+    const int o_begin = begin[blockIdx.x], o_end = begin[blockIdx.x + 1];
+    if (o_begin == o_end) return;
+    const int b0 = ostart[o_begin], b1 = ostart[o_end];
+    const bool fits = b1 - b0 <= CB_CAP;
+    const double *sv = cb_smem + (b0 & 1);
+    unsigned short *sl0 = reinterpret_cast<unsigned short *>(cb_smem + CB_CAP + 2);
+    const unsigned short *sl = sl0 + (b0 & 7) - b0; // by sorted triplet
+    if (threadIdx.x == 0) cb_prefetch(ostart + o_begin, ostart + o_end + 1);
+    if (fits)
+    {
+        // 16 bytes at a time from the even place at or before the first (buf has a spare
+        // value at its end)
+        const double *src = buf + (b0 & ~1);
+        const int pairs = (b1 - (b0 & ~1) + 1) / 2;
+        for (int k = threadIdx.x; k < pairs; k += CB_THREADS)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(cb_smem + 2 * k)),
+                         "l"(src + 2 * k)
+                         : "memory");
+        const unsigned short *lsrc = local + (b0 & ~7);
+        const int octs = (b1 - (b0 & ~7) + 7) / 8;
+        for (int k = threadIdx.x; k < octs; k += CB_THREADS)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(sl0 + 8 * k)),
+                         "l"(lsrc + 8 * k)
+                         : "memory");
+    }
+    constexpr int U = 4;
+    bool waited = false;
+    for (int o0 = o_begin + threadIdx.x; o0 < o_end || !waited; o0 += U * CB_THREADS)
+    {
+        int q0[U], q1[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+        {
+            const int o = o0 + j * CB_THREADS;
+            q0[j] = o < o_end ? __ldcs(ostart + o) : 0;
+            q1[j] = o < o_end ? __ldcs(ostart + o + 1) : 0;
+        }
+        if (!waited)
+        {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            waited = true;
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+        {
+            if (q0[j] >= q1[j]) continue;
+            double acc = __dadd_rn(0.0, fits ? sv[sl[q0[j]]] : buf[q0[j]]);
+            for (int q = q0[j] + 1; q < q1[j]; ++q) acc = __dadd_rn(acc, fits ? sv[sl[q]] : buf[q]);
+            __stcs(C + o0 + j * CB_THREADS, acc);
         }
     }
 }
 
+void bucket_build(const int *ostart, const int *perm, int n, int nout, CoalesceBuckets &B, cudaStream_t s)
+{
+    SDL_CUDA(cudaFuncSetAttribute(k_cb_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CB_SMEM));
+    SDL_CUDA(cudaFuncSetAttribute(k_cb_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CB_CHUNK_SMEM));
+    SDL_CUDA(cudaFuncSetAttribute(k_cb_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CB_ORDER_SMEM));
+    B.n = n;
+    B.nb = (int)(((long long)n + CB_SPAN - 1) / CB_SPAN);
+    B.nchunks = (int)(((long long)n + CB_CHUNK - 1) / CB_CHUNK);
+    B.begin.reset((size_t)B.nb + 1);
+    B.to.reset((size_t)n);
+    B.from.reset((size_t)n);
+    B.local.reset((size_t)n + 8);
+    B.buf.reset((size_t)n + 1);
+    const int range = CB_CHUNK * ((B.nchunks + CB_RANGES - 1) / CB_RANGES);
+    int shift = 0;
+    while ((n - 1) >> shift >= CB_BINS) ++shift;
+    SDL_LAUNCH(k_cb_begin, B.nb / 256 + 1, 256, 0, s, ostart, nout, B.nb, B.begin.get());
+    SDL_LAUNCH(k_cb_plan, B.nb, CB_THREADS, 0, s, perm, B.begin.get(), ostart, range, B.to.get(),
+               B.local.get());
+    SDL_LAUNCH(k_cb_order, B.nchunks, CB_CHUNK_THREADS, CB_ORDER_SMEM, s, B.to.get(), n, shift, B.from.get());
+}
+
 } // namespace
 
-int coalesce_sorted_build(const int *rows, const int *cols, int n, int m, int ncols, DevBuf<int> &Cp, DevBuf<int> &Ci,
-                          DevBuf<int> &perm, DevBuf<int> &ostart, cudaStream_t s)
+int coalesce_build(const int *rows, const int *cols, int n, int m, int ncols, DevBuf<int> &Cp, DevBuf<int> &Ci,
+                   DevBuf<int> &perm, DevBuf<int> &ostart, CoalesceBuckets &buckets, cudaStream_t s)
 {
+    buckets = CoalesceBuckets{};
     Cp.reset((size_t)m + 1);
     perm.reset((size_t)std::max(1, n));
     if (n == 0)
@@ -203,13 +474,15 @@ int coalesce_sorted_build(const int *rows, const int *cols, int n, int m, int nc
     // tiles of the n triplets and the one position after them
     const int ntiles = (int)((long long)n / CS_TILE + 1);
     DevBuf<int> outs((size_t)ntiles), first((size_t)ntiles + 1);
-    SDL_LAUNCH(k_cs_count, ntiles, CS_TILE / CS_ITEMS, 0, s, ka.get(), n, outs.get());
+    SDL_LAUNCH(k_cs_count, ntiles, CS_THREADS, 0, s, ka.get(), n, outs.get());
     const int nout = exclusive_scan_i32_checked(outs.get(), first.get(), ntiles, s);
+    if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "coalesce plan: the sort of the triplets did not finish");
     Ci.reset((size_t)std::max(1, nout));
     ostart.reset((size_t)nout + 1);
-    SDL_LAUNCH(k_cs_emit, ntiles, CS_TILE / CS_ITEMS, 0, s, ka.get(), n, m, col_bits, first.get(), ostart.get(),
-               Ci.get(), Cp.get());
-    if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "coalesce plan: the sort of the triplets did not finish");
+    SDL_LAUNCH(k_cs_emit, ntiles, CS_THREADS, 0, s, ka.get(), n, m, col_bits, first.get(), ostart.get(), Ci.get(),
+               Cp.get());
+    if (n >= COALESCE_BUCKET_MIN) bucket_build(ostart.get(), perm.get(), n, nout, buckets, s);
+    SDL_CUDA(cudaStreamSynchronize(s));
     return nout;
 }
 
@@ -220,214 +493,12 @@ void coalesce_order_fill(const int *ostart, const int *perm, const double *x, co
     SDL_LAUNCH(k_coal_fill, grid_coal(nout, 256), 256, 0, s, ostart, perm, x, f, nout, C);
 }
 
-// ------------------------------------------------------------------ bucketed refill
-// For large inputs the one-pass refill gathers every triplet value at random from
-// an array far larger than L2, so DRAM moves whole sectors for 8 useful bytes. The
-// bucketed refill splits it into two streaming-friendly passes:
-//  1. the values are read in input order, a chunk of CO_CHUNK triplets per CTA,
-//     and written into output-range buckets (bucket b holds the triplets of outputs
-//     [b * span, (b + 1) * span)), each chunk's triplets of one bucket as one
-//     contiguous run, after the chunk's runs of that bucket from earlier chunks --
-//     so every bucket holds its triplets in input order;
-//  2. the one-pass refill, reading from the buckets instead of the input: an
-//     output's triplets now lie in one bucket of a few MB, which stays in L2 while
-//     the outputs of that range are summed.
-// The sums are the same sums in the same order (ascending triplet per output,
-// from +0.0), so the result is bit-identical to the one-pass refill.
-namespace {
-// Outputs per bucket (a power of two; more when the buckets would exceed
-// CO_MAX_BUCKETS): the buckets being summed in pass 2 stay in L2, and a chunk's
-// run per bucket is chunk / buckets values long.
-#ifndef SDL_COALESCE_SPAN_LOG2
-#define SDL_COALESCE_SPAN_LOG2 20
-#endif
-constexpr int COALESCE_SPAN_LOG2 = SDL_COALESCE_SPAN_LOG2;
-// CTAs per SM of the gather pass over the buckets
-#ifndef SDL_COALESCE_FILL_CTAS
-#define SDL_COALESCE_FILL_CTAS 8
-#endif
-constexpr int COALESCE_FILL_CTAS = SDL_COALESCE_FILL_CTAS;
-constexpr int CO_CHUNK = 4096;
-constexpr int CO_THREADS = 256;
-constexpr int CO_MAX_BUCKETS = 512;
-
-// Output index of every triplet (inverse of the output-order permutation).
-__global__ void k_cb_owner(const int *__restrict__ ostart, const int *__restrict__ perm, int nout,
-                           int *__restrict__ owner)
+void coalesce_bucket_fill(const CoalesceBuckets &B, const int *ostart, const double *x, const double *f, double *C,
+                          cudaStream_t s)
 {
-    for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < nout; o += (long long)gridDim.x * blockDim.x)
-        for (int q = ostart[o]; q < ostart[o + 1]; ++q) owner[perm[q]] = (int)o;
-}
-
-// Per chunk: its triplets stably ordered by bucket (bitonic sort of bucket << 12 |
-// index in shared memory), the order (lperm), each bucket's first position in it
-// (cbound, nb + 1 per chunk), each bucket's count (count, bucket-major for the
-// scan over chunks) and every triplet's rank inside its bucket's run (rank).
-__global__ void __launch_bounds__(CO_THREADS) k_cb_chunks(const int *__restrict__ owner, int n, int span, int nb,
-                                                         unsigned short *__restrict__ lperm, int *__restrict__ cbound,
-                                                         int *__restrict__ count, int nchunks,
-                                                         unsigned short *__restrict__ rank)
-{
-    __shared__ unsigned key[CO_CHUNK];
-    __shared__ int bstart[CO_MAX_BUCKETS + 1];
-    const int c = blockIdx.x;
-    const long long t0 = (long long)c * CO_CHUNK;
-    const int cnt = (int)(n - t0 < CO_CHUNK ? n - t0 : CO_CHUNK);
-    for (int i = threadIdx.x; i < CO_CHUNK; i += CO_THREADS)
-        key[i] = i < cnt ? ((unsigned)(owner[t0 + i] / span) << 12) | (unsigned)i : 0xffffffffu;
-    for (int b = threadIdx.x; b <= nb; b += CO_THREADS) bstart[b] = cnt;
-    __syncthreads();
-    for (int k = 2; k <= CO_CHUNK; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1)
-        {
-            for (int i = threadIdx.x; i < CO_CHUNK; i += CO_THREADS)
-            {
-                const int l = i ^ j;
-                if (l > i)
-                {
-                    const unsigned a = key[i], b = key[l];
-                    if (((i & k) == 0) == (a > b))
-                    {
-                        key[i] = b;
-                        key[l] = a;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    // first position of every bucket present in the chunk; absent buckets take the
-    // start of the next present one (filled backwards below)
-    for (int i = threadIdx.x; i < cnt; i += CO_THREADS)
-    {
-        const int b = (int)(key[i] >> 12);
-        if (i == 0 || (int)(key[i - 1] >> 12) != b) bstart[b] = i;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        for (int b = nb - 1; b >= 0; --b) bstart[b] = min(bstart[b], bstart[b + 1]);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < cnt; i += CO_THREADS)
-    {
-        const int b = (int)(key[i] >> 12), li = (int)(key[i] & 0xfffu);
-        lperm[t0 + i] = (unsigned short)li;
-        rank[t0 + li] = (unsigned short)(i - bstart[b]);
-    }
-    for (int b = threadIdx.x; b <= nb; b += CO_THREADS)
-    {
-        cbound[(long long)c * (nb + 1) + b] = bstart[b];
-        if (b < nb) count[(long long)b * nchunks + c] = bstart[b + 1] - bstart[b];
-    }
-}
-
-// Bucket position of the triplet in every output-order slot.
-__global__ void k_cb_perm2(const int *__restrict__ perm, const int *__restrict__ owner,
-                           const unsigned short *__restrict__ rank, const long long *__restrict__ dst, int n, int span,
-                           int nchunks, int *__restrict__ perm2)
-{
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-    {
-        const int t = perm[q];
-        const int b = owner[t] / span, c = t / CO_CHUNK;
-        perm2[q] = (int)(dst[(long long)b * nchunks + c] + rank[t]);
-    }
-}
-
-// Pass 1: a CTA per chunk; the chunk's values (times their factors) are staged in
-// shared memory, then every warp writes the runs of its share of the buckets.
-__global__ void __launch_bounds__(CO_THREADS) k_cb_scatter(const double *__restrict__ x, const double *__restrict__ f,
-                                                          int n, int nb, const unsigned short *__restrict__ lperm,
-                                                          const int *__restrict__ cbound,
-                                                          const long long *__restrict__ dstc,
-                                                          double *__restrict__ buf)
-{
-    __shared__ double xs[CO_CHUNK];
-    __shared__ int bs[CO_MAX_BUCKETS + 1];
-    __shared__ long long ds[CO_MAX_BUCKETS];
-    __shared__ unsigned short lp[CO_CHUNK];
-    const int c = blockIdx.x;
-    const long long t0 = (long long)c * CO_CHUNK;
-    const int cnt = (int)(n - t0 < CO_CHUNK ? n - t0 : CO_CHUNK);
-    for (int i = threadIdx.x; i < cnt; i += CO_THREADS)
-    {
-        xs[i] = f ? __dmul_rn(__ldcs(f + t0 + i), __ldcs(x + t0 + i)) : __ldcs(x + t0 + i);
-        lp[i] = __ldcs(lperm + t0 + i);
-    }
-    for (int b = threadIdx.x; b <= nb; b += CO_THREADS) bs[b] = __ldcs(cbound + (long long)c * (nb + 1) + b);
-    for (int b = threadIdx.x; b < nb; b += CO_THREADS) ds[b] = __ldcs(dstc + (long long)c * nb + b);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int b = warp; b < nb; b += CO_THREADS / 32)
-    {
-        const int i0 = bs[b], i1 = bs[b + 1];
-        if (i0 == i1) continue;
-        double *out = buf + ds[b];
-        for (int i = i0 + lane; i < i1; i += 32) out[i - i0] = xs[lp[i]];
-    }
-}
-
-// Chunk-major copy of the bucket-major run offsets (what a chunk's CTA reads).
-__global__ void k_cb_transpose_dst(const long long *__restrict__ dst, int nb, int nchunks, long long *__restrict__ dstc)
-{
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < (long long)nb * nchunks;
-         k += (long long)gridDim.x * blockDim.x)
-    {
-        const long long b = k / nchunks, c = k - b * nchunks;
-        dstc[c * nb + b] = dst[k];
-    }
-}
-} // namespace
-
-void coalesce_bucket_build(const int *ostart, const int *perm, int n, int nout, CoalesceBuckets &B, cudaStream_t s)
-{
-    B = CoalesceBuckets{};
-    if (n < COALESCE_BUCKET_MIN || nout <= 0) return;
-    Runtime &rt = runtime();
-    int span = 1 << COALESCE_SPAN_LOG2;
-    while ((long long)(nout + span - 1) / span > CO_MAX_BUCKETS) span <<= 1;
-    const int nb = (nout + span - 1) / span;
-    const int nchunks = (int)(((long long)n + CO_CHUNK - 1) / CO_CHUNK);
-    DevBuf<int> owner((size_t)n);
-    SDL_LAUNCH(k_cb_owner, grid_coal(nout, 256), 256, 0, s, ostart, perm, nout, owner.get());
-    B.lperm.reset((size_t)n);
-    B.cbound.reset((size_t)nchunks * (nb + 1));
-    DevBuf<int> count((size_t)nb * nchunks);
-    DevBuf<long long> count64((size_t)nb * nchunks);
-    DevBuf<unsigned short> rank((size_t)n);
-    SDL_LAUNCH(k_cb_chunks, nchunks, CO_THREADS, 0, s, owner.get(), n, span, nb, B.lperm.get(), B.cbound.get(),
-               count.get(), nchunks, rank.get());
-    // run offsets: bucket-major exclusive scan of the per-chunk counts
-    widen_i32(count.get(), count64.get(), (long long)nb * nchunks, s);
-    B.dst.reset((size_t)nb * nchunks + 1);
-    const long long total = exclusive_scan_i64(count64.get(), B.dst.get(), (long long)nb * nchunks, s);
-    if (total != n) fail(SDL_ERR_INTERNAL, "coalesce buckets: runs do not cover the triplets");
-    B.perm2.reset((size_t)n);
-    SDL_LAUNCH(k_cb_perm2, grid_coal(n, 256), 256, 0, s, perm, owner.get(), rank.get(), B.dst.get(), n, span,
-               nchunks, B.perm2.get());
-    // the scatter reads every chunk's run offsets in one piece
-    DevBuf<long long> dstc((size_t)nb * nchunks);
-    SDL_LAUNCH(k_cb_transpose_dst, grid_coal((long long)nb * nchunks, 256), 256, 0, s, B.dst.get(), nb, nchunks,
-               dstc.get());
-    B.dst = std::move(dstc);
-    B.buf.reset((size_t)n);
-    B.nb = nb;
-    B.nchunks = nchunks;
-    B.n = n;
-    SDL_CUDA(cudaStreamSynchronize(s));
-    (void)rt;
-}
-
-void coalesce_bucket_fill(const CoalesceBuckets &B, const int *ostart, const double *x, const double *f, int nout,
-                          double *C, cudaStream_t s)
-{
-    SDL_LAUNCH(k_cb_scatter, B.nchunks, CO_THREADS, 0, s, x, f, B.n, B.nb, B.lperm.get(), B.cbound.get(), B.dst.get(),
+    SDL_LAUNCH(k_cb_scatter, B.nchunks, CB_CHUNK_THREADS, CB_CHUNK_SMEM, s, x, f, B.n, B.from.get(), B.to.get(),
                B.buf.get());
-    // few outputs in flight (SMs x COALESCE_FILL_CTAS x 256 threads x 4 outputs: a
-    // bucket or two), so the buckets being summed stay in L2
-    const int grid = (int)std::max<long long>(
-        1, std::min<long long>(((long long)nout + 255) / 256, (long long)runtime().num_sms * COALESCE_FILL_CTAS));
-    SDL_LAUNCH(k_coal_fill, grid, 256, 0, s, ostart, B.perm2.get(), B.buf.get(), nullptr, nout, C);
+    SDL_LAUNCH(k_cb_sum, B.nb, CB_THREADS, CB_SMEM, s, B.begin.get(), ostart, B.local.get(), B.buf.get(), C);
 }
 
 } // namespace sdl

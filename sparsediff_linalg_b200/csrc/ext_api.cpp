@@ -35,8 +35,6 @@ struct sdl_coalesce
 
 namespace sdl {
 void coalesce_fill_scaled(const sdl_coalesce *C, const double *x, const double *d, double *Cx, cudaStream_t s);
-int coalesce_sorted_build(const int *rows, const int *cols, int n, int m, int ncols, DevBuf<int> &Cp, DevBuf<int> &Ci,
-                          DevBuf<int> &perm, DevBuf<int> &ostart, cudaStream_t s);
 void coalesce_order_fill(const int *ostart, const int *perm, const double *x, const double *f, int nout, double *C,
                          cudaStream_t s);
 } // namespace sdl
@@ -342,8 +340,7 @@ extern "C" sdl_status sdl_coalesce_create(const int *rows, const int *cols, int 
         c->m = m;
         c->n = n;
         c->nnz_in = nnz_in;
-        c->nout = coalesce_sorted_build(rows, cols, nnz_in, m, n, c->Cp, c->Ci, c->perm, c->ostart, s);
-        coalesce_bucket_build(c->ostart.get(), c->perm.get(), nnz_in, c->nout, c->buckets, s);
+        c->nout = coalesce_build(rows, cols, nnz_in, m, n, c->Cp, c->Ci, c->perm, c->ostart, c->buckets, s);
         *out = c.release();
     });
 }
@@ -376,7 +373,7 @@ namespace sdl {
 void coalesce_fill_scaled(const sdl_coalesce *C, const double *x, const double *d, double *Cx, cudaStream_t s)
 {
     if (C->buckets.active())
-        coalesce_bucket_fill(C->buckets, C->ostart.get(), x, d, C->nout, Cx, s);
+        coalesce_bucket_fill(C->buckets, C->ostart.get(), x, d, Cx, s);
     else
         coalesce_order_fill(C->ostart.get(), C->perm.get(), x, d, C->nout, Cx, s);
 }

@@ -355,22 +355,6 @@ void validate_compressed(const int *d_p, const int *d_idx, int rows, int cols, i
     if (h & 4) fail(SDL_ERR_INVALID, std::string(what) + ": index out of range");
 }
 
-// ------------------------------------------------------------------ widen
-namespace {
-__global__ void k_widen(const int *__restrict__ src, long long *__restrict__ dst, long long n)
-{
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
-        dst[k] = src[k];
-}
-} // namespace
-
-void widen_i32(const int *d_src, long long *d_dst, long long n, cudaStream_t s)
-{
-    if (n <= 0) return;
-    const int grid = (int)std::min<long long>((n + 255) / 256, (long long)runtime().num_sms * 8);
-    SDL_LAUNCH(k_widen, grid, 256, 0, s, d_src, d_dst, n);
-}
-
 // ------------------------------------------------------------------ gather
 namespace {
 // out[k] = x[src[k]], four consecutive positions per thread: one 16-byte load of

@@ -81,3 +81,33 @@ def test_coalesce_sort_edges_bit_exact(sdl, orc, n, m, ncols, kind):
     wp, wi, wx = orc.coalesce(rows.astype(np.int32), cols.astype(np.int32), x, m, ncols)
     assert np.array_equal(C.Cp.cpu().numpy(), wp) and np.array_equal(C.Ci.cpu().numpy(), wi)
     assert np.array_equal(bits(Cx.cpu().numpy()), bits(wx))
+
+
+# ---------------------------------------------------------------- bucketed refill
+MIN = 10 << 20  # triplets from which a refill goes through buckets
+
+
+# the smallest input that takes it; outputs of so many triplets that they fill a bucket
+# (22528 values) exactly, exceed it by one or take most of the input; few buckets' worth
+# of single-triplet outputs; values and factors from buffers at odd offsets
+@pytest.mark.parametrize("n,heavy", [(MIN, 0), (MIN + 1, 22528), (MIN + 3, 22529), (MIN + 2, 3000000)])
+def test_coalesce_buckets_edges_bit_exact(sdl, n, heavy):
+    import torch
+    from oracle import parallel
+    from sparsediff_linalg_b200.device import Coalesce
+    rng = np.random.default_rng(n + heavy)
+    m, ncols = 5001, 4003
+    rows, cols = rng.integers(0, m, n), rng.integers(0, ncols, n)
+    at = rng.permutation(n)[:heavy]
+    rows[at], cols[at] = 1500, 7
+    rows, cols = rows.astype(np.int32), cols.astype(np.int32)
+    x = rng.standard_normal(n + 1)
+    x[::3] = -0.0
+    C = Coalesce(T(rows), T(cols), m, ncols)
+    xd = T(x)
+    for off in (0, 1):
+        Cx = torch.full((C.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+        C.fill(xd[off:off + n], Cx)
+        wp, wi, wx = parallel.coalesce(rows, cols, x[off:off + n].copy(), m, ncols)[:3]
+        assert np.array_equal(C.Cp.cpu().numpy(), wp) and np.array_equal(C.Ci.cpu().numpy(), wi)
+        assert np.array_equal(bits(Cx.cpu().numpy()), bits(wx))
