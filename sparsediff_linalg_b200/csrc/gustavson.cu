@@ -37,8 +37,6 @@
 
 namespace sdl {
 
-void segment_sort_u64(unsigned long long *d_keys, const int *d_off, int nseg, int nkeys,
-                      cudaStream_t s);
 
 namespace {
 
@@ -112,15 +110,46 @@ __global__ void k_bin_count(const unsigned char *__restrict__ cls, int n, int nb
     if (threadIdx.x < nbins && sh[threadIdx.x]) atomicAdd(&counts[threadIdx.x], sh[threadIdx.x]);
 }
 
-__global__ void k_bin_scatter(const unsigned char *__restrict__ cls, int n, int nbins,
-                              int *__restrict__ cursor, int *__restrict__ lists)
+// The items of every class (classes >= nbins are dropped), class after class as the
+// counts give them. A CTA counts its items of each class in shared memory and takes
+// their places with one add per class: with an add per item on the same few counters,
+// 40000 rows took 28 us, against 4.6 us.
+constexpr int BIN_TILE = 2048;
+__global__ void __launch_bounds__(256) k_bin_scatter(const unsigned char *__restrict__ cls, int n, int nbins,
+                                                     const int *__restrict__ counts, int *__restrict__ cursor,
+                                                     int *__restrict__ lists)
 {
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-         k += (long long)gridDim.x * blockDim.x)
+    __shared__ int cnt[16], base[16];
+    if (threadIdx.x < 16) cnt[threadIdx.x] = 0;
+    __syncthreads();
+    const long long k0 = blockIdx.x * (long long)BIN_TILE + threadIdx.x;
+    int c[BIN_TILE / 256], at[BIN_TILE / 256];
+#pragma unroll
+    for (int j = 0; j < BIN_TILE / 256; ++j)
     {
-        int c = cls[k];
-        if (c < nbins) lists[atomicAdd(&cursor[c], 1)] = (int)k;
+        const long long k = k0 + 256 * j;
+        c[j] = k < n ? cls[k] : 255;
     }
+#pragma unroll
+    for (int j = 0; j < BIN_TILE / 256; ++j)
+    {
+        // one add per warp and class
+        const unsigned grp = __match_any_sync(FULL_MASK, c[j]);
+        int b = 0;
+        if (c[j] < nbins && lane_id() == __ffs(grp) - 1) b = atomicAdd(&cnt[c[j]], __popc(grp));
+        at[j] = __shfl_sync(FULL_MASK, b, __ffs(grp) - 1) + __popc(grp & lanemask_lt());
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < nbins && cnt[threadIdx.x])
+    {
+        int before = 0;
+        for (int q = 0; q < (int)threadIdx.x; ++q) before += counts[q];
+        base[threadIdx.x] = before + atomicAdd(&cursor[threadIdx.x], cnt[threadIdx.x]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < BIN_TILE / 256; ++j)
+        if (c[j] < nbins) lists[base[c[j]] + at[j]] = (int)(k0 + 256 * j);
 }
 
 __global__ void k_sym_classify(const long long *__restrict__ ub, int m_out, int warp_max,
@@ -2044,19 +2073,15 @@ void bin_items(const unsigned char *d_cls, int n, int nbins, DevBuf<int> &lists,
 {
     Runtime &rt = runtime();
     DevBuf<int> cnt(2 * nbins);
+    lists.reset(std::max(1, n));
     SDL_CUDA(cudaMemsetAsync(cnt.get(), 0, cnt.bytes(), s));
-    int grid = grid_for(n, 256, rt.num_sms * 8);
-    SDL_LAUNCH(k_bin_count, grid, 256, 0, s, d_cls, n, nbins, cnt.get());
+    SDL_LAUNCH(k_bin_count, grid_for(n, 256, rt.num_sms * 8), 256, 0, s, d_cls, n, nbins, cnt.get());
+    SDL_LAUNCH(k_bin_scatter, std::max(1, (n + BIN_TILE - 1) / BIN_TILE), 256, 0, s, d_cls, n, nbins, cnt.get(),
+               cnt.get() + nbins, lists.get());
     SDL_CUDA(cudaMemcpyAsync(count, cnt.get(), nbins * sizeof(int), cudaMemcpyDeviceToHost, s));
     SDL_CUDA(cudaStreamSynchronize(s));
     offset[0] = 0;
     for (int c = 0; c < nbins; ++c) offset[c + 1] = offset[c] + count[c];
-    lists.reset(std::max(1, offset[nbins]));
-    if (offset[nbins] == 0) return;
-    SDL_CUDA(cudaMemcpyAsync(cnt.get() + nbins, offset, nbins * sizeof(int),
-                             cudaMemcpyHostToDevice, s));
-    SDL_LAUNCH(k_bin_scatter, grid, 256, 0, s, d_cls, n, nbins, cnt.get() + nbins, lists.get());
-    SDL_CUDA(cudaStreamSynchronize(s));
 }
 
 template <class K>

@@ -8,9 +8,10 @@
 // sorted by e; because source positions grow in row-major order, that restores
 // exactly upstream's order (ties inside one source row included).
 //
-// Segments are sorted by size class: <= 32 keys in registers by one warp, <= 1024
-// in shared memory by one warp, <= 8192 in shared memory by one CTA, larger ones by
-// a CTA merge sort through a global scratch buffer.
+// Segments of up to 64 keys (nearly all) are sorted tile by tile: a key's place is the
+// number of smaller keys in its segment, counted in shared memory. Longer segments go by
+// size class: <= 1024 in shared memory by one warp, <= 8192 in shared memory by one CTA,
+// larger ones by a CTA merge sort through a global scratch buffer.
 #include <algorithm>
 #include <vector>
 
@@ -21,12 +22,33 @@ namespace sdl {
 namespace {
 
 constexpr int SCATTER_TILE = 2048;
+constexpr int SCATTER_THREADS = 256;
+constexpr int SCATTER_ITEMS = SCATTER_TILE / SCATTER_THREADS;
 
-__global__ void k_count_idx(const int *__restrict__ idx, int nnz, int *__restrict__ cnt)
+// Entries per column, and every entry's place among its column's (in the order the adds
+// happen to take). What bounds it: the latency of the adds, so eight entries per thread
+// are in flight together. 1.5M entries: 26 us here and 41 us in the scatter, against 19 and
+// 70 us with one entry at a time and a second add per entry in the scatter.
+__global__ void __launch_bounds__(SCATTER_THREADS) k_count_idx(const int *__restrict__ idx, int nnz,
+                                                               int *__restrict__ cnt, int *__restrict__ slot)
 {
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nnz;
-         e += (long long)gridDim.x * blockDim.x)
-        atomicAdd(&cnt[idx[e]], 1);
+    const long long e0 = blockIdx.x * (long long)SCATTER_TILE + threadIdx.x;
+    int c[SCATTER_ITEMS];
+#pragma unroll
+    for (int j = 0; j < SCATTER_ITEMS; ++j)
+    {
+        const long long e = e0 + j * SCATTER_THREADS;
+        c[j] = e < nnz ? idx[e] : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < SCATTER_ITEMS; ++j)
+        if (c[j] >= 0) c[j] = atomicAdd(&cnt[c[j]], 1);
+#pragma unroll
+    for (int j = 0; j < SCATTER_ITEMS; ++j)
+    {
+        const long long e = e0 + j * SCATTER_THREADS;
+        if (e < nnz) slot[e] = c[j];
+    }
 }
 
 // Last r in [lo, hi) with p[r] <= e (p non-decreasing, p[lo] <= e < p[hi]).
@@ -43,99 +65,155 @@ __device__ __forceinline__ int row_of(const int *p, int lo, int hi, int e)
     return lo;
 }
 
-// keys[Tp[c] + slot] = (e << 32) | row for every source entry e = (row, c).
-__global__ void k_scatter_keys(const int *__restrict__ p, const int *__restrict__ idx,
-                               int rows, int nnz, const int *__restrict__ Tp,
-                               int *__restrict__ fill, unsigned long long *__restrict__ keys)
+// The same by a whole warp, 32 probes at a time.
+__device__ __forceinline__ int warp_row_of(const int *p, int lo, int hi, int e)
 {
-    __shared__ int r_lo, r_hi;
-    long long e0 = (long long)blockIdx.x * SCATTER_TILE;
-    long long e1 = min((long long)nnz, e0 + SCATTER_TILE);
-    if (e0 >= e1) return;
-    if (p && threadIdx.x == 0)
+    const int lane = lane_id();
+    while (hi - lo > 1)
     {
-        r_lo = row_of(p, 0, rows, (int)e0);
-        r_hi = row_of(p, r_lo, rows, (int)(e1 - 1)) + 1;
+        const int step = (hi - lo + 31) / 32, at = lo + step * lane; // p[lo] <= e: lane 0 holds
+        const unsigned le = __ballot_sync(FULL_MASK, at < hi && p[at] <= e);
+        const int last = 31 - __clz(le);
+        lo += step * last;
+        hi = min(hi, lo + step);
     }
-    __syncthreads();
-    for (long long e = e0 + threadIdx.x; e < e1; e += blockDim.x)
+    return lo;
+}
+
+// keys[Tp[c] + slot] = (e << 32) | row for every source entry e = (row, c).
+__global__ void __launch_bounds__(SCATTER_THREADS) k_scatter_keys(const int *__restrict__ p,
+                                                                  const int *__restrict__ idx, int rows, int nnz,
+                                                                  const int *__restrict__ Tp,
+                                                                  const int *__restrict__ slot,
+                                                                  unsigned long long *__restrict__ keys)
+{
+    __shared__ int r_first, r_last, sp[SCATTER_TILE];
+    const long long e0 = (long long)blockIdx.x * SCATTER_TILE;
+    const int cnt = (int)min((long long)SCATTER_TILE, nnz - e0);
+    int at[SCATTER_ITEMS];
+#pragma unroll
+    for (int j = 0; j < SCATTER_ITEMS; ++j)
     {
-        int r = p ? row_of(p, r_lo, r_hi, (int)e) : (int)e;
-        int c = idx[e];
-        int slot = atomicAdd(&fill[c], 1);
-        keys[Tp[c] + slot] = ((unsigned long long)e << 32) | (unsigned)r;
+        const int i = threadIdx.x + j * SCATTER_THREADS;
+        at[j] = i < cnt ? idx[e0 + i] : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < SCATTER_ITEMS; ++j)
+        if (at[j] >= 0) at[j] = Tp[at[j]] + slot[e0 + threadIdx.x + j * SCATTER_THREADS];
+    int lo = 0, n_r = 0;
+    if (p)
+    {
+        // the tile's rows; their offsets in shared memory where they fit
+        if (threadIdx.x < 64)
+        {
+            const int r = warp_row_of(p, 0, rows, (int)(threadIdx.x < 32 ? e0 : e0 + cnt - 1));
+            if (threadIdx.x == 0) r_first = r;
+            if (threadIdx.x == 32) r_last = r;
+        }
+        __syncthreads();
+        lo = r_first;
+        n_r = r_last - lo + 1;
+        if (n_r <= SCATTER_TILE)
+        {
+            for (int k = threadIdx.x; k < n_r; k += SCATTER_THREADS) sp[k] = p[lo + k];
+            __syncthreads();
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < SCATTER_ITEMS; ++j)
+    {
+        if (at[j] < 0) continue;
+        const int e = (int)e0 + threadIdx.x + j * SCATTER_THREADS;
+        const int r = !p ? e : n_r <= SCATTER_TILE ? lo + row_of(sp, 0, n_r, e) : row_of(p, lo, lo + n_r, e);
+        keys[at[j]] = ((unsigned long long)e << 32) | (unsigned)r;
     }
 }
 
-// size classes of segments
+// size classes of segments beyond SEG_SHORT keys
+constexpr int SEG_SHORT = 64;
 enum
 {
-    SEG_W32 = 0,
-    SEG_W1K,
+    SEG_W1K = 0,
     SEG_C8K,
     SEG_BIG,
     SEG_NCLS
 };
+// Keys of a CTA of k_seg_rank: few where the segments outnumber the keys, since a key's
+// search then goes through global memory, and is a chain of about 20 loads (4000 keys over
+// 1M segments: the conversion 204 -> 179 us).
+constexpr int RANK_TILE = 2048, RANK_TILE_SPARSE = 256;
+constexpr int RANK_THREADS = 256;
 
-__global__ void k_seg_classify(const int *__restrict__ off, int nseg, int *__restrict__ counts,
-                               int *__restrict__ list_pos, unsigned char *__restrict__ cls)
+// First segment that starts in each tile of `tile` keys (nseg past the last), and the
+// segments beyond SEG_SHORT keys, listed per class.
+__global__ void k_seg_tiles(const int *__restrict__ off, int nseg, int tile, int ntiles, int *__restrict__ first,
+                            int *__restrict__ counts, int *__restrict__ lists)
 {
-    __shared__ int sh[SEG_NCLS];
-    if (threadIdx.x < SEG_NCLS) sh[threadIdx.x] = 0;
-    __syncthreads();
-    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < nseg;
+    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s <= nseg;
          s += (long long)gridDim.x * blockDim.x)
     {
-        int len = off[s + 1] - off[s];
-        int c = len <= 1 ? 255 : len <= 32 ? SEG_W32 : len <= 1024 ? SEG_W1K : len <= 8192 ? SEG_C8K : SEG_BIG;
-        cls[s] = (unsigned char)c;
-        if (c != 255) atomicAdd(&sh[c], 1);
-    }
-    __syncthreads();
-    if (threadIdx.x < SEG_NCLS && sh[threadIdx.x]) atomicAdd(&counts[threadIdx.x], sh[threadIdx.x]);
-    (void)list_pos;
-}
-
-__global__ void k_seg_scatter(const unsigned char *__restrict__ cls, int nseg,
-                              int *__restrict__ cursor, int *__restrict__ lists)
-{
-    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < nseg;
-         s += (long long)gridDim.x * blockDim.x)
-    {
-        int c = cls[s];
-        if (c == 255) continue;
-        int at = atomicAdd(&cursor[c], 1);
-        lists[at] = (int)s;
-    }
-}
-
-// <= 32 keys: one warp, keys in registers, shuffle bitonic network.
-__global__ void k_segsort_w32(const int *__restrict__ list, int count, const int *__restrict__ off,
-                              unsigned long long *__restrict__ keys)
-{
-    const int lane = lane_id();
-    const int wpb = blockDim.x >> 5;
-    for (long long w = blockIdx.x * (long long)wpb + (threadIdx.x >> 5); w < count;
-         w += (long long)gridDim.x * wpb)
-    {
-        int s = list[w];
-        int b = off[s], len = off[s + 1] - b;
-        unsigned long long v = lane < len ? keys[b + lane] : ~0ull;
-#pragma unroll
-        for (int k = 2; k <= 32; k <<= 1)
+        const int o = off[s];
+        const int b0 = s ? off[s - 1] / tile + 1 : 0;
+        const int b1 = s < nseg ? o / tile : ntiles;
+        for (int b = b0; b <= b1; ++b) first[b] = (int)s;
+        if (s == nseg) break;
+        const int len = off[s + 1] - o;
+        if (len > SEG_SHORT)
         {
-#pragma unroll
-            for (int j = k >> 1; j > 0; j >>= 1)
-            {
-                unsigned long long o = __shfl_xor_sync(FULL_MASK, v, j);
-                bool lower = (lane & j) == 0;
-                bool asc = (lane & k) == 0;
-                // keep min if (lower == asc), else max
-                bool take_min = (lower == asc);
-                v = take_min ? (o < v ? o : v) : (o > v ? o : v);
-            }
+            const int c = len <= 1024 ? SEG_W1K : len <= 8192 ? SEG_C8K : SEG_BIG;
+            // a class's segments are at most nkeys / 65 together: its list starts there
+            lists[c * (long long)(off[nseg] / (SEG_SHORT + 1)) + atomicAdd(&counts[c], 1)] = (int)s;
         }
-        if (lane < len) keys[b + lane] = v;
+    }
+}
+
+// The segments that start in a tile and have at most SEG_SHORT keys: every key finds its
+// segment (a search over the tile's offsets, in shared memory where they fit) and its
+// place in it. Writes the two halves of the key there, in order. What bounds it: about
+// 120 instructions per 32 keys; 1.5M keys in segments of 9 take 33 us, where listing the
+// segments and sorting each by a warp's bitonic network took 175 us.
+template <int TILE>
+__global__ void __launch_bounds__(RANK_THREADS) k_seg_rank(const unsigned long long *__restrict__ keys,
+                                                           const int *__restrict__ off, int nkeys,
+                                                           const int *__restrict__ first, int *__restrict__ lo_out,
+                                                           int *__restrict__ hi_out)
+{
+    __shared__ unsigned long long sk[TILE + SEG_SHORT];
+    __shared__ int so[TILE + 1];
+    const int k0 = blockIdx.x * TILE;
+    const int cnt = (int)min((long long)TILE + SEG_SHORT - 1, (long long)nkeys - k0);
+    const int c0 = first[blockIdx.x], nc = first[blockIdx.x + 1] - c0;
+    if (nc == 0) return;
+    for (int k = threadIdx.x; k < cnt; k += RANK_THREADS) sk[k] = keys[k0 + k];
+    const bool fit = nc <= TILE;
+    if (fit)
+        for (int k = threadIdx.x; k <= nc; k += RANK_THREADS) so[k] = off[c0 + k];
+    __syncthreads();
+    const int *o = fit ? so : off + c0; // offsets of the tile's segments, nc + 1 of them
+    const int from = o[0] - k0, to = min(cnt, o[nc] - k0);
+    // the segments of all of a thread's keys are searched for together
+    constexpr int U = (TILE + SEG_SHORT + RANK_THREADS - 1) / RANK_THREADS;
+    int seg[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) seg[j] = 0;
+    for (int w = 1 << (31 - __clz(nc)); w; w >>= 1)
+    {
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            if (seg[j] + w < nc && o[seg[j] + w] <= k0 + from + (int)threadIdx.x + j * RANK_THREADS) seg[j] += w;
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j)
+    {
+        const int k = from + threadIdx.x + j * RANK_THREADS;
+        if (k >= to) break;
+        const int b = o[seg[j]] - k0, e = o[seg[j] + 1] - k0;
+        if (e - b > SEG_SHORT) continue;
+        const unsigned long long key = sk[k];
+        int r = b;
+        for (int i = b; i < e; ++i) r += sk[i] < key;
+        lo_out[k0 + r] = (int)(key & 0xffffffffu);
+        hi_out[k0 + r] = (int)(key >> 32);
     }
 }
 
@@ -246,57 +324,44 @@ __global__ void k_segsort_big(const int *__restrict__ list, int count, const int
     }
 }
 
-__global__ void k_unpack_keys(const unsigned long long *__restrict__ keys, int n,
-                              int *__restrict__ Ti, int *__restrict__ src)
+// The two halves of the sorted keys of the listed segments, a CTA per segment.
+__global__ void k_unpack_segs(const int *__restrict__ list, int count, const int *__restrict__ off,
+                              const unsigned long long *__restrict__ keys, int *__restrict__ lo_out,
+                              int *__restrict__ hi_out)
 {
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-         q += (long long)gridDim.x * blockDim.x)
-    {
-        unsigned long long k = keys[q];
-        src[q] = (int)(k >> 32);
-        Ti[q] = (int)(k & 0xffffffffu);
-    }
+    for (int w = blockIdx.x; w < count; w += gridDim.x)
+        for (int q = off[list[w]] + threadIdx.x; q < off[list[w] + 1]; q += blockDim.x)
+        {
+            lo_out[q] = (int)(keys[q] & 0xffffffffu);
+            hi_out[q] = (int)(keys[q] >> 32);
+        }
 }
 
-} // namespace
-
-// Sort every segment [off[s], off[s+1]) of keys ascending (keys unique per segment).
-void segment_sort_u64(unsigned long long *d_keys, const int *d_off, int nseg, int nkeys,
-                      cudaStream_t s)
+// Sorts every segment [off[s], off[s+1]) of keys ascending (keys unique per segment) and
+// writes the keys' two halves in that order; keys is scratch.
+void segment_sort(unsigned long long *d_keys, const int *d_off, int nseg, int nkeys, int *lo_out, int *hi_out,
+                  cudaStream_t s)
 {
-    if (nseg <= 0 || nkeys <= 1) return;
     Runtime &rt = runtime();
-    DevBuf<int> counts(2 * SEG_NCLS);
-    DevBuf<unsigned char> cls(nseg);
+    const bool sparse = nseg > nkeys;
+    const int tile = sparse ? RANK_TILE_SPARSE : RANK_TILE, ntiles = (nkeys - 1) / tile + 1;
+    const int stride = nkeys / (SEG_SHORT + 1);
+    DevBuf<int> first((size_t)ntiles + 1), counts(SEG_NCLS), lists((size_t)SEG_NCLS * stride + 1);
     SDL_CUDA(cudaMemsetAsync(counts.get(), 0, counts.bytes(), s));
-    int grid = (int)std::min<long long>((nseg + 255) / 256, (long long)rt.num_sms * 8);
-    SDL_LAUNCH(k_seg_classify, grid, 256, 0, s, d_off, nseg, counts.get(), nullptr, cls.get());
+    const int grid = (int)std::min<long long>(((long long)nseg + 256) / 256, (long long)rt.num_sms * 8);
+    SDL_LAUNCH(k_seg_tiles, grid, 256, 0, s, d_off, nseg, tile, ntiles, first.get(), counts.get(), lists.get());
     int h[SEG_NCLS];
     SDL_CUDA(cudaMemcpyAsync(h, counts.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+    const auto rank = sparse ? k_seg_rank<RANK_TILE_SPARSE> : k_seg_rank<RANK_TILE>;
+    SDL_LAUNCH(rank, ntiles, RANK_THREADS, 0, s, d_keys, d_off, nkeys, first.get(), lo_out, hi_out);
     SDL_CUDA(cudaStreamSynchronize(s));
-    int start[SEG_NCLS + 1];
-    start[0] = 0;
-    for (int c = 0; c < SEG_NCLS; ++c) start[c + 1] = start[c] + h[c];
-    if (start[SEG_NCLS] == 0) return;
-    DevBuf<int> lists(start[SEG_NCLS]);
-    SDL_CUDA(cudaMemcpyAsync(counts.get() + SEG_NCLS, start, SEG_NCLS * sizeof(int),
-                             cudaMemcpyHostToDevice, s));
-    SDL_LAUNCH(k_seg_scatter, grid, 256, 0, s, cls.get(), nseg, counts.get() + SEG_NCLS,
-               lists.get());
     const int cap = rt.num_sms * 16;
-    if (h[SEG_W32])
-    {
-        int g = std::min((h[SEG_W32] + 7) / 8, cap);
-        SDL_LAUNCH(k_segsort_w32, g, 256, 0, s, lists.get() + start[SEG_W32], h[SEG_W32], d_off,
-                   d_keys);
-    }
     if (h[SEG_W1K])
     {
         int g = std::min((h[SEG_W1K] + 3) / 4, cap);
         size_t sm = 4 * 1024 * sizeof(unsigned long long);
         SDL_CUDA(cudaFuncSetAttribute(k_segsort_w1k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        SDL_LAUNCH(k_segsort_w1k, g, 128, sm, s, lists.get() + start[SEG_W1K], h[SEG_W1K], d_off,
-                   d_keys);
+        SDL_LAUNCH(k_segsort_w1k, g, 128, sm, s, lists.get(), h[SEG_W1K], d_off, d_keys);
     }
     if (h[SEG_C8K] || h[SEG_BIG])
     {
@@ -306,25 +371,30 @@ void segment_sort_u64(unsigned long long *d_keys, const int *d_off, int nseg, in
         if (h[SEG_C8K])
         {
             int g = std::min(h[SEG_C8K], cap);
-            SDL_LAUNCH(k_segsort_c8k, g, 512, sm, s, lists.get() + start[SEG_C8K], h[SEG_C8K],
-                       d_off, d_keys);
+            SDL_LAUNCH(k_segsort_c8k, g, 512, sm, s, lists.get() + SEG_C8K * (size_t)stride, h[SEG_C8K], d_off,
+                       d_keys);
         }
         if (h[SEG_BIG])
         {
             DevBuf<unsigned long long> scratch(nkeys);
             int g = std::min(h[SEG_BIG], rt.num_sms);
-            SDL_LAUNCH(k_segsort_big, g, 1024, sm, s, lists.get() + start[SEG_BIG], h[SEG_BIG],
-                       d_off, d_keys, scratch.get());
+            SDL_LAUNCH(k_segsort_big, g, 1024, sm, s, lists.get() + SEG_BIG * (size_t)stride, h[SEG_BIG], d_off,
+                       d_keys, scratch.get());
             SDL_CUDA(cudaStreamSynchronize(s)); // scratch is freed on return
         }
     }
-    SDL_CUDA(cudaStreamSynchronize(s)); // lists / cls are freed on return
+    for (int c = 0; c < SEG_NCLS; ++c)
+        if (h[c])
+            SDL_LAUNCH(k_unpack_segs, std::min(h[c], cap), 256, 0, s, lists.get() + c * (size_t)stride, h[c], d_off,
+                       d_keys, lo_out, hi_out);
+    SDL_CUDA(cudaStreamSynchronize(s)); // the lists are freed on return
 }
+
+} // namespace
 
 void transpose_build(const int *d_p, const int *d_idx, int rows, int cols, int nnz,
                      TransposePlan &out, cudaStream_t s)
 {
-    Runtime &rt = runtime();
     out.rows = rows;
     out.cols = cols;
     out.nnz = nnz;
@@ -337,19 +407,15 @@ void transpose_build(const int *d_p, const int *d_idx, int rows, int cols, int n
         SDL_CUDA(cudaStreamSynchronize(s));
         return;
     }
-    DevBuf<int> cnt((size_t)cols + 1);
+    DevBuf<int> cnt((size_t)cols + 1), slot((size_t)nnz);
     SDL_CUDA(cudaMemsetAsync(cnt.get(), 0, cnt.bytes(), s));
-    int grid = (int)std::min<long long>((nnz + 255) / 256, (long long)rt.num_sms * 8);
-    SDL_LAUNCH(k_count_idx, grid, 256, 0, s, d_idx, nnz, cnt.get());
+    const int tiles = (int)(((long long)nnz + SCATTER_TILE - 1) / SCATTER_TILE);
+    SDL_LAUNCH(k_count_idx, tiles, SCATTER_THREADS, 0, s, d_idx, nnz, cnt.get(), slot.get());
     exclusive_scan_i32_checked(cnt.get(), out.Tp.get(), cols, s);
-    SDL_CUDA(cudaMemsetAsync(cnt.get(), 0, cnt.bytes(), s));
     DevBuf<unsigned long long> keys(nnz);
-    int tiles = (int)((nnz + SCATTER_TILE - 1) / SCATTER_TILE);
-    SDL_LAUNCH(k_scatter_keys, tiles, 256, 0, s, d_p, d_idx, rows, nnz, out.Tp.get(), cnt.get(),
+    SDL_LAUNCH(k_scatter_keys, tiles, SCATTER_THREADS, 0, s, d_p, d_idx, rows, nnz, out.Tp.get(), slot.get(),
                keys.get());
-    segment_sort_u64(keys.get(), out.Tp.get(), cols, nnz, s);
-    SDL_LAUNCH(k_unpack_keys, grid, 256, 0, s, keys.get(), nnz, out.Ti.get(), out.src.get());
-    SDL_CUDA(cudaStreamSynchronize(s));
+    segment_sort(keys.get(), out.Tp.get(), cols, nnz, out.Ti.get(), out.src.get(), s);
 }
 
 } // namespace sdl

@@ -111,3 +111,31 @@ def test_coalesce_buckets_edges_bit_exact(sdl, n, heavy):
         wp, wi, wx = parallel.coalesce(rows, cols, x[off:off + n].copy(), m, ncols)[:3]
         assert np.array_equal(C.Cp.cpu().numpy(), wp) and np.array_equal(C.Ci.cpu().numpy(), wi)
         assert np.array_equal(bits(Cx.cpu().numpy()), bits(wx))
+
+
+# ---------------------------------------------------------------- transpose
+# columns of every sorting class and its edges (64 keys counted in place, 1024 a warp,
+# 8192 a CTA), beside empty and short ones; entries around the 2048-entry tiles; far more
+# columns than entries, far more rows than entries, and columns repeated inside a row
+@pytest.mark.parametrize("rows,cols,lens", [
+    (1, 1, [1]), (5, 3, [0, 3, 0]), (700, 40, [64, 65, 63, 0, 1, 2] * 3), (3000, 9, [1024, 1025, 1, 8192, 8193, 64]),
+    (2047, 2047, [1] * 2047), (2048, 64, [32] * 64), (100000, 70, [64] * 32 + [1]), (50, 500000, [3] * 1000),
+    (4, 3000, [0, 2] * 1500), (20000, 6, [20001, 0, 17000, 64, 5])])
+def test_transpose_segment_edges(sdl, orc, rows, cols, lens):
+    import torch
+    from sparsediff_linalg_b200.device import Transpose
+    rng = np.random.default_rng(rows + cols)
+    at = np.sort(rng.permutation(cols)[:min(len(lens), cols)])
+    col = np.repeat(at, lens[:len(at)])
+    nnz = len(col)
+    row = rng.integers(0, rows, nnz)
+    order = np.lexsort((col, row))
+    row, col = row[order], col[order].astype(np.int32)
+    p = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=rows))]).astype(np.int32)
+    x = rng.standard_normal(nnz)
+    t = Transpose(T(p), T(col), rows, cols)
+    tx = torch.empty(max(1, nnz), dtype=torch.float64, device="cuda")[:nnz]
+    t.fill(T(x), tx)
+    wp, wi, wx = orc.transpose(p, col, x, rows, cols)
+    assert np.array_equal(t.Tp.cpu().numpy(), wp) and np.array_equal(t.Ti.cpu().numpy(), wi)
+    assert np.array_equal(bits(tx.cpu().numpy()), bits(wx))
