@@ -445,6 +445,7 @@ void bucket_build(const int *ostart, const int *perm, int n, int nout, CoalesceB
 int coalesce_build(const int *rows, const int *cols, int n, int m, int ncols, DevBuf<int> &Cp, DevBuf<int> &Ci,
                    DevBuf<int> &perm, DevBuf<int> &ostart, CoalesceBuckets &buckets, cudaStream_t s)
 {
+    const FreeScope frees;
     buckets = CoalesceBuckets{};
     Cp.reset((size_t)m + 1);
     perm.reset((size_t)std::max(1, n));

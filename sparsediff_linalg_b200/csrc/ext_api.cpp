@@ -334,8 +334,9 @@ extern "C" sdl_status sdl_coalesce_create(const int *rows, const int *cols, int 
         *out = nullptr;
         if (nnz_in < 0 || m < 0 || n < 0) fail(SDL_ERR_INVALID, "negative size");
         cudaStream_t s = pick_stream(stream);
-        validate_compressed(nullptr, rows, 0, m, nnz_in, "coalesce rows", s);
-        validate_compressed(nullptr, cols, 0, n, nnz_in, "coalesce cols", s);
+        const ValidateJob jobs[2] = {{nullptr, rows, 0, m, nnz_in, "coalesce rows"},
+                                     {nullptr, cols, 0, n, nnz_in, "coalesce cols"}};
+        validate_all(jobs, 2, s);
         auto c = std::make_unique<sdl_coalesce>();
         c->m = m;
         c->n = n;

@@ -2180,9 +2180,10 @@ void validate_product(const ProductDesc &d, const TuneConfig &cfg, Product &P, c
     P.m_out = (int)m_out_ll;
     P.n = d.A_n;
     P.n_L = d.A_m / d.blocks;
-    validate_compressed(d.Lp, d.Li, d.L_m, P.n_L, d.L_nnz, "product operand L", s);
-    validate_compressed(d.Ap, d.Ai, d.A_m, d.A_n, d.A_nnz, "product operand A", s);
-    if (d.L_map) validate_compressed(nullptr, d.L_map, 0, INT_MAX, d.L_nnz, "product L_map", s);
+    const ValidateJob jobs[3] = {{d.Lp, d.Li, d.L_m, P.n_L, d.L_nnz, "product operand L"},
+                                 {d.Ap, d.Ai, d.A_m, d.A_n, d.A_nnz, "product operand A"},
+                                 {nullptr, d.L_map, 0, INT_MAX, d.L_nnz, "product L_map"}};
+    validate_all(jobs, d.L_map ? 3 : 2, s);
 }
 
 // ------------------------------------------------------------ rows beyond the tile budget
@@ -2700,6 +2701,7 @@ __global__ void k_class_hits(const unsigned char *__restrict__ pcls, const int *
 void product_symbolic(const ProductDesc &d, const TuneConfig &cfg, Product &P, cudaStream_t s,
                       bool keep_row_terms)
 {
+    const FreeScope frees;
     NvtxRange nvtx_range_("sdl: symbolic pass");
     Runtime &rt = runtime();
     validate_product(d, cfg, P, s);
@@ -3045,6 +3047,7 @@ void product_oneshot_learned(const ProductDesc &d, const TuneConfig &cfg, const 
 
 void product_complete_plan(Product &P, cudaStream_t s)
 {
+    const FreeScope frees;
     if (P.plan_ready) return;
     if (P.m_out > 0) build_schedule(P.desc, P, P.row_terms.get(), s);
     SDL_CUDA(cudaStreamSynchronize(s));

@@ -1,12 +1,14 @@
 // Library runtime: device selection, the library stream, error words, counted
 // device allocations, and the scan / iota / validation primitives every phase
 // uses.
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
 #include <unordered_map>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "sdl_internal.h"
 #include "sdl_device.cuh"
@@ -106,6 +108,10 @@ void release_idle(DevCache &c, int dev)
 }
 } // namespace
 
+namespace {
+void free_pending();
+}
+
 void *dev_alloc(size_t bytes)
 {
     runtime();
@@ -113,7 +119,7 @@ void *dev_alloc(size_t bytes)
     int dev = 0;
     SDL_CUDA(cudaGetDevice(&dev));
     DevCache &c = dev_cache();
-    std::lock_guard<std::mutex> g(c.mu);
+    std::unique_lock<std::mutex> g(c.mu);
     g_dev_allocs.fetch_add(1, std::memory_order_relaxed);
     auto it = c.idle.lower_bound({dev, want});
     if (it != c.idle.end() && it->first.first == dev && it->first.second <= 2 * want)
@@ -130,6 +136,9 @@ void *dev_alloc(size_t bytes)
     if (e != cudaSuccess)
     {
         cudaGetLastError();
+        g.unlock();
+        free_pending(); // what this thread's build has let go of so far
+        g.lock();
         release_idle(c, dev);
         e = cudaMalloc(&p, want);
     }
@@ -149,30 +158,83 @@ void *dev_alloc(size_t bytes)
     return p;
 }
 
+// Returns blocks to the cache after one device synchronisation (or to the driver, where
+// the cache is full or the blocks belong to another device than the current one).
+static void dev_free_blocks(void *const *blocks, size_t n)
+{
+    DevCache &c = dev_cache();
+    std::lock_guard<std::mutex> g(c.mu);
+    int cur = 0;
+    cudaGetDevice(&cur);
+    const bool synced = cudaDeviceSynchronize() == cudaSuccess;
+    if (!synced) cudaGetLastError();
+    for (size_t k = 0; k < n; ++k)
+    {
+        void *p = blocks[k];
+        auto it = c.live.find(p);
+        if (it == c.live.end())
+        {
+            cudaFree(p);
+            continue;
+        }
+        const size_t bytes = it->second.first;
+        const int dev = it->second.second;
+        c.live.erase(it);
+        if (!synced || cur != dev || c.idle_bytes[dev] + bytes > c.cap[dev])
+        {
+            cudaFree(p);
+            cudaGetLastError();
+            continue;
+        }
+        c.idle.insert({{dev, bytes}, p});
+        c.idle_bytes[dev] += bytes;
+    }
+}
+
+// Blocks freed while the calling thread is inside a FreeScope wait for its end (or until
+// they reach FREE_SCOPE_BYTES), so a build synchronises the device once instead of once
+// per scratch buffer.
+namespace {
+constexpr size_t FREE_SCOPE_BYTES = (size_t)1 << 30;
+struct PendingFrees
+{
+    int depth = 0;
+    size_t bytes = 0;
+    std::vector<void *> blocks;
+};
+thread_local PendingFrees t_pending;
+
+void free_pending()
+{
+    std::vector<void *> blocks;
+    blocks.swap(t_pending.blocks);
+    t_pending.bytes = 0;
+    if (!blocks.empty()) dev_free_blocks(blocks.data(), blocks.size());
+}
+} // namespace
+
+FreeScope::FreeScope() { ++t_pending.depth; }
+FreeScope::~FreeScope()
+{
+    if (--t_pending.depth == 0) free_pending();
+}
+
 void dev_free(void *p)
 {
     if (!p) return;
-    DevCache &c = dev_cache();
-    std::lock_guard<std::mutex> g(c.mu);
-    auto it = c.live.find(p);
-    if (it == c.live.end())
+    if (t_pending.depth == 0)
     {
-        cudaFree(p);
+        dev_free_blocks(&p, 1);
         return;
     }
-    const size_t bytes = it->second.first;
-    const int dev = it->second.second;
-    c.live.erase(it);
-    int cur = 0;
-    cudaGetDevice(&cur);
-    if (cur != dev || c.idle_bytes[dev] + bytes > c.cap[dev] || cudaDeviceSynchronize() != cudaSuccess)
+    t_pending.blocks.push_back(p);
     {
-        cudaGetLastError();
-        cudaFree(p);
-        return;
+        DevCache &c = dev_cache();
+        std::lock_guard<std::mutex> g(c.mu);
+        auto it = c.live.find(p);
+        if (it != c.live.end()) t_pending.bytes += it->second.first;
     }
-    c.idle.insert({{dev, bytes}, p});
-    c.idle_bytes[dev] += bytes;
+    if (t_pending.bytes >= FREE_SCOPE_BYTES) free_pending();
 }
 
 void release_cached_device_memory()
@@ -312,47 +374,68 @@ void fill_iota(int *d, int n, cudaStream_t s)
 
 // ------------------------------------------------------------------ validation
 namespace {
-// bit 1: p[0] != 0 or p[rows] != nnz; bit 2: p decreasing; bit 4: index out of range
-__global__ void k_validate(const int *p, const int *idx, int rows, int cols, int nnz,
-                           int *flags)
+struct ValidateJobs
 {
+    ValidateJob job[VALIDATE_MAX];
+};
+
+// flags[k], job k (blockIdx.y): bit 1: p[0] != 0 or p[rows] != nnz; bit 2: p decreasing;
+// bit 4: index out of range
+__global__ void k_validate(ValidateJobs jobs, int *flags)
+{
+    const ValidateJob J = jobs.job[blockIdx.y];
     long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     int f = 0;
-    if (tid == 0 && p)
+    if (tid == 0 && J.p)
     {
-        if (p[0] != 0 || p[rows] != nnz) f |= 1;
+        if (J.p[0] != 0 || J.p[J.rows] != J.nnz) f |= 1;
     }
-    if (p)
-        for (long long r = tid; r < rows; r += stride)
-            if (p[r + 1] < p[r]) f |= 2;
-    for (long long k = tid; k < nnz; k += stride)
+    if (J.p)
+        for (long long r = tid; r < J.rows; r += stride)
+            if (J.p[r + 1] < J.p[r]) f |= 2;
+    for (long long k = tid; k < J.nnz; k += stride)
     {
-        int c = idx[k];
-        if (c < 0 || c >= cols) f |= 4;
+        int c = J.idx[k];
+        if (c < 0 || c >= J.cols) f |= 4;
     }
-    if (f) atomicOr(flags, f);
+    if (f) atomicOr(flags + blockIdx.y, f);
 }
 } // namespace
+
+void validate_all(const ValidateJob *jobs, int n, cudaStream_t s)
+{
+    ValidateJobs J{};
+    long long work = 1;
+    for (int k = 0; k < n; ++k)
+    {
+        const ValidateJob &j = jobs[k];
+        if (j.rows < 0 || j.cols < 0 || j.nnz < 0) fail(SDL_ERR_INVALID, std::string(j.what) + ": negative size");
+        if (j.nnz > 0 && !j.idx) fail(SDL_ERR_INVALID, std::string(j.what) + ": null index array");
+        work = std::max<long long>({work, j.rows, j.nnz});
+        J.job[k] = j;
+    }
+    const int grid = (int)std::min<long long>((work + 255) / 256, 148LL * 8);
+    DevBuf<int> flags(VALIDATE_MAX);
+    SDL_CUDA(cudaMemsetAsync(flags.get(), 0, flags.bytes(), s));
+    SDL_LAUNCH(k_validate, dim3(grid, n), 256, 0, s, J, flags.get());
+    int h[VALIDATE_MAX] = {};
+    SDL_CUDA(cudaMemcpyAsync(h, flags.get(), n * sizeof(int), cudaMemcpyDeviceToHost, s));
+    SDL_CUDA(cudaStreamSynchronize(s));
+    for (int k = 0; k < n; ++k)
+    {
+        const std::string what(jobs[k].what);
+        if (h[k] & 1) fail(SDL_ERR_INVALID, what + ": offsets must start at 0 and end at nnz");
+        if (h[k] & 2) fail(SDL_ERR_INVALID, what + ": offsets must be non-decreasing");
+        if (h[k] & 4) fail(SDL_ERR_INVALID, what + ": index out of range");
+    }
+}
 
 void validate_compressed(const int *d_p, const int *d_idx, int rows, int cols, int nnz,
                          const char *what, cudaStream_t s)
 {
-    if (rows < 0 || cols < 0 || nnz < 0) fail(SDL_ERR_INVALID, std::string(what) + ": negative size");
-    if (nnz > 0 && !d_idx) fail(SDL_ERR_INVALID, std::string(what) + ": null index array");
-    Runtime &rt = runtime();
-    long long work = std::max<long long>(rows, nnz);
-    int grid = (int)std::max<long long>(1, std::min<long long>((work + 255) / 256, 148LL * 8));
-    DevBuf<int> flags(1);
-    SDL_CUDA(cudaMemsetAsync(flags.get(), 0, sizeof(int), s));
-    SDL_LAUNCH(k_validate, grid, 256, 0, s, d_p, d_idx, rows, cols, nnz, flags.get());
-    int h = 0;
-    SDL_CUDA(cudaMemcpyAsync(&h, flags.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
-    SDL_CUDA(cudaStreamSynchronize(s));
-    (void)rt;
-    if (h & 1) fail(SDL_ERR_INVALID, std::string(what) + ": offsets must start at 0 and end at nnz");
-    if (h & 2) fail(SDL_ERR_INVALID, std::string(what) + ": offsets must be non-decreasing");
-    if (h & 4) fail(SDL_ERR_INVALID, std::string(what) + ": index out of range");
+    const ValidateJob j{d_p, d_idx, rows, cols, nnz, what};
+    validate_all(&j, 1, s);
 }
 
 // ------------------------------------------------------------------ gather

@@ -84,7 +84,16 @@ int take_device_error(cudaStream_t s);
 
 // ---------------------------------------------------------------- memory
 void *dev_alloc(size_t bytes); // from the block cache or cudaMalloc, counted; throws on failure
-void dev_free(void *p);         // into the block cache (after a device synchronisation) or cudaFree
+void dev_free(void *p);
+// While one exists, the device blocks that this thread frees are held back and freed
+// together when the outermost one ends, after one device synchronisation.
+struct FreeScope
+{
+    FreeScope();
+    ~FreeScope();
+    FreeScope(const FreeScope &) = delete;
+    FreeScope &operator=(const FreeScope &) = delete;
+};         // into the block cache (after a device synchronisation) or cudaFree
 void release_cached_device_memory(); // frees the current device's cached blocks
 extern std::atomic<unsigned long long> g_dev_allocs;
 
@@ -146,6 +155,15 @@ void fill_iota(int *d, int n, cudaStream_t s);
 // SDL_ERR_INVALID otherwise.
 void validate_compressed(const int *d_p, const int *d_idx, int rows, int cols, int nnz,
                          const char *what, cudaStream_t s);
+// The same for up to VALIDATE_MAX structures, in one launch and one wait.
+constexpr int VALIDATE_MAX = 3;
+struct ValidateJob
+{
+    const int *p, *idx;
+    int rows, cols, nnz;
+    const char *what;
+};
+void validate_all(const ValidateJob *jobs, int n, cudaStream_t s);
 
 // ---------------------------------------------------------------- transpose
 // Stable transpose of a compressed structure (rows x cols, nnz entries): Tp has

@@ -395,6 +395,7 @@ void segment_sort(unsigned long long *d_keys, const int *d_off, int nseg, int nk
 void transpose_build(const int *d_p, const int *d_idx, int rows, int cols, int nnz,
                      TransposePlan &out, cudaStream_t s)
 {
+    const FreeScope frees;
     out.rows = rows;
     out.cols = cols;
     out.nnz = nnz;
