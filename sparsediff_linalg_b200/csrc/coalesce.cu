@@ -348,13 +348,6 @@ __global__ void __launch_bounds__(CB_CHUNK_THREADS) k_cb_scatter(const double *_
     }
 }
 
-// Starts reading the 16-byte words of [first, last) into L2.
-__device__ __forceinline__ void cb_prefetch(const int *first, const int *last)
-{
-    const uintptr_t a = (uintptr_t)first & ~(uintptr_t)15, b = ((uintptr_t)last + 15) & ~(uintptr_t)15;
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(b - a)) : "memory");
-}
-
 // Pass 2: a CTA per bucket, a thread per output, four outputs at a time so that their
 // loads are in flight together (the first ones beside the bucket's copy).
 __global__ void __launch_bounds__(CB_THREADS) k_cb_sum(const int *__restrict__ begin, const int *__restrict__ ostart,
@@ -369,7 +362,7 @@ __global__ void __launch_bounds__(CB_THREADS) k_cb_sum(const int *__restrict__ b
     const double *sv = cb_smem + (b0 & 1);
     unsigned short *sl0 = reinterpret_cast<unsigned short *>(cb_smem + CB_CAP + 2);
     const unsigned short *sl = sl0 + (b0 & 7) - b0; // by sorted triplet
-    if (threadIdx.x == 0) cb_prefetch(ostart + o_begin, ostart + o_end + 1);
+    if (threadIdx.x == 0) prefetch_l2(ostart + o_begin, ostart + o_end + 1);
     if (fits)
     {
         // 16 bytes at a time from the even place at or before the first (buf has a spare

@@ -17,9 +17,11 @@
 //             bitmap over column windows (larger rows; the bitmap yields the
 //             columns already sorted);
 //   numeric:  row tiles (rows of <= TILE_T terms, grouped into CTA-sized tiles,
-//             with an output-major schedule built once per pattern), CTA + shared
+//             with an entry-major schedule built once per pattern); larger rows in
+//             windows of their outputs, or by output-major term lists; without either
+//             (the allocation-free refill, products beyond 31-bit offsets) CTA + shared
 //             accumulator (<= 8192 output entries), CTA + accumulator in C.x itself
-//             with a global column->position map (larger rows).
+//             with a global column->position map.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -2187,6 +2189,19 @@ void validate_product(const ProductDesc &d, const TuneConfig &cfg, Product &P, c
 }
 
 // ------------------------------------------------------------ rows beyond the tile budget
+// A row beyond the tile budget is refilled in windows: consecutive outputs with about
+// WIN_TARGET terms together (at most 2^WIN_BITS outputs and WIN_TERMS terms). A CTA
+// computes the window's products in upstream's visiting order -- so an entry's value is
+// read once for its run of terms, and a long row of A contiguously -- into shared memory,
+// and sums every output from there. Rows of more than WIN_MULT terms per output keep
+// output-major lists: at 20 terms per output the refill took 272 us against 506 us, at 48
+// 337 against 339 us, and an output's places are put in order by one thread.
+constexpr int WIN_BITS = 11;
+constexpr int WIN_TERMS = 4096;
+constexpr int WIN_TARGET = 3072;
+constexpr int WIN_MULT = 32;
+constexpr int WIN_THREADS = 256;
+
 // Term counts and output counts of the big rows.
 __global__ void k_big_sizes(const int *__restrict__ rows, int nbig, const long long *__restrict__ ub,
                             const int *__restrict__ Cp, long long *__restrict__ terms, long long *__restrict__ outs)
@@ -2201,13 +2216,15 @@ __global__ void k_big_sizes(const int *__restrict__ rows, int nbig, const long l
 }
 
 // One CTA per big row at a time (grid-stride over the rows): every term of the row,
-// in upstream's visiting order t (stored at the row's term offset + t), gets the key
-// = its output's index among all big-row outputs and its {A position, entry-value
-// slot}. Output positions come from a per-CTA global map column -> position; only
+// in upstream's visiting order t (stored at the row's term offset + t), gets a key and
+// its {A position, entry-value slot}. The key is its output's index among all big-row
+// outputs (bout_off), or, with `wins` (per row its first window and the windows' width),
+// its window << WIN_BITS | the output's place in the window. Output positions come from a per-CTA global map column -> position; only
 // the row's own columns are ever read, so it needs no clearing.
 __global__ void __launch_bounds__(512, 2) k_big_terms(const int *__restrict__ rows, int nbig,
                                                       const int *__restrict__ tterm_off,
-                                                      const int *__restrict__ bout_off, NumArgs a,
+                                                      const int *__restrict__ bout_off,
+                                                      const int2 *__restrict__ wins, NumArgs a,
                                                       int *__restrict__ posmap_all, int n,
                                                       unsigned *__restrict__ keys, uint2 *__restrict__ data,
                                                       const int *__restrict__ order, int *__restrict__ next_row)
@@ -2220,7 +2237,6 @@ __global__ void __launch_bounds__(512, 2) k_big_terms(const int *__restrict__ ro
     ch.len = ch.s + blockDim.x;
     ch.scr = ch.len + blockDim.x;
     int *posmap = posmap_all + (long long)blockIdx.x * n;
-    uint4 *rmap = reinterpret_cast<uint4 *>(posmap_all) + (long long)blockIdx.x * ((n + 63) / 64);
     __shared__ int q_sh;
     // the rows in the order `order` gives (largest first), handed out by a counter
     for (;;)
@@ -2236,6 +2252,7 @@ __global__ void __launch_bounds__(512, 2) k_big_terms(const int *__restrict__ ro
         for (int q = threadIdx.x; q < nr; q += blockDim.x) posmap[a.Ci[cs + q]] = q;
         __syncthreads();
         const long long base = tterm_off[it];
+        const int2 win = wins ? wins[it] : make_int2(0, 1);
         long long cursor = 0;
         const int ls = a.Lp[r], le = a.Lp[r + 1];
         for (int c = ls; c < le; c += blockDim.x)
@@ -2255,7 +2272,8 @@ __global__ void __launch_bounds__(512, 2) k_big_terms(const int *__restrict__ ro
                     atomicOr(a.err, 1);
                     continue;
                 }
-                keys[base + t] = (unsigned)(bout_off[it] + pos);
+                keys[base + t] = wins ? (unsigned)(win.x + pos / win.y) << WIN_BITS | (unsigned)(pos % win.y)
+                                      : (unsigned)(bout_off[it] + pos);
                 data[base + t] = make_uint2((unsigned)jj, slot);
             }
             cursor += total;
@@ -2265,21 +2283,186 @@ __global__ void __launch_bounds__(512, 2) k_big_terms(const int *__restrict__ ro
     }
 }
 
-// After the stable sort by output: the first pair of every output (every output
-// has a term, so each output index starts exactly one run).
-__global__ void k_big_starts(const unsigned *__restrict__ keys, int T, int O, int *__restrict__ ostart,
+// After the stable sort by (key >> shift): the first pair of every output or window (each
+// has a term, so each starts exactly one run).
+__global__ void k_big_starts(const unsigned *__restrict__ keys, int T, int shift, int O, int *__restrict__ ostart,
                              int *__restrict__ err)
 {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < T;
          i += (long long)gridDim.x * blockDim.x)
     {
-        const unsigned k = keys[i];
+        const unsigned k = keys[i] >> shift;
         if (k >= (unsigned)O)
         {
             atomicOr(err, 1);
             continue;
         }
-        if (i == 0 || keys[i - 1] != k) ostart[k] = (int)i;
+        if (i == 0 || keys[i - 1] >> shift != k) ostart[k] = (int)i;
+    }
+}
+
+// Largest window of the sorted pairs.
+__global__ void k_win_max(const int *__restrict__ begin, int nwin, int *__restrict__ out)
+{
+    int m = 0;
+    for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < nwin; w += (long long)gridDim.x * blockDim.x)
+        m = max(m, begin[w + 1] - begin[w]);
+    m = __reduce_max_sync(FULL_MASK, m);
+    if (lane_id() == 0) atomicMax(out, m);
+}
+
+// A CTA per window: its descriptor, and its terms' places output by output: counted out
+// with shared-memory adds, then every output's places put in order (visiting order).
+__global__ void __launch_bounds__(WIN_THREADS) k_win_build(const int *__restrict__ rows, int nrows,
+                                                           const int2 *__restrict__ wins,
+                                                           const int *__restrict__ begin,
+                                                           const unsigned *__restrict__ keys,
+                                                           const uint2 *__restrict__ pairs, const int *__restrict__ Cp,
+                                                           long long nA, long long nV, BigWindow *__restrict__ win,
+                                                           const int *__restrict__ wout,
+                                                           unsigned short *__restrict__ terms,
+                                                           unsigned short *__restrict__ start, int *__restrict__ err)
+{
+    __shared__ int cur[1 << WIN_BITS], scr[32], row_sh;
+    __shared__ unsigned short list[WIN_TERMS];
+    const int w = blockIdx.x;
+    if (threadIdx.x == 0)
+    {
+        int lo = 0, hi = nrows; // last row whose first window is <= w
+        while (hi - lo > 1)
+        {
+            const int mid = (lo + hi) >> 1;
+            if (wins[mid].x <= w)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        row_sh = lo;
+    }
+    constexpr int PER = (1 << WIN_BITS) / WIN_THREADS;
+    for (int o = threadIdx.x; o < 1 << WIN_BITS; o += WIN_THREADS) cur[o] = 0;
+    __syncthreads();
+    const int it = row_sh, row = rows[it];
+    const int2 wn = wins[it];
+    const int first = (w - wn.x) * wn.y; // of the row's outputs
+    const int nout = min(wn.y, Cp[row + 1] - Cp[row] - first);
+    const int b = begin[w], n = begin[w + 1] - b;
+    for (int i = threadIdx.x; i < n; i += WIN_THREADS)
+    {
+        const uint2 q = pairs[b + i];
+        if ((long long)q.x >= nA || (long long)q.y >= nV) atomicOr(err, 1);
+        atomicAdd(&cur[keys[b + i] & ((1 << WIN_BITS) - 1)], 1);
+    }
+    __syncthreads();
+    int c[PER], sum = 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+    {
+        c[k] = cur[threadIdx.x * PER + k];
+        sum += c[k];
+        if ((c[k] > 0) != ((int)threadIdx.x * PER + k < nout)) atomicOr(err, 1); // every output has a term
+    }
+    int run = block_incl_scan_int(sum, scr) - sum;
+    const int s0 = wout[w];
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+    {
+        const int o = threadIdx.x * PER + k;
+        if (o <= nout) start[s0 + o] = (unsigned short)run;
+        cur[o] = run;
+        run += c[k];
+    }
+    if (threadIdx.x == WIN_THREADS - 1 && nout == 1 << WIN_BITS) start[s0 + nout] = (unsigned short)run;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += WIN_THREADS)
+        list[atomicAdd(&cur[keys[b + i] & ((1 << WIN_BITS) - 1)], 1)] = (unsigned short)i;
+    __syncthreads();
+    for (int o = threadIdx.x; o < nout; o += WIN_THREADS)
+    {
+        const int e = cur[o], f = o ? cur[o - 1] : 0; // the output's places end at e now
+        for (int i = f + 1; i < e; ++i)
+        {
+            const unsigned short x = list[i];
+            int j = i;
+            for (; j > f && list[j - 1] > x; --j) list[j] = list[j - 1];
+            list[j] = x;
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += WIN_THREADS) terms[b + i] = list[i];
+    if (threadIdx.x == 0) win[w] = BigWindow{b, n, Cp[row] + first, nout, s0, 0};
+}
+
+// Refill of the windows, a CTA each. What bounds it: the latency of the gathers of V and
+// A.x at 48 warps per SM (L1 26 %, L2 33 % hits), with HBM at 60 % of its bandwidth: 8 + 2
+// bytes per term, 2 + 8 per output, and A.x once per row of C. On the skewed 1M x 1M
+// product (399M terms, 302M outputs) 3.95 -> 2.15 ms against output-major lists, whose
+// two gathers per term each touch a sector of their own. Six CTAs per SM rather than 5
+// (2.32 ms) or 8 (3.8 ms: spills), windows of 3072 terms rather than 1536 (2.73 ms) or
+// 6144 (3.2 ms), the second phase's lists fetched into L2 during the first (2.21 ms
+// without).
+template <bool BATCHED>
+__global__ void __launch_bounds__(WIN_THREADS, 6) k_win_refill(const BigWindow *__restrict__ win,
+                                                            const uint2 *__restrict__ pairs,
+                                                            const unsigned short *__restrict__ terms,
+                                                            const unsigned short *__restrict__ start,
+                                                            const ProdPtrs *__restrict__ vals_dev, ProdPtrs vals,
+                                                            const double *__restrict__ V)
+{
+    extern __shared__ double wsm[];
+    const BigWindow D = win[blockIdx.x];
+    ProdPtrs P = vals;
+    if (BATCHED) P = *vals_dev;
+    const double *Vp = (P.Lx || P.d) ? V : nullptr;
+    const double *__restrict__ Ax = P.Ax;
+    const unsigned short *st = start + D.start, *tm = terms + D.pairs;
+    if (threadIdx.x == 0)
+    {
+        prefetch_l2(tm, tm + D.nterms);
+        prefetch_l2(st, st + D.nout + 1);
+    }
+    constexpr int U = 4; // terms and outputs of a thread whose loads are in flight together
+    const uint2 *pr = pairs + D.pairs;
+    for (int i0 = threadIdx.x; i0 < D.nterms; i0 += U * WIN_THREADS)
+    {
+        uint2 q[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            if (i0 + j * WIN_THREADS < D.nterms) q[j] = __ldcs(pr + i0 + j * WIN_THREADS);
+        double v[U], x[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            if (i0 + j * WIN_THREADS < D.nterms)
+            {
+                v[j] = Vp ? Vp[q[j].y] : 1.0;
+                x[j] = Ax[q[j].x];
+            }
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            if (i0 + j * WIN_THREADS < D.nterms) wsm[i0 + j * WIN_THREADS] = __dmul_rn(v[j], x[j]);
+    }
+    __syncthreads();
+    double *C = P.Cx + D.out;
+    for (int o0 = threadIdx.x; o0 < D.nout; o0 += U * WIN_THREADS)
+    {
+        int a[U], e[U], l[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+        {
+            const int o = o0 + j * WIN_THREADS;
+            a[j] = o < D.nout ? st[o] : 0;
+            e[j] = o < D.nout ? st[o + 1] : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) l[j] = a[j] < e[j] ? tm[a[j]] : 0;
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+        {
+            if (a[j] >= e[j]) continue;
+            double acc = __dadd_rn(0.0, wsm[l[j]]);
+            for (int i = a[j] + 1; i < e[j]; ++i) acc = __dadd_rn(acc, wsm[tm[i]]);
+            __stcs(C + o0 + j * WIN_THREADS, acc);
+        }
     }
 }
 
@@ -2350,75 +2533,192 @@ __global__ void __launch_bounds__(256) k_big_refill(const int *__restrict__ brow
     P.Cx[cpos] = acc;
 }
 
-// Output-major term lists of the rows beyond the tile budget (k_big_terms, a stable
-// radix sort by output, k_big_starts). Kept within 31-bit offsets; larger products
-// keep the CTA kernels.
-void build_big_lists(const ProductDesc &d, Product &P, const long long *ub, const NumArgs &na, cudaStream_t s)
+// The big rows of a product on the host: their rows, terms and outputs.
+struct BigRows
+{
+    std::vector<int> rows;
+    std::vector<long long> terms, outs;
+    long long T = 0, O = 0;
+    void add(int row, long long t, long long o)
+    {
+        rows.push_back(row);
+        terms.push_back(t);
+        outs.push_back(o);
+        T += t;
+        O += o;
+    }
+    int n() const { return (int)rows.size(); }
+};
+
+template <class E>
+DevBuf<E> to_device(const std::vector<E> &v, cudaStream_t s)
+{
+    DevBuf<E> d(v.size());
+    SDL_CUDA(cudaMemcpyAsync(d.get(), v.data(), v.size() * sizeof(E), cudaMemcpyHostToDevice, s));
+    return d;
+}
+
+// The terms of the big rows B with their keys (k_big_terms), in visiting order.
+void big_terms(const Product &P, const BigRows &B, const int *rows, const int *bout_off, const int2 *wins,
+               const NumArgs &na, unsigned *keys, uint2 *pairs, cudaStream_t s)
+{
+    Runtime &rt = runtime();
+    const int nb = B.n();
+    std::vector<int> toff((size_t)nb + 1, 0), ord(nb);
+    for (int i = 0; i < nb; ++i)
+    {
+        toff[i + 1] = toff[i] + (int)B.terms[i];
+        ord[i] = i;
+    }
+    // the rows by term count, largest first (a counter hands them out)
+    std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return B.terms[x] > B.terms[y]; });
+    const DevBuf<int> dtoff = to_device(toff, s), order = to_device(ord, s);
+    DevBuf<int> counter(1);
+    SDL_CUDA(cudaMemsetAsync(counter.get(), 0, sizeof(int), s));
+    const long long per_slot = std::max(1, P.n);
+    const int slots = (int)std::min<long long>(
+        {(long long)rt.num_sms * 2, std::max<long long>(1, (2LL << 30) / (per_slot * 4)), (long long)nb});
+    DevBuf<int> posmap((size_t)slots * per_slot);
+    const int th = 512;
+    const size_t sm = (3 * (size_t)th + 32) * 4;
+    SDL_LAUNCH(k_big_terms, slots, th, sm, s, rows, nb, dtoff.get(), bout_off, wins, na, posmap.get(), P.n, keys,
+               pairs, order.get(), counter.get());
+    if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "product plan: a term column is missing from its row");
+}
+
+int bits_for(long long v) // of the values 0 .. v - 1
+{
+    int b = 1;
+    while (b < 32 && (1LL << b) < v) ++b;
+    return b;
+}
+
+// Windows of the rows B (false: a window holds more than WIN_TERMS terms, or there are
+// too many). The windows of a row have about WIN_TARGET >> halve terms.
+bool build_windows(Product &P, const BigRows &B, int halve, const NumArgs &na, cudaStream_t s)
+{
+    Runtime &rt = runtime();
+    const int nb = B.n();
+    std::vector<int2> wins(nb);
+    std::vector<int> wout; // first entry of each window in win_start
+    long long starts = 0, nwin = 0;
+    for (int i = 0; i < nb; ++i)
+    {
+        const long long want = (long long)(WIN_TARGET >> halve) * B.outs[i] / std::max(1LL, B.terms[i]);
+        const int width = (int)std::max(1LL, std::min<long long>(want, 1 << WIN_BITS));
+        wins[i] = make_int2((int)nwin, width);
+        const long long k = (B.outs[i] + width - 1) / width;
+        if (nwin + k >= 1LL << (32 - WIN_BITS)) return false;
+        nwin += k;
+        for (long long q = 0; q < k; ++q)
+        {
+            wout.push_back((int)starts);
+            starts += std::min<long long>(width, B.outs[i] - q * width) + 1;
+        }
+    }
+    if (starts > INT_MAX) return false;
+    const int T = (int)B.T, W = (int)nwin;
+    const DevBuf<int> rows = to_device(B.rows, s), dwout = to_device(wout, s);
+    const DevBuf<int2> dwins = to_device(wins, s);
+    DevBuf<unsigned> keys(T), keys2(T);
+    DevBuf<uint2> tmp(T);
+    P.win_pairs.reset(T);
+    big_terms(P, B, rows.get(), nullptr, dwins.get(), na, keys.get(), P.win_pairs.get(), s);
+    if (radix_sort_pairs(keys.get(), P.win_pairs.get(), keys2.get(), tmp.get(), T, WIN_BITS, bits_for(W), s))
+    {
+        std::swap(keys, keys2);
+        std::swap(P.win_pairs, tmp);
+    }
+    keys2.release();
+    tmp.release();
+    DevBuf<int> begin((size_t)W + 1), largest(1);
+    SDL_CUDA(cudaMemcpyAsync(begin.get() + W, &T, sizeof(int), cudaMemcpyHostToDevice, s));
+    SDL_CUDA(cudaMemsetAsync(largest.get(), 0, sizeof(int), s));
+    SDL_LAUNCH(k_big_starts, grid_for(T, 256, rt.num_sms * 8), 256, 0, s, keys.get(), T, WIN_BITS, W, begin.get(),
+               rt.d_error);
+    if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "product plan: heavy-row windows are inconsistent");
+    SDL_LAUNCH(k_win_max, grid_for(W, 256, rt.num_sms * 4), 256, 0, s, begin.get(), W, largest.get());
+    int most = 0;
+    SDL_CUDA(cudaMemcpyAsync(&most, largest.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+    SDL_CUDA(cudaStreamSynchronize(s));
+    if (most > WIN_TERMS)
+    {
+        P.win_pairs.release();
+        return false;
+    }
+    P.win.reset(W);
+    P.win_terms.reset(T);
+    P.win_start.reset((size_t)starts);
+    SDL_LAUNCH(k_win_build, W, WIN_THREADS, 0, s, rows.get(), nb, dwins.get(), begin.get(), keys.get(),
+               P.win_pairs.get(), P.Cp.get(), (long long)P.desc.A_nnz, (long long)P.desc.L_nnz * P.desc.blocks,
+               P.win.get(), dwout.get(), P.win_terms.get(), P.win_start.get(), rt.d_error);
+    if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "product plan: heavy-row windows are inconsistent");
+    P.nwin = W;
+    P.win_most = most;
+    return true;
+}
+
+// Output-major term lists of the rows B (a stable sort by output, k_big_starts).
+void build_lists(Product &P, const BigRows &B, const NumArgs &na, cudaStream_t s)
+{
+    Runtime &rt = runtime();
+    const int nb = B.n(), T = (int)B.T, O = (int)B.O;
+    std::vector<int> ooff((size_t)nb + 1, 0);
+    for (int i = 0; i < nb; ++i) ooff[i + 1] = ooff[i] + (int)B.outs[i];
+    P.brows = to_device(B.rows, s);
+    P.bout_off = to_device(ooff, s);
+    DevBuf<unsigned> keys(T), keys2(T);
+    DevBuf<uint2> tmp(T);
+    P.bpairs.reset(T);
+    big_terms(P, B, P.brows.get(), P.bout_off.get(), nullptr, na, keys.get(), P.bpairs.get(), s);
+    if (radix_sort_pairs(keys.get(), P.bpairs.get(), keys2.get(), tmp.get(), T, 0, bits_for(O), s))
+    {
+        std::swap(keys, keys2);
+        std::swap(P.bpairs, tmp);
+    }
+    P.bostart.reset((size_t)O + 1);
+    SDL_CUDA(cudaMemcpyAsync(P.bostart.get() + O, &T, sizeof(int), cudaMemcpyHostToDevice, s));
+    SDL_LAUNCH(k_big_starts, grid_for(T, 256, rt.num_sms * 8), 256, 0, s, keys.get(), T, 0, O, P.bostart.get(),
+               rt.d_error);
+    if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "product plan: heavy-row term lists are inconsistent");
+    P.nbig = nb;
+    P.big_outputs = O;
+}
+
+// Refill forms of the rows beyond the tile budget. Kept within 31-bit offsets; larger
+// products keep the CTA kernels.
+void build_big_rows(Product &P, const long long *ub, const NumArgs &na, cudaStream_t s)
 {
     Runtime &rt = runtime();
     P.big_lists = false;
+    P.nwin = P.nbig = P.big_outputs = 0;
     const int nbig = P.num_count[NUM_C2K] + P.num_count[NUM_C8K] + P.num_count[NUM_GMEM];
     if (nbig == 0) return;
     const int *rows = P.num_rows.get() + P.num_offset[NUM_C2K]; // classes C2K, C8K, GMEM are adjacent
-    DevBuf<long long> terms(nbig), outs(nbig), toff((size_t)nbig + 1), ooff((size_t)nbig + 1);
+    DevBuf<long long> terms(nbig), outs(nbig);
     SDL_LAUNCH(k_big_sizes, grid_for(nbig, 256, rt.num_sms * 8), 256, 0, s, rows, nbig, ub, P.Cp.get(),
                terms.get(), outs.get());
-    const long long T = exclusive_scan_i64(terms.get(), toff.get(), nbig, s);
-    const long long O = exclusive_scan_i64(outs.get(), ooff.get(), nbig, s);
+    std::vector<long long> ht(nbig), ho(nbig);
+    std::vector<int> hr(nbig);
+    SDL_CUDA(cudaMemcpyAsync(ht.data(), terms.get(), nbig * sizeof(long long), cudaMemcpyDeviceToHost, s));
+    SDL_CUDA(cudaMemcpyAsync(ho.data(), outs.get(), nbig * sizeof(long long), cudaMemcpyDeviceToHost, s));
+    SDL_CUDA(cudaMemcpyAsync(hr.data(), rows, nbig * sizeof(int), cudaMemcpyDeviceToHost, s));
+    SDL_CUDA(cudaStreamSynchronize(s));
+    BigRows W, L;
+    long long T = 0, O = 0;
+    for (int i = 0; i < nbig; ++i)
+    {
+        T += ht[i];
+        O += ho[i];
+        (ht[i] <= WIN_MULT * ho[i] ? W : L).add(hr[i], ht[i], ho[i]);
+    }
     if (T >= INT_MAX || O >= INT_MAX || T < O) return; // the CTA kernels handle them
-    // 32-bit copies of the offsets (the sort and the refill take int offsets)
-    std::vector<long long> ht((size_t)nbig + 1), ho((size_t)nbig + 1);
-    SDL_CUDA(cudaMemcpyAsync(ht.data(), toff.get(), ht.size() * sizeof(long long), cudaMemcpyDeviceToHost, s));
-    SDL_CUDA(cudaMemcpyAsync(ho.data(), ooff.get(), ho.size() * sizeof(long long), cudaMemcpyDeviceToHost, s));
+    bool windows = W.n() == 0;
+    for (int halve = 0; halve <= 2 && !windows; ++halve) windows = build_windows(P, W, halve, na, s);
+    if (!windows)
+        for (int i = 0; i < W.n(); ++i) L.add(W.rows[i], W.terms[i], W.outs[i]);
+    if (L.n()) build_lists(P, L, na, s);
     SDL_CUDA(cudaStreamSynchronize(s));
-    std::vector<int> hti(ht.begin(), ht.end()), hoi(ho.begin(), ho.end());
-    DevBuf<int> toff32 = DevBuf<int>((size_t)nbig + 1);
-    P.bout_off.reset((size_t)nbig + 1);
-    SDL_CUDA(cudaMemcpyAsync(toff32.get(), hti.data(), hti.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-    SDL_CUDA(cudaMemcpyAsync(P.bout_off.get(), hoi.data(), hoi.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-    // terms -> (output, pair), then a stable sort by output
-    const long long per_slot = std::max(1, P.n);
-    const int slots = (int)std::min<long long>(
-        {(long long)rt.num_sms * 2, std::max<long long>(1, (2LL << 30) / (per_slot * 4)), (long long)nbig});
-    // the rows by term count, largest first (a counter hands them out)
-    std::vector<int> ord(nbig);
-    {
-        std::vector<long long> tc(nbig);
-        for (int i = 0; i < nbig; ++i) tc[i] = ht[i + 1] - ht[i];
-        for (int i = 0; i < nbig; ++i) ord[i] = i;
-        std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return tc[x] > tc[y]; });
-    }
-    DevBuf<int> order((size_t)nbig), counter(1);
-    SDL_CUDA(cudaMemcpyAsync(order.get(), ord.data(), (size_t)nbig * sizeof(int), cudaMemcpyHostToDevice, s));
-    SDL_CUDA(cudaMemsetAsync(counter.get(), 0, sizeof(int), s));
-    {
-        DevBuf<int> posmap((size_t)slots * per_slot);
-        DevBuf<unsigned> keys(std::max<long long>(1, T)), keys2(std::max<long long>(1, T));
-        DevBuf<uint2> tmp(std::max<long long>(1, T));
-        P.bpairs.reset(std::max<long long>(1, T));
-        const int th = 512;
-        const size_t sm = (3 * (size_t)th + 32) * 4;
-        SDL_LAUNCH(k_big_terms, slots, th, sm, s, rows, nbig, toff32.get(), P.bout_off.get(), na, posmap.get(), P.n,
-                   keys.get(), P.bpairs.get(), order.get(), counter.get());
-        if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "product plan: a term column is missing from its row");
-        int bits = 1;
-        while (bits < 32 && (1LL << bits) < O) ++bits;
-        if (radix_sort_pairs(keys.get(), P.bpairs.get(), keys2.get(), tmp.get(), (int)T, bits, s))
-        {
-            std::swap(keys, keys2);
-            std::swap(P.bpairs, tmp);
-        }
-        P.bostart.reset((size_t)O + 1);
-        SDL_CUDA(cudaMemcpyAsync(P.bostart.get() + O, &hti[nbig], sizeof(int), cudaMemcpyHostToDevice, s));
-        SDL_LAUNCH(k_big_starts, grid_for(T, 256, rt.num_sms * 8), 256, 0, s, keys.get(), (int)T, (int)O,
-                   P.bostart.get(), rt.d_error);
-        if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "product plan: heavy-row term lists are inconsistent");
-    }
-    P.brows.reset(nbig);
-    SDL_CUDA(cudaMemcpyAsync(P.brows.get(), rows, (size_t)nbig * sizeof(int), cudaMemcpyDeviceToDevice, s));
-    SDL_CUDA(cudaStreamSynchronize(s));
-    P.nbig = nbig;
-    P.big_outputs = (int)O;
     P.big_lists = true;
 }
 
@@ -2607,7 +2907,7 @@ void build_schedule(const ProductDesc &d, Product &P, const long long *ub, cudaS
         P.max_tile_terms = hmx[0];
         P.max_tile_ent = hmx[1];
     }
-    build_big_lists(d, P, ub, na, s);
+    build_big_rows(P, ub, na, s);
     if (P.num_count[NUM_GMEM] && !P.big_lists)
     {
         long long per_slot = std::max(1, P.n);
@@ -3378,10 +3678,21 @@ void product_numeric(const Product &P, const double *Lx, const double *dvec, con
 
 void big_lists_refill(const Product &P, const ProdPtrs *ptrs, cudaStream_t s, ProdPtrs vals, const double *V)
 {
-    if (!P.big_lists || P.big_outputs == 0) return;
-    const int grid = (P.big_outputs + 255) / 256;
+    if (!P.big_lists) return;
     const long long nV = (long long)P.desc.L_nnz * P.desc.blocks;
     if (!V) V = P.V.get();
+    if (P.nwin)
+    {
+        const size_t sm = (size_t)P.win_most * sizeof(double);
+        if (ptrs)
+            SDL_LAUNCH(k_win_refill<true>, P.nwin, WIN_THREADS, sm, s, P.win.get(), P.win_pairs.get(),
+                       P.win_terms.get(), P.win_start.get(), ptrs, vals, V);
+        else
+            SDL_LAUNCH(k_win_refill<false>, P.nwin, WIN_THREADS, sm, s, P.win.get(), P.win_pairs.get(),
+                       P.win_terms.get(), P.win_start.get(), ptrs, vals, V);
+    }
+    if (P.big_outputs == 0) return;
+    const int grid = (P.big_outputs + 255) / 256;
     if (ptrs)
         SDL_LAUNCH(k_big_refill<true>, grid, 256, 0, s, P.brows.get(), P.nbig, P.bout_off.get(), P.big_outputs,
                    P.bostart.get(), P.bpairs.get(), P.Cp.get(), ptrs, vals, V, nV, (long long)P.desc.A_nnz,

@@ -61,15 +61,16 @@ struct CooSource
     __device__ unsigned val(int i) const { return (unsigned)i; }
 };
 
-// Byte `byte` of a key.
-__device__ __forceinline__ unsigned digit(unsigned key, int byte) { return __byte_perm(key, 0, byte) & 255u; }
-__device__ __forceinline__ unsigned digit(unsigned long long key, int byte)
+// The 8 bits of a key from bit `bit` on.
+__device__ __forceinline__ unsigned digit(unsigned key, int bit) { return (key >> bit) & 255u; }
+__device__ __forceinline__ unsigned digit(unsigned long long key, int bit)
 {
-    return __byte_perm((unsigned)key, (unsigned)(key >> 32), byte) & 255u;
+    return __byte_perm((unsigned)key, (unsigned)(key >> 32), bit >> 3) & 255u; // (whole bytes)
 }
 
 template <class Src>
-__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(Src src, int n, int passes, unsigned *__restrict__ hist)
+__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(Src src, int n, int low_bit, int passes,
+                                                       unsigned *__restrict__ hist)
 {
     __shared__ unsigned cnt[RS_MAX_PASSES * 256];
     for (int k = threadIdx.x; k < passes * 256; k += RS_THREADS) cnt[k] = 0;
@@ -92,7 +93,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(Src src, int n, int pass
             for (int p = 0; p < passes; ++p)
             {
                 // neighbours often share their high digits: one add for the warp then
-                const unsigned d = digit(key[j], p);
+                const unsigned d = digit(key[j], low_bit + 8 * p);
                 const unsigned same = __ballot_sync(FULL_MASK, d == __shfl_sync(FULL_MASK, d, 0));
                 if ((same & act) == act)
                 {
@@ -141,7 +142,7 @@ constexpr size_t rs_smem_bytes()
 }
 
 template <class K, class V, class W, class Src>
-__global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(Src src, int n, int byte,
+__global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(Src src, int n, int bit,
                                                                   const unsigned *__restrict__ hist, W *words,
                                                                   int *__restrict__ ticket, K *__restrict__ okeys,
                                                                   V *__restrict__ ovals, int *__restrict__ err)
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(Src src, int n,
 #pragma unroll
     for (int j = 0; j < RS_ITEMS; ++j)
     {
-        const unsigned dg = digit(key[j], byte);
+        const unsigned dg = digit(key[j], bit);
         int *c = &wc[w][dg];
         const unsigned grp = warp_match8(dg);
         rank[j] = *c + __popc(grp & lanemask_lt());
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(Src src, int n,
         wc[ww][d] = total;
         total += c;
     }
-    if (d == 255) total -= RS_TILE - tn;
+    if (d == (int)digit(~K(0), bit)) total -= RS_TILE - tn;
     volatile W *word = words + (size_t)tile * 256 + d;
     *word = (W(tile ? 1 : 2) << TileWord<W>::SHIFT) | W(total);
     const int lstart = block_incl_scan_int(total, scr) - total; // (ends with a barrier)
@@ -202,7 +203,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(Src src, int n,
 #pragma unroll
     for (int j = 0; j < RS_ITEMS; ++j)
     {
-        const int pos = wc[w][digit(key[j], byte)] + rank[j];
+        const int pos = wc[w][digit(key[j], bit)] + rank[j];
         sk[pos] = key[j];
         sv[pos] = val[j];
     }
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(Src src, int n,
     for (int j = threadIdx.x; j < tn; j += RS_THREADS)
     {
         const K k = sk[j];
-        const unsigned pos = (unsigned)(gbase[digit(k, byte)] + j);
+        const unsigned pos = (unsigned)(gbase[digit(k, bit)] + j);
         if (pos < (unsigned)n) // (always, unless a look-back wait ran out)
         {
             okeys[pos] = k;
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS) k_rs_pass(Src src, int n,
 }
 
 template <class K, class V, class W, class Src>
-void rs_pass(const Src &src, int n, int byte, const unsigned *hist, W *words, int *ticket, K *okeys, V *ovals,
+void rs_pass(const Src &src, int n, int bit, const unsigned *hist, W *words, int *ticket, K *okeys, V *ovals,
              int ntiles, cudaStream_t s)
 {
     const auto kern = k_rs_pass<K, V, W, Src>;
@@ -264,14 +265,16 @@ void rs_pass(const Src &src, int n, int byte, const unsigned *hist, W *words, in
                                           (int)rs_smem_bytes<K, V>()));
     }
     SDL_CUDA(cudaMemsetAsync(words, 0, (size_t)ntiles * 256 * sizeof(W), s));
-    SDL_LAUNCH(kern, ntiles, RS_THREADS, (rs_smem_bytes<K, V>()), s, src, n, byte, hist, words, ticket, okeys, ovals,
+    SDL_LAUNCH(kern, ntiles, RS_THREADS, (rs_smem_bytes<K, V>()), s, src, n, bit, hist, words, ticket, okeys, ovals,
                runtime().d_error);
 }
 
-// Sorts the n pairs of `first` by the low `bits` bits of the key: pass 0 writes them to
+// Sorts the n pairs of `first` by `bits` bits of the key from low_bit on (a multiple of 8
+// for 64-bit keys): pass 0 writes them to
 // (kb, vb), the next to (ka, va), and so on. True if they end in (kb, vb).
 template <class K, class V, class W, class Src>
-bool rs_sort(const Src &first, K *ka, V *va, K *kb, V *vb, int n, int bits, cudaStream_t s)
+bool rs_sort(const Src &first, K *ka, V *va, K *kb, V *vb, int n, int low_bit, int bits,
+             cudaStream_t s)
 {
     const int ntiles = (int)(((long long)n + RS_TILE - 1) / RS_TILE);
     const int passes = std::max(1, (bits + 7) / 8);
@@ -279,7 +282,7 @@ bool rs_sort(const Src &first, K *ka, V *va, K *kb, V *vb, int n, int bits, cuda
     SDL_CUDA(cudaMemsetAsync(hist.get(), 0, hist.bytes(), s));
     DevBuf<W> words((size_t)ntiles * 256);
     const int grid = std::min(ntiles, runtime().num_sms * 8);
-    SDL_LAUNCH(k_rs_hist<Src>, grid, RS_THREADS, 0, s, first, n, passes, hist.get());
+    SDL_LAUNCH(k_rs_hist<Src>, grid, RS_THREADS, 0, s, first, n, low_bit, passes, hist.get());
     bool in_b = false;
     for (int p = 0; p < passes; ++p, in_b = !in_b)
     {
@@ -287,9 +290,10 @@ bool rs_sort(const Src &first, K *ka, V *va, K *kb, V *vb, int n, int bits, cuda
         K *ok = in_b ? ka : kb;
         V *ov = in_b ? va : vb;
         if (p == 0)
-            rs_pass<K, V, W>(first, n, 0, hist.get(), words.get(), ticket, ok, ov, ntiles, s);
+            rs_pass<K, V, W>(first, n, low_bit, hist.get(), words.get(), ticket, ok, ov, ntiles, s);
         else
-            rs_pass<K, V, W>(PairSource<K, V>{in_b ? kb : ka, in_b ? vb : va}, n, p, hist.get() + 256 * p,
+            rs_pass<K, V, W>(PairSource<K, V>{in_b ? kb : ka, in_b ? vb : va}, n,
+                             low_bit + 8 * p, hist.get() + 256 * p,
                              words.get(), ticket, ok, ov, ntiles, s);
     }
     return in_b;
@@ -299,14 +303,15 @@ constexpr int RS_WORD32_MAX = 1 << 30; // pairs that a 32-bit tile word can coun
 
 } // namespace
 
-bool radix_sort_pairs(unsigned *keys, uint2 *vals, unsigned *keys_tmp, uint2 *vals_tmp, int n, int key_bits,
-                      cudaStream_t s)
+bool radix_sort_pairs(unsigned *keys, uint2 *vals, unsigned *keys_tmp, uint2 *vals_tmp, int n, int low_bit,
+                      int bits, cudaStream_t s)
 {
     if (n <= 0) return false;
     const PairSource<unsigned, uint2> src{keys, vals};
-    return n < RS_WORD32_MAX ? rs_sort<unsigned, uint2, unsigned>(src, keys, vals, keys_tmp, vals_tmp, n, key_bits, s)
-                             : rs_sort<unsigned, uint2, unsigned long long>(src, keys, vals, keys_tmp, vals_tmp, n,
-                                                                            key_bits, s);
+    return n < RS_WORD32_MAX
+               ? rs_sort<unsigned, uint2, unsigned>(src, keys, vals, keys_tmp, vals_tmp, n, low_bit, bits, s)
+               : rs_sort<unsigned, uint2, unsigned long long>(src, keys, vals, keys_tmp, vals_tmp, n, low_bit, bits,
+                                                              s);
 }
 
 bool radix_sort_coo(const int *rows, const int *cols, int n, int row_bits, int col_bits, unsigned long long *ka,
@@ -315,8 +320,8 @@ bool radix_sort_coo(const int *rows, const int *cols, int n, int row_bits, int c
     const CooSource src{rows, cols, col_bits};
     const int bits = row_bits + col_bits;
     return n < RS_WORD32_MAX
-               ? rs_sort<unsigned long long, unsigned, unsigned>(src, ka, va, kb, vb, n, bits, s)
-               : rs_sort<unsigned long long, unsigned, unsigned long long>(src, ka, va, kb, vb, n, bits, s);
+               ? rs_sort<unsigned long long, unsigned, unsigned>(src, ka, va, kb, vb, n, 0, bits, s)
+               : rs_sort<unsigned long long, unsigned, unsigned long long>(src, ka, va, kb, vb, n, 0, bits, s);
 }
 
 } // namespace sdl

@@ -185,4 +185,12 @@ __device__ __forceinline__ int lower_bound_dev(const K *a, int n, K key)
     return lo;
 }
 
+// Starts reading the 16-byte words that hold [first, last) into L2 (one thread).
+template <class E>
+__device__ __forceinline__ void prefetch_l2(const E *first, const E *last)
+{
+    const uintptr_t a = (uintptr_t)first & ~(uintptr_t)15, b = ((uintptr_t)last + 15) & ~(uintptr_t)15;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(b - a)) : "memory");
+}
+
 } // namespace sdl

@@ -206,13 +206,13 @@ int coalesce_build(const int *rows, const int *cols, int n, int m, int ncols, De
                    DevBuf<int> &perm, DevBuf<int> &ostart, CoalesceBuckets &buckets, cudaStream_t s);
 void coalesce_bucket_fill(const CoalesceBuckets &B, const int *ostart, const double *x, const double *f, double *C,
                           cudaStream_t s);
-// Stable radix sorts (csrc/radix.cu): of (key, payload) pairs by the low key_bits bits,
-// using the second pair of buffers as scratch -- true if the result is in them; and of
+// Stable radix sorts (csrc/radix.cu): of (key, payload) pairs by `bits` bits of the key
+// from low_bit on, using the second pair of buffers as scratch -- true if the result is in them; and of
 // COO triplets by (row, column), giving row << col_bits | column and the triplet, in the
 // first pair of buffers (false) or the second (true). A wait that runs out sets the
 // device error word.
-bool radix_sort_pairs(unsigned *keys, uint2 *vals, unsigned *keys_tmp, uint2 *vals_tmp, int n, int key_bits,
-                      cudaStream_t s);
+bool radix_sort_pairs(unsigned *keys, uint2 *vals, unsigned *keys_tmp, uint2 *vals_tmp, int n, int low_bit,
+                      int bits, cudaStream_t s);
 bool radix_sort_coo(const int *rows, const int *cols, int n, int row_bits, int col_bits, unsigned long long *ka,
                     unsigned *va, unsigned long long *kb, unsigned *vb, cudaStream_t s);
 
@@ -343,6 +343,13 @@ struct ProductDesc
     int A_m = 0, A_n = 0, A_nnz = 0;
 };
 
+// Outputs [out, out + nout) of C, of one row beyond the tile budget.
+struct BigWindow
+{
+    int pairs, nterms; // its pairs
+    int out, nout;
+    int start, pad; // its outputs' entries of win_start (nout + 1)
+};
 struct Product
 {
     ProductDesc desc;
@@ -365,9 +372,18 @@ struct Product
     DevBuf<double> V;      // entry values of the current refill (L_nnz * blocks)
     DevBuf<int> gmem_scratch; // posmap scratch for NUM_GMEM rows (slots x n ints)
     int gmem_slots = 0;
-    // Rows beyond the tile budget, output-major: every output's terms as {A
-    // position, entry-value slot} pairs in upstream's visiting order (big_lists).
+    // Rows beyond the tile budget, by the terms' {A position, entry-value slot} pairs
+    // (big_lists: every such row has its pairs in one of the two forms).
+    // Windows: a few thousand terms of consecutive outputs of one row, its pairs in
+    // upstream's visiting order; per output its terms' places in the window.
     bool big_lists = false;
+    int nwin = 0, win_most = 0; // win_most: terms of the largest window
+    DevBuf<BigWindow> win;
+    DevBuf<uint2> win_pairs;
+    DevBuf<unsigned short> win_terms; // the terms' places, output by output
+    DevBuf<unsigned short> win_start; // first of every output's (and one past the last's)
+    // Output-major lists, for rows of many terms per output: every output's pairs, in
+    // upstream's visiting order.
     int nbig = 0, big_outputs = 0;
     DevBuf<int> brows;          // the rows (big row i = brows[i])
     DevBuf<int> bout_off;       // outputs of big rows before big row i (nbig + 1)
@@ -461,7 +477,7 @@ bool pipe_refill(const Product &P);
 bool entry_values_are_lx(const Product &P, const double *Lx, const double *dvec);
 // Copies `n` descriptors, setting `prod`.
 void rebase_tiles(const TileDesc *src, int n, int prod, TileDesc *dst, cudaStream_t s);
-// The larger rows of one product from their output-major term lists (needs
+// The larger rows of one product from their windows and term lists (needs
 // P.big_lists), values as in tile_refill.
 // V: the entry values to read (null: the product's own scratch).
 void big_lists_refill(const Product &P, const ProdPtrs *ptrs, cudaStream_t s, ProdPtrs vals = ProdPtrs{},

@@ -139,3 +139,59 @@ def test_transpose_segment_edges(sdl, orc, rows, cols, lens):
     wp, wi, wx = orc.transpose(p, col, x, rows, cols)
     assert np.array_equal(t.Tp.cpu().numpy(), wp) and np.array_equal(t.Ti.cpu().numpy(), wi)
     assert np.array_equal(bits(tx.cpu().numpy()), bits(wx))
+
+
+# ---------------------------------------------------------------- rows beyond the tile budget
+# windows of about one term per output, of many (few outputs a window), rows of so many
+# that they keep lists, rows whose columns crowd so that windows are halved, and rows with
+# one output of more terms than a window holds; one row of exactly one window and its edges
+@pytest.mark.parametrize("kind,nL,nA,n,per_row", [
+    ("even", 12, 3000, 200000, 5), ("even", 7, 2500, 2500, 20), ("even", 5, 2000, 300, 40),
+    ("crowded", 9, 4000, 60000, 6), ("hot", 6, 6000, 90000, 3), ("even", 3, 1025, 2048, 2),
+    ("even", 2, 1024, 2047, 3), ("even", 4, 20000, 2049, 1)])
+def test_large_row_windows_bit_exact(sdl, orc, kind, nL, nA, n, per_row):
+    import torch
+    from sparsediff_linalg_b200.device import Batch, Product
+    rng = np.random.default_rng(nA + n)
+    rows = []
+    for _ in range(nA):
+        if kind == "crowded":   # most columns in a twentieth of the range
+            c = np.where(rng.random(per_row) < 0.8, rng.integers(0, n // 20, per_row), rng.integers(0, n, per_row))
+        elif kind == "hot":     # one column in every row
+            c = np.concatenate([[7], rng.integers(0, n, per_row)])
+        else:
+            c = rng.integers(0, n, per_row)
+        rows.append(np.unique(c))
+    Bp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    Bi = np.concatenate(rows).astype(np.int32)
+    lens = rng.integers(nA // 2, nA + 1, nL)
+    lens[0], lens[-1] = nA, 3
+    Ap = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    Ai = np.concatenate([np.sort(rng.permutation(nA)[:k]) for k in lens]).astype(np.int32)
+    P = Product(T(Ap), T(Ai), T(Bp), T(Bi), n)
+    Q = Product(T(Ap), T(Ai), T(Bp), T(Bi), n)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    batch = Batch([P, Q], stream=s)
+    for rnd in range(2):
+        Ax, Bx, d = rng.standard_normal(len(Ai)), rng.standard_normal(len(Bi)), rng.uniform(0.1, 10, nA)
+        Ax[::3] = -0.0
+        wp, wi, wx = orc.spgemm((Ap, Ai, Ax, nL, nA), (Bp, Bi, Bx, nA, n))
+        assert np.array_equal(P.Cp.cpu().numpy(), wp) and np.array_equal(P.Ci.cpu().numpy(), wi)
+        C = torch.full((P.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+        P.fill(T(Ax), None, T(Bx), C)
+        assert np.array_equal(bits(C.cpu().numpy()), bits(wx))
+        # the same with a diagonal, single and batched: (a * d) * b, one rounding each
+        wd = orc.spgemm((Ap, Ai, Ax * d[Ai], nL, nA), (Bp, Bi, Bx, nA, n))[2]
+        dev = [T(Ax), T(d), T(Bx)]
+        C.fill_(float("nan"))
+        P.fill(dev[0], dev[1], dev[2], C)
+        assert np.array_equal(bits(C.cpu().numpy()), bits(wd))
+        out = [torch.full((P.nnz,), float("nan"), dtype=torch.float64, device="cuda") for _ in range(2)]
+        for i in range(2):
+            batch.bind(i, dev[0], dev[1], dev[2], out[i])
+        torch.cuda.synchronize()
+        batch.refill(stream=s)
+        torch.cuda.synchronize()
+        for o in out:
+            assert np.array_equal(bits(o.cpu().numpy()), bits(wd))
