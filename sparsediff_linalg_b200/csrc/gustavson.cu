@@ -176,14 +176,15 @@ __global__ void k_mask_classes(const unsigned char *__restrict__ mask, int m_out
         if (!mask[r]) cls[r] = 255;
 }
 
-// Numeric class and tile weight of every output row. A tile row costs its terms,
+// Numeric class, tile weight and terms in tiles of every output row. A tile row costs its terms,
 // one unit per 16 of its L entries and TILE_T / TILE_THREADS units; a larger row
 // costs TILE_T, so it always ends its tile. Rows with more than TILE_MAX_LROW L
 // entries never join a tile (the 18-bit entry index of a term word stays in range).
 constexpr int TILE_MAX_LROW = 131072;
 __global__ void k_num_classify(const long long *__restrict__ ub, const int *__restrict__ Cp,
                                const int *__restrict__ Lp, int L_m, int m_out, int tile_max,
-                               unsigned char *__restrict__ cls, long long *__restrict__ weight)
+                               unsigned char *__restrict__ cls, long long *__restrict__ weight,
+                               long long *__restrict__ tterms)
 {
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < m_out;
          r += (long long)gridDim.x * blockDim.x)
@@ -206,6 +207,7 @@ __global__ void k_num_classify(const long long *__restrict__ ub, const int *__re
         cls[r] = (unsigned char)c;
         const long long lw = (lenL + 15) / 16 + TILE_T / TILE_THREADS;
         weight[r] = c == NUM_TILE ? u + lw : (c == 255 ? lw : TILE_T);
+        tterms[r] = c == NUM_TILE ? u : 0;
     }
 }
 
@@ -811,29 +813,31 @@ struct BuildSmem
 {
     int *cnt; // TILE_ACC: terms per output
     int *cur; // TILE_ACC: list cursor of an output with three or more terms, -1 otherwise
-    int *row_cs, *row_nr, *row_ls, *row_b, *row_outoff, *row_eoff;
+    int *ci;  // TILE_ACC: columns of the tile's outputs
+    unsigned *tw; // TILE_ACC: the terms, entry << TW_BITS | output
+    int *row_nr, *row_ls, *row_b, *row_outoff, *row_eoff;
     int *e_incl, *e_s, *e_len, *e_row;
     int *scr;
-    int *misc; // [1]: list outputs of a chunk, [2]: their terms
+    int *misc; // [0]: entries up to the last with a term, [1]: list outputs of a chunk, [2]: their terms
 };
+constexpr int TW_BITS = 11; // an output of a tile
+static_assert(TILE_ACC <= 1 << TW_BITS, "a tile's outputs fit its packed terms");
 constexpr size_t build_smem_bytes()
 {
-    return ((size_t)2 * TILE_ACC + 4 * TILE_THREADS + 2 * (TILE_THREADS + 1) + 4 * TILE_THREADS + 32 + 4) * 4;
+    return ((size_t)4 * TILE_ACC + 3 * TILE_THREADS + 2 * (TILE_THREADS + 1) + 4 * TILE_THREADS + 32 + 4) * 4;
 }
 
-// Term enumeration of one tile, shared by both passes of the schedule build. The
-// tile's L entries (every entry of its rows, in order: entry e is schedule entry
-// vbase + e) are taken 256 at a time; fe(e, s, toff, len, slot) is called for each
-// by its thread (s = A.p[k], toff = offset of its first term in the tile, len = its
-// terms, slot = index of its value in V),
-// then ft(valid, e, u, o) for every term in upstream's visiting order, 256
-// consecutive terms per step (valid false for the idle threads of the last step,
-// so every thread takes every barrier): u is the term's index in the tile, o its
-// output inside the tile window.
-template <class FE, class FT>
-__device__ __forceinline__ int tile_terms(const NumArgs &a, const BuildSmem &t, int nrows, int total_raw, FE fe,
-                                           FT ft)
+// Enumerates the terms of one tile in upstream's visiting order into t.tw and counts
+// them per output; returns their number. The tile's L entries (every entry of its rows,
+// in order: entry e is schedule entry vbase + e) are taken 256 at a time; fe(e, s, toff,
+// len, slot) is called for each by its thread (s = A.p[k], toff = offset of its first
+// term in the tile, len = its terms, slot = index of its value in V). The searches of
+// four terms per thread (a term's entry, its column among the row's outputs) run
+// together: each is a chain of dependent shared-memory reads.
+template <class FE>
+__device__ __forceinline__ int tile_terms(const NumArgs &a, const BuildSmem &t, int nrows, int total_raw, FE fe)
 {
+    constexpr int U = 4;
     const int tid = threadIdx.x;
     int cursor = 0;
     for (int ec = 0; ec < total_raw; ec += TILE_THREADS)
@@ -857,29 +861,53 @@ __device__ __forceinline__ int tile_terms(const NumArgs &a, const BuildSmem &t, 
         t.e_row[tid] = lrow;
         __syncthreads();
         const int total = t.e_incl[TILE_THREADS - 1];
-        const int nent = min(TILE_THREADS, total_raw - ec);
-        for (int base = 0; base < total; base += TILE_THREADS)
+        for (int base = tid; base < total; base += U * TILE_THREADS)
         {
-            const int uu = base + tid;
-            bool valid = uu < total;
-            int el = 0, o = 0;
-            if (valid)
+            int el[U], j[U], lo[U], w[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) el[q] = -1; // last entry whose terms end at or before the term
+#pragma unroll
+            for (int step = TILE_THREADS / 2; step; step >>= 1)
+#pragma unroll
+                for (int q = 0; q < U; ++q)
+                    if (t.e_incl[el[q] + step] <= base + q * TILE_THREADS) el[q] += step;
+#pragma unroll
+            for (int q = 0; q < U; ++q)
             {
-                el = cta_entry_of(t.e_incl, nent, uu);
-                const int jj = t.e_s[el] + uu - (t.e_incl[el] - t.e_len[el]);
-                const int j = a.Ai[jj];
-                const int lr = t.e_row[el];
-                const int w = t.row_nr[lr];
-                const int *crow = a.Ci + t.row_cs[lr];
-                const int pos = lower_bound_dev(crow, w, j);
-                if (pos >= w || crow[pos] != j)
+                const int uu = base + q * TILE_THREADS;
+                j[q] = -1;
+                w[q] = lo[q] = 0;
+                if (uu >= total) continue;
+                ++el[q];
+                j[q] = a.Ai[t.e_s[el[q]] + uu - (t.e_incl[el[q]] - t.e_len[el[q]])];
+                const int lr = t.e_row[el[q]];
+                lo[q] = t.row_outoff[lr];
+                w[q] = t.row_nr[lr];
+            }
+            // lower bound of j among ci[lo, lo + w)
+            for (int step = 1 << TW_BITS; step; step >>= 1)
+            {
+#pragma unroll
+                for (int q = 0; q < U; ++q)
+                    if (step <= w[q] && t.ci[lo[q] + step - 1] < j[q])
+                    {
+                        lo[q] += step;
+                        w[q] -= step;
+                    }
+            }
+#pragma unroll
+            for (int q = 0; q < U; ++q)
+            {
+                const int uu = base + q * TILE_THREADS;
+                if (uu >= total) continue;
+                if (w[q] == 0 || t.ci[lo[q]] != j[q] || cursor + uu >= TILE_ACC)
                 {
                     atomicOr(a.err, 1);
-                    valid = false;
+                    continue;
                 }
-                o = t.row_outoff[lr] + pos;
+                t.tw[cursor + uu] = (unsigned)(ec + el[q]) << TW_BITS | (unsigned)lo[q];
+                atomicAdd(&t.cnt[lo[q]], 1);
             }
-            ft(valid, ec + el, cursor + uu, o);
         }
         cursor += total;
         __syncthreads();
@@ -902,26 +930,37 @@ __global__ void k_value_rows(const int *__restrict__ L_map, const int *__restric
     }
 }
 
+// What the schedule build reports: the words of X handed out, the largest window, term
+// count and entry count of a tile, and whether X was too small.
+struct SchedTotals
+{
+    unsigned long long x_used;
+    int max_out, max_terms, max_ent, x_over;
+};
+
 // Compiles the entry-major refill schedule of one tile (one CTA per tile, once per
 // pattern): the ES records of the tile's entries, one word per term (see TileDesc), and the
 // list section of the outputs with three or more terms: nlist + 1 headers
 // (output | first list item << 12) and the term indices of each such output in
-// upstream's visiting order.
-// COUNT pass: the numbers of term words and list-section words of every tile.
-// BUILD pass: writes everything at the offsets the scans of those numbers gave.
-template <bool BUILD>
+// upstream's visiting order. A tile's words start at its first row's term prefix; its
+// list section takes its words of X (x_cap of them) from a counter, so that one pass is
+// enough: counting them first, and searching for every term's entry and column again in
+// the second pass, one term of a thread at a time, took 325 us for 6.4M terms against
+// 107 us.
 __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
     NumArgs a, const unsigned char *__restrict__ rcls, const int *__restrict__ tile_start,
-    long long *__restrict__ tile_nterms, long long *__restrict__ tile_nx,
-    const long long *__restrict__ word_begin, const long long *__restrict__ x_begin,
-    TileDesc *__restrict__ tiles, unsigned *__restrict__ W, unsigned *__restrict__ X, int2 *__restrict__ ES)
+    const long long *__restrict__ term_pref, TileDesc *__restrict__ tiles, int *__restrict__ tile_nent,
+    unsigned *__restrict__ W, unsigned *__restrict__ X, long long x_cap, int2 *__restrict__ ES,
+    SchedTotals *__restrict__ totals)
 {
     extern __shared__ __align__(16) int bsm[];
+    __shared__ long long x_begin;
     BuildSmem t;
     t.cnt = bsm;
     t.cur = t.cnt + TILE_ACC;
-    t.row_cs = t.cur + TILE_ACC;
-    t.row_nr = t.row_cs + TILE_THREADS;
+    t.ci = t.cur + TILE_ACC;
+    t.tw = reinterpret_cast<unsigned *>(t.ci + TILE_ACC);
+    t.row_nr = reinterpret_cast<int *>(t.tw + TILE_ACC);
     t.row_ls = t.row_nr + TILE_THREADS;
     t.row_b = t.row_ls + TILE_THREADS;
     t.row_outoff = t.row_b + TILE_THREADS;
@@ -935,19 +974,20 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
     const int tid = threadIdx.x;
     const int tile = blockIdx.x;
     const int r0 = tile_start[tile], nrows = tile_start[tile + 1] - r0;
+    const int out0 = a.Cp[r0];
     for (int q = tid; q < TILE_ACC; q += TILE_THREADS) t.cnt[q] = 0;
+    if (tid == 0) t.misc[0] = 0;
     int nr = 0, ne = 0;
     if (tid < nrows)
     {
         const int r = r0 + tid;
         const int b = r / a.L_m, rr = r - b * a.L_m;
-        const int cs = a.Cp[r], ls = a.Lp[rr];
+        const int ls = a.Lp[rr];
         const int c = rcls[r];
-        if (c == NUM_TILE) nr = a.Cp[r + 1] - cs;
+        if (c == NUM_TILE) nr = a.Cp[r + 1] - a.Cp[r];
         // every L entry of the tile's rows up to a larger row (always the last row),
         // so that entry e of the tile is entry vbase + e
         if (c == NUM_TILE || c == 255) ne = a.Lp[rr + 1] - ls;
-        t.row_cs[tid] = cs;
         t.row_nr[tid] = nr;
         t.row_ls[tid] = ls;
         t.row_b[tid] = b;
@@ -971,20 +1011,22 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
         if (tid == 0) atomicOr(a.err, 2);
         return; // cannot happen with the tile weights; the host reports it
     }
+    for (int o = tid; o < total_out; o += TILE_THREADS) t.ci[o] = a.Ci[out0 + o];
     const int b0 = r0 / a.L_m;
     const int vb = b0 * a.L_nnz + a.Lp[r0 - b0 * a.L_m];
-    const long long wb = BUILD ? word_begin[tile] : 0, xb = BUILD ? x_begin[tile] : 0;
+    const long long wb = term_pref[r0];
 
-    // pass A: terms per output; the ES records of the entries
-    const int nterms = tile_terms(
-        a, t, nrows, total_raw,
-        [&](int e, int s, int toff, int len, int slot) {
-            if (BUILD && len > 0) ES[vb + e] = make_int2(s - toff, slot);
-            if (e >= (1 << 18) && len > 0) atomicOr(a.err, 2);
-        },
-        [&](bool valid, int, int, int o) {
-            if (valid) atomicAdd(&t.cnt[o], 1);
-        });
+    // terms per output; the ES records of the entries
+    int last_ent = 0;
+    const int nterms = tile_terms(a, t, nrows, total_raw, [&](int e, int s, int toff, int len, int slot) {
+        if (len > 0)
+        {
+            ES[vb + e] = make_int2(s - toff, slot);
+            last_ent = e + 1;
+            if (e >= (1 << 18)) atomicOr(a.err, 2);
+        }
+    });
+    atomicMax(&t.misc[0], last_ent);
     __syncthreads();
     // outputs with three or more terms: list index and first item
     int nlist = 0, nitems = 0;
@@ -994,13 +1036,17 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
         const int c = o < total_out ? t.cnt[o] : 0;
         if (o < total_out && c == 0) atomicOr(a.err, 1); // every output has a term
         const int m = c >= 3 ? 1 : 0;
+        if (!__syncthreads_or(m))
+        {
+            if (o < total_out) t.cur[o] = -1;
+            continue;
+        }
         const int im = block_incl_scan_int(m, t.scr);
         const int it = block_incl_scan_int(m ? c : 0, t.scr);
-        if (o < total_out)
-        {
-            t.cur[o] = m ? nitems + it - c : -1;
-            if (BUILD && m) X[xb + nlist + im - 1] = (unsigned)o | ((unsigned)(nitems + it - c) << 12);
-        }
+        // header words are written once the section's place is known: the list index
+        // beside the first item
+        if (o < total_out) t.cur[o] = m ? nitems + it - c : -1;
+        if (o < total_out && m) t.ci[o] = nlist + im - 1; // (the columns are no longer needed)
         if (tid == TILE_THREADS - 1)
         {
             t.misc[1] = im;
@@ -1011,62 +1057,66 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
         nitems += t.misc[2];
         __syncthreads();
     }
-    if (!BUILD)
-    {
-        if (tid == 0)
-        {
-            tile_nterms[tile] = nterms;
-            tile_nx[tile] = nlist ? nlist + 1 + nitems : 0;
-        }
-        return;
-    }
-    if (nlist && tid == 0) X[xb + nlist] = (unsigned)nitems << 12;
-    // pass B: the term words; the term indices of list outputs into their lists in
-    // visiting order (warps take turns, equal outputs inside a warp ranked by lane)
-    unsigned *xl = X + xb + nlist + 1;
-    const int warp = tid >> 5, lane = lane_id();
-    tile_terms(
-        a, t, nrows, total_raw, [&](int, int, int, int, int) {},
-        [&](bool valid, int e, int u, int o) {
-            bool listed = false;
-            if (valid)
-            {
-                const int c = t.cnt[o];
-                const unsigned kind = c == 1 ? TERM_ONE : (c == 2 ? TERM_PAIR : TERM_LIST);
-                W[wb + u] = ((unsigned)e << 14) | (kind << 12) | (unsigned)o;
-                listed = kind == TERM_LIST;
-            }
-            if (!nlist) return; // uniform over the block
-            for (int w = 0; w < TILE_THREADS / 32; ++w)
-            {
-                if (warp == w)
-                {
-                    const int key = listed ? o : -(lane + 1);
-                    const unsigned grp = __match_any_sync(FULL_MASK, key);
-                    int slot = 0;
-                    if (listed) slot = t.cur[o] + __popc(grp & lanemask_lt());
-                    __syncwarp();
-                    if (listed)
-                    {
-                        xl[slot] = (unsigned)u;
-                        if (lane == 31 - __clz(grp)) t.cur[o] += __popc(grp);
-                    }
-                }
-                __syncthreads();
-            }
-        });
     if (tid == 0)
     {
+        const long long nx = nlist ? (long long)nlist + 1 + nitems : 0;
+        long long xb = nx ? (long long)atomicAdd(&totals->x_used, (unsigned long long)nx) : 0;
+        if (xb + nx > x_cap)
+        {
+            totals->x_over = 1;
+            xb = -1;
+        }
+        x_begin = xb;
+        atomicMax(&totals->max_out, total_out);
+        atomicMax(&totals->max_terms, nterms);
+        atomicMax(&totals->max_ent, t.misc[0]);
+        tile_nent[tile] = t.misc[0];
         TileDesc dsc;
         dsc.vbase = vb;
         dsc.word_begin = (int)wb;
         dsc.nterms = nterms;
-        dsc.out_begin = t.row_cs[0];
+        dsc.out_begin = out0;
         dsc.nout = total_out;
         dsc.x_begin = nlist ? (int)xb : -1;
         dsc.nlist = nlist;
         dsc.prod = 0;
         tiles[tile] = dsc;
+    }
+    __syncthreads();
+    const long long xb = x_begin;
+    // the term words
+    for (int u = tid; u < nterms; u += TILE_THREADS)
+    {
+        const unsigned x = t.tw[u], o = x & ((1u << TW_BITS) - 1);
+        const int c = t.cnt[o];
+        const unsigned kind = c == 1 ? TERM_ONE : (c == 2 ? TERM_PAIR : TERM_LIST);
+        W[wb + u] = (x >> TW_BITS) << 14 | kind << 12 | o;
+    }
+    if (nlist == 0 || xb < 0) return; // (a section without a place: the build runs again)
+    for (int o = tid; o < total_out; o += TILE_THREADS)
+        if (t.cur[o] >= 0) X[xb + t.ci[o]] = (unsigned)o | ((unsigned)t.cur[o] << 12);
+    if (tid == 0) X[xb + nlist] = (unsigned)nitems << 12;
+    __syncthreads(); // the cursors move from here on
+    // the terms of list outputs into their lists in visiting order: a warp takes the terms
+    // 32 at a time, equal outputs ranked by lane
+    if (tid >= 32) return;
+    unsigned *xl = X + xb + nlist + 1;
+    for (int base = 0; base < nterms; base += 32)
+    {
+        const int u = base + tid;
+        const int o = u < nterms ? (int)(t.tw[u] & ((1u << TW_BITS) - 1)) : 0;
+        const bool listed = u < nterms && t.cnt[o] >= 3;
+        if (!__ballot_sync(FULL_MASK, listed)) continue;
+        const unsigned grp = __match_any_sync(FULL_MASK, listed ? o : -(tid + 1));
+        int slot = 0;
+        if (listed) slot = t.cur[o] + __popc(grp & lanemask_lt());
+        __syncwarp();
+        if (listed)
+        {
+            xl[slot] = (unsigned)u;
+            if (tid == 31 - __clz(grp)) t.cur[o] += __popc(grp);
+        }
+        __syncwarp();
     }
 }
 
@@ -2779,41 +2829,6 @@ __global__ void k_validate_schedule(const TileDesc *__restrict__ tiles, int ntil
     }
 }
 
-// Largest window (outputs) of the plan's tiles.
-__global__ void k_tile_max_out(const TileDesc *__restrict__ tiles, int ntiles, int *__restrict__ out)
-{
-    int m = 0;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < ntiles;
-         t += (long long)gridDim.x * blockDim.x)
-        m = max(m, tiles[t].nout);
-    atomicMax(out, m);
-}
-
-// Entries of every tile (its largest entry index + 1, from its term words; entry
-// indices grow along a tile's words) and the largest term and entry counts of a tile.
-__global__ void k_tile_nent(const TileDesc *__restrict__ tiles, int ntiles, const unsigned *__restrict__ W,
-                            int *__restrict__ nent, int *__restrict__ mx)
-{
-    const int lane = lane_id(), wpb = blockDim.x >> 5;
-    int mt = 0, me = 0;
-    for (long long t = blockIdx.x * (long long)wpb + (threadIdx.x >> 5); t < ntiles; t += (long long)gridDim.x * wpb)
-    {
-        const TileDesc D = tiles[t];
-        int e = -1;
-        for (int u = lane; u < D.nterms; u += 32) e = max(e, (int)(W[D.word_begin + u] >> 14));
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) e = max(e, __shfl_xor_sync(FULL_MASK, e, o));
-        if (lane == 0) nent[t] = e + 1;
-        mt = max(mt, D.nterms);
-        me = max(me, e + 1);
-    }
-    if (lane == 0)
-    {
-        atomicMax(&mx[0], mt);
-        atomicMax(&mx[1], me);
-    }
-}
-
 // Everything the refill needs once C's structure is known: row classes, the
 // compiled tile schedule and the larger rows' scratch.
 void build_schedule(const ProductDesc &d, Product &P, const long long *ub, cudaStream_t s)
@@ -2821,14 +2836,15 @@ void build_schedule(const ProductDesc &d, Product &P, const long long *ub, cudaS
     NvtxRange nvtx_range_("sdl: refill plan");
     Runtime &rt = runtime();
     const int m_out = P.m_out;
-    DevBuf<long long> weight(m_out), wpref((size_t)m_out + 1);
+    DevBuf<long long> weight(m_out), wpref((size_t)m_out + 1), tterms(m_out), tpref((size_t)m_out + 1);
     DevBuf<unsigned char> rcls(m_out);
     // rows with more terms than tile_max leave the tiles for the larger-row kernels
     const int tile_max = P.cfg.tile_max_terms > 0 ? std::min(TILE_T, P.cfg.tile_max_terms) : TILE_T;
     SDL_LAUNCH(k_num_classify, grid_for(m_out, 256, rt.num_sms * 8), 256, 0, s, ub, P.Cp.get(), d.Lp, d.L_m,
-               m_out, tile_max, rcls.get(), weight.get());
+               m_out, tile_max, rcls.get(), weight.get(), tterms.get());
     bin_items(rcls.get(), m_out, NUM_NBINS, P.num_rows, P.num_count, P.num_offset, s);
     exclusive_scan_i64(weight.get(), wpref.get(), m_out, s);
+    const long long word_total = exclusive_scan_i64(tterms.get(), tpref.get(), m_out, s);
     DevBuf<int> flag(m_out), tile_of((size_t)m_out + 1);
     const int budget = P.cfg.tile_budget > 0 ? std::max(TILE_T / 8, std::min(TILE_T, P.cfg.tile_budget)) : TILE_T;
     SDL_LAUNCH(k_tile_flags, grid_for(m_out, 256, rt.num_sms * 8), 256, 0, s, wpref.get(), m_out, budget,
@@ -2862,51 +2878,52 @@ void build_schedule(const ProductDesc &d, Product &P, const long long *ub, cudaS
         else
             value_order = 1;
     }
-    DevBuf<long long> tile_nterms(nt), tile_nx(nt), word_begin((size_t)nt + 1), x_begin((size_t)nt + 1);
     NumArgs na{d.Lp, d.Li, d.L_map, d.L_m, P.n_L, nullptr, nullptr, d.Ap, d.Ai, nullptr,
                P.Cp.get(), P.Ci.get(), nullptr, rt.d_error, d.L_nnz, value_order};
-    set_smem(k_tile_schedule<false>, build_smem_bytes());
-    set_smem(k_tile_schedule<true>, build_smem_bytes());
-    SDL_LAUNCH(k_tile_schedule<false>, P.ntiles, TILE_THREADS, build_smem_bytes(), s, na, rcls.get(),
-               tile_start.get(), tile_nterms.get(), tile_nx.get(), nullptr, nullptr, nullptr, nullptr,
-               nullptr, nullptr);
-    const long long word_total = exclusive_scan_i64(tile_nterms.get(), word_begin.get(), P.ntiles, s);
-    const long long x_total = exclusive_scan_i64(tile_nx.get(), x_begin.get(), P.ntiles, s);
-    if (word_total > INT_MAX || x_total > INT_MAX)
+    if (word_total > INT_MAX)
         fail(SDL_ERR_OVERFLOW, "product: the tile rows' terms exceed the schedule's 31-bit offsets");
     P.tiles.reset(nt);
+    P.tile_nent.reset(nt);
     // W and ES carry 16 bytes past their ends: the staged refill's bulk copies round
     // a tile's runs out to 16-byte boundaries
     P.W.reset(std::max<long long>(1, word_total) + 4);
-    P.X.reset(std::max<long long>(1, x_total));
     P.V.reset(std::max<long long>(1, nV));
     P.ES.reset(std::max<long long>(1, nV) + 2);
-    SDL_LAUNCH(k_tile_schedule<true>, P.ntiles, TILE_THREADS, build_smem_bytes(), s, na, rcls.get(),
-               tile_start.get(), nullptr, nullptr, word_begin.get(), x_begin.get(), P.tiles.get(),
-               P.W.get(), P.X.get(), P.ES.get());
-    if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "product plan: a term column is missing from its row");
-    if (P.ntiles > 0)
+    // the list sections, at most 4 words per 3 terms and one per tile: built in scratch
+    // (again where X_SCRATCH words were not enough), then copied to their exact size
+    constexpr long long X_SCRATCH = 64LL << 20;
+    long long x_cap = std::max<long long>(1, std::min<long long>(word_total / 3 * 4 + 4 + P.ntiles, X_SCRATCH));
+    DevBuf<SchedTotals> totals(1);
+    SchedTotals h{};
+    DevBuf<unsigned> xs;
+    while (P.ntiles > 0)
     {
+        xs.reset((size_t)x_cap);
+        SDL_CUDA(cudaMemsetAsync(totals.get(), 0, sizeof(SchedTotals), s));
+        SDL_LAUNCH(k_tile_schedule, P.ntiles, TILE_THREADS, build_smem_bytes(), s, na, rcls.get(), tile_start.get(),
+                   tpref.get(), P.tiles.get(), P.tile_nent.get(), P.W.get(), xs.get(), x_cap, P.ES.get(),
+                   totals.get());
+        SDL_CUDA(cudaMemcpyAsync(&h, totals.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+        SDL_CUDA(cudaStreamSynchronize(s));
+        if (!h.x_over) break;
+        x_cap = (long long)h.x_used;
+    }
+    const long long x_total = (long long)h.x_used;
+    if (x_total > INT_MAX)
+        fail(SDL_ERR_OVERFLOW, "product: the tile rows' terms exceed the schedule's 31-bit offsets");
+    P.X.reset(std::max<long long>(1, x_total));
+    if (x_total)
+        SDL_CUDA(cudaMemcpyAsync(P.X.get(), xs.get(), (size_t)x_total * sizeof(unsigned), cudaMemcpyDeviceToDevice, s));
+    P.max_tile_out = h.max_out;
+    P.max_tile_terms = h.max_terms;
+    P.max_tile_ent = h.max_ent;
+    if (P.ntiles > 0)
         SDL_LAUNCH(k_validate_schedule, grid_for(P.ntiles, 1, rt.num_sms * 8), 256, 0, s, P.tiles.get(), P.ntiles,
                    P.W.get(), word_total, P.X.get(), x_total, P.ES.get(), nV, (long long)d.A_nnz,
                    (long long)P.nnz, rt.d_error);
-        if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "product plan: the refill schedule failed its bounds check");
-        DevBuf<int> mo(1);
-        SDL_CUDA(cudaMemsetAsync(mo.get(), 0, sizeof(int), s));
-        SDL_LAUNCH(k_tile_max_out, grid_for(P.ntiles, 256, rt.num_sms * 4), 256, 0, s, P.tiles.get(), P.ntiles,
-                   mo.get());
-        SDL_CUDA(cudaMemcpyAsync(&P.max_tile_out, mo.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
-        P.tile_nent.reset((size_t)P.ntiles);
-        DevBuf<int> mx(2);
-        SDL_CUDA(cudaMemsetAsync(mx.get(), 0, mx.bytes(), s));
-        SDL_LAUNCH(k_tile_nent, grid_for(P.ntiles, 8, rt.num_sms * 8), 256, 0, s, P.tiles.get(), P.ntiles, P.W.get(),
-                   P.tile_nent.get(), mx.get());
-        int hmx[2] = {0, 0};
-        SDL_CUDA(cudaMemcpyAsync(hmx, mx.get(), sizeof(hmx), cudaMemcpyDeviceToHost, s));
-        SDL_CUDA(cudaStreamSynchronize(s));
-        P.max_tile_terms = hmx[0];
-        P.max_tile_ent = hmx[1];
-    }
+    const int bad_plan = take_device_error(s);
+    if (bad_plan & 3) fail(SDL_ERR_INTERNAL, "product plan: a term column is missing from its row");
+    if (bad_plan) fail(SDL_ERR_INTERNAL, "product plan: the refill schedule failed its bounds check");
     build_big_rows(P, ub, na, s);
     if (P.num_count[NUM_GMEM] && !P.big_lists)
     {
