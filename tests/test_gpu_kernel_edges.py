@@ -195,3 +195,35 @@ def test_large_row_windows_bit_exact(sdl, orc, kind, nL, nA, n, per_row):
         torch.cuda.synchronize()
         for o in out:
             assert np.array_equal(bits(o.cpu().numpy()), bits(wd))
+
+
+# ---------------------------------------------------------------- symbolic warp sorts
+# rows whose terms fill the sorted sizes (32, 64, 128, 256, 512) exactly, miss or exceed
+# them by one, with columns repeated inside a row or not at all; empty rows between
+@pytest.mark.parametrize("n", [40, 700, 100000])
+def test_row_sort_edges_bit_exact(sdl, orc, n):
+    import torch
+    from sparsediff_linalg_b200.device import Product
+    rng = np.random.default_rng(n)
+    want = [1, 2, 31, 32, 33, 0, 63, 64, 65, 127, 128, 129, 0, 0, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025]
+    rows = [np.unique(rng.integers(0, n, k)) for k in rng.integers(1, 30, 400)]
+    blens = np.array([len(r) for r in rows])
+    ent = []
+    for w in want:  # distinct rows of B whose lengths add up to w
+        left, mine = w, []
+        for k in rng.permutation(400):
+            if blens[k] <= left:
+                mine.append(k)
+                left -= blens[k]
+        ent.append(np.sort(np.array(mine, np.int64)))
+    Ap = np.concatenate([[0], np.cumsum([len(e) for e in ent])]).astype(np.int32)
+    Ai = np.concatenate(ent).astype(np.int32)
+    Bp = np.concatenate([[0], np.cumsum(blens)]).astype(np.int32)
+    Bi = np.concatenate(rows).astype(np.int32)
+    Ax, Bx = rng.standard_normal(len(Ai)), rng.standard_normal(len(Bi))
+    P = Product(T(Ap), T(Ai), T(Bp), T(Bi), n)
+    C = torch.full((P.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+    P.fill(T(Ax), None, T(Bx), C)
+    wp, wi, wx = orc.spgemm((Ap, Ai, Ax, len(want), 400), (Bp, Bi, Bx, 400, n))
+    assert np.array_equal(P.Cp.cpu().numpy(), wp) and np.array_equal(P.Ci.cpu().numpy(), wi)
+    assert np.array_equal(bits(C.cpu().numpy()), bits(wx))
