@@ -146,7 +146,7 @@ extern "C" sdl_status sdl_product_tuning(const sdl_product *P, int *warp_max_ter
         const TuneConfig &c = P->P.cfg;
         if (warp_max_terms) *warp_max_terms = c.warp_max_terms;
         if (rows_per_cta_warp) *rows_per_cta_warp = c.rows_per_cta_warp;
-        if (tile_budget) *tile_budget = c.tile_budget > 0 ? c.tile_budget : TILE_T;
+        if (tile_budget) *tile_budget = c.tile_budget > 0 ? c.tile_budget : TILE_BUDGET;
         if (refill_ctas_per_sm) *refill_ctas_per_sm = c.refill_ctas_per_sm;
         if (refill_us) *refill_us = P->tuned.refill_us;
         if (default_refill_us) *default_refill_us = P->tuned.default_refill_us;

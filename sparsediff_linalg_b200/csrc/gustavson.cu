@@ -177,8 +177,8 @@ __global__ void k_mask_classes(const unsigned char *__restrict__ mask, int m_out
 }
 
 // Numeric class, tile weight and terms in tiles of every output row. A tile row costs its terms,
-// one unit per 16 of its L entries and TILE_T / TILE_THREADS units; a larger row
-// costs TILE_T, so it always ends its tile. Rows with more than TILE_MAX_LROW L
+// one unit per 16 of its L entries and TILE_ROW_COST units; a larger row
+// costs TILE_BUDGET, so it always ends its tile. Rows with more than TILE_MAX_LROW L
 // entries never join a tile (the 18-bit entry index of a term word stays in range).
 constexpr int TILE_MAX_LROW = 131072;
 __global__ void k_num_classify(const long long *__restrict__ ub, const int *__restrict__ Cp,
@@ -205,13 +205,13 @@ __global__ void k_num_classify(const long long *__restrict__ ub, const int *__re
         else
             c = NUM_GMEM;
         cls[r] = (unsigned char)c;
-        const long long lw = (lenL + 15) / 16 + TILE_T / TILE_THREADS;
-        weight[r] = c == NUM_TILE ? u + lw : (c == 255 ? lw : TILE_T);
+        const long long lw = (lenL + 15) / 16 + TILE_ROW_COST;
+        weight[r] = c == NUM_TILE ? u + lw : (c == 255 ? lw : TILE_BUDGET);
         tterms[r] = c == NUM_TILE ? u : 0;
     }
 }
 
-// tile index of every row = floor(exclusive weight prefix / TILE_T); flag rows that
+// tile index of every row = floor(exclusive weight prefix / budget); flag rows that
 // start a tile
 __global__ void k_tile_flags(const long long *__restrict__ wpref, int m_out, int budget, int *__restrict__ flag)
 {
@@ -846,8 +846,8 @@ void compact_rows(const int *Cp, int m_out, int nnz, const long long *off0, cons
 
 // ------------------------------------------------------------ numeric kernels
 // ------------------------------------------------------------ row tiles
-// Outputs and terms of a tile are each below 2 * TILE_T.
-constexpr int TILE_ACC = 2 * TILE_T;
+// Outputs and terms of a tile are each below TILE_ACC.
+constexpr int TILE_ACC = TILE_BUDGET + TILE_T;
 
 // last index q in [0, n) with a[q] <= key (a non-decreasing, a[0] <= key)
 __device__ __forceinline__ int last_le(const int *a, int n, int key)
@@ -875,7 +875,7 @@ struct BuildSmem
     int *scr;
     int *misc; // [0]: entries up to the last with a term, [1]: list outputs of a chunk, [2]: their terms
 };
-constexpr int TW_BITS = 11; // an output of a tile
+constexpr int TW_BITS = 12; // an output of a tile
 static_assert(TILE_ACC <= 1 << TW_BITS, "a tile's outputs fit its packed terms");
 constexpr size_t build_smem_bytes()
 {
@@ -1250,10 +1250,6 @@ __global__ void __launch_bounds__(256) k_entry_values_batched(const EntChunk *__
 #ifndef SDL_REFILL_MINB
 #define SDL_REFILL_MINB 5
 #endif
-#ifndef SDL_REFILL_UNROLL
-#define SDL_REFILL_UNROLL 4
-#endif
-constexpr int RUNROLL = SDL_REFILL_UNROLL; // terms per thread whose loads are in flight together
 // Refill CTAs: 256 threads with windows of TILE_ACC outputs (every plan; the batched
 // refill), or 128 threads with windows of TILE_ACC / 2 for plans whose tiles have at
 // most that many outputs (tile budget and tile rows of at most TILE_T / 2 terms: a
@@ -1265,6 +1261,20 @@ template <int NT>
 __host__ __device__ constexpr int win_of()
 {
     return NT == REFILL_THREADS ? TILE_ACC : TILE_ACC / 2;
+}
+// Terms per thread whose loads are in flight together. A step of the 256-thread CTA
+// covers nearly every tile whole (1280 terms; a tile has TILE_BUDGET less its rows' costs,
+// give or take half a row): with tiles of a weight of 1024 and steps of 1024 terms, two
+// tiles in five took a second, nearly empty step, and more terms per tile spread its fixed
+// work further. B^T D A of 100000 x 50000 40.8 -> 37.1 us, 128 uneven products 1281 ->
+// 1160 us. Steps of 1280 with a weight of 1024: 38.8 and 1189 us; 1088: 39.4 and 1173;
+// 1184: 37.7 and 1154; 1248: 39.0 and 1153; steps of 1536: 39.1 and 1172. Windows of 2432
+// outputs, a sixth CTA or only four per SM: 45-48 and 1400-1600 us (the windows and L1
+// share the SM's memory).
+template <int NT>
+__host__ __device__ constexpr int runroll()
+{
+    return NT == REFILL_THREADS ? 5 : 4;
 }
 template <int NT>
 __host__ __device__ constexpr int refill_minb()
@@ -1395,10 +1405,10 @@ __device__ __forceinline__ bool rf_mbar_wait(unsigned long long *bar, unsigned p
 
 template <int NT>
 __device__ __forceinline__ void load_terms(const unsigned *__restrict__ W, int nterms, int base,
-                                           unsigned (&w)[RUNROLL])
+                                           unsigned (&w)[runroll<NT>()])
 {
 #pragma unroll
-    for (int j = 0; j < RUNROLL; ++j)
+    for (int j = 0; j < runroll<NT>(); ++j)
     {
         const int u = base + threadIdx.x + j * NT;
         w[j] = u < nterms ? W[u] : (TERM_LIST << 12); // a list word is skipped by the term pass
@@ -1496,7 +1506,7 @@ __global__ void __launch_bounds__(NT, refill_minb<NT>()) k_tile_refill(
     const int *__restrict__ tile_nent, int wcap, int ecap)
 {
     constexpr int WIN = win_of<NT>();
-    constexpr int RSTEP = RUNROLL * NT;
+    constexpr int RUNROLL = runroll<NT>(), RSTEP = RUNROLL * NT;
     extern __shared__ __align__(16) double rsm[];
     TileDesc *dsc = reinterpret_cast<TileDesc *>(rsm + 2 * WIN);
     ProdBase *bse = reinterpret_cast<ProdBase *>(dsc + 4);
@@ -2901,7 +2911,7 @@ void build_schedule(const ProductDesc &d, Product &P, const long long *ub, cudaS
     exclusive_scan_i64(weight.get(), wpref.get(), m_out, s);
     const long long word_total = exclusive_scan_i64(tterms.get(), tpref.get(), m_out, s);
     DevBuf<int> flag(m_out), tile_of((size_t)m_out + 1);
-    const int budget = P.cfg.tile_budget > 0 ? std::max(TILE_T / 8, std::min(TILE_T, P.cfg.tile_budget)) : TILE_T;
+    const int budget = P.cfg.tile_budget > 0 ? std::max(TILE_T / 8, std::min(TILE_BUDGET, P.cfg.tile_budget)) : TILE_BUDGET;
     SDL_LAUNCH(k_tile_flags, grid_for(m_out, 256, rt.num_sms * 8), 256, 0, s, wpref.get(), m_out, budget,
                flag.get());
     P.ntiles = exclusive_scan_i32_checked(flag.get(), tile_of.get(), m_out, s);
@@ -3797,9 +3807,9 @@ void product_replan(Product &P, const TuneConfig &c, cudaStream_t s)
 {
     if (c.refill_threads != REFILL_THREADS && c.refill_threads != REFILL_THREADS_SMALL)
         fail(SDL_ERR_INVALID, "refill threads must be 256 or 128");
-    if (c.tile_budget < 0 || c.tile_budget > TILE_T || c.tile_max_terms < 0 || c.tile_max_terms > TILE_T ||
+    if (c.tile_budget < 0 || c.tile_budget > TILE_BUDGET || c.tile_max_terms < 0 || c.tile_max_terms > TILE_T ||
         c.refill_ctas_per_sm < 0)
-        fail(SDL_ERR_INVALID, "tile budget / largest tile row must lie in [0, TILE_T]");
+        fail(SDL_ERR_INVALID, "tile budget / largest tile row must lie in [0, TILE_BUDGET] / [0, TILE_T]");
     if (P.m_out == 0) return;
     Runtime &rt = runtime();
     Product Q;
@@ -3891,14 +3901,14 @@ TuneResult product_autotune(Product &P, int reps, cudaStream_t s)
     TuneConfig best_cfg = base;
     bool have_best = false;
     Product best;
-    const int budgets[] = {TILE_T, 3 * TILE_T / 4, TILE_T / 2};
+    const int budgets[] = {TILE_BUDGET, 3 * TILE_T / 4, TILE_T / 2};
     const int ctas[] = {0, 4, 3};
     for (int b : budgets)
     {
         Product Q;
         TuneConfig c = sym_best;
-        c.tile_budget = b == TILE_T ? 0 : b;
-        if (b == TILE_T && (c.tile_budget == stage1.cfg.tile_budget))
+        c.tile_budget = b == TILE_BUDGET ? 0 : b;
+        if (b == TILE_BUDGET && (c.tile_budget == stage1.cfg.tile_budget))
             Q = std::move(stage1);
         else
             build(c, Q);

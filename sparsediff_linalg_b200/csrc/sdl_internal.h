@@ -236,15 +236,18 @@ enum
     NUM_GMEM, // larger rows: CTA per row, accumulator in C.x itself
     NUM_NBINS
 };
-// Term budget of a row tile. A tile row costs TILE_T / 256 extra units and a larger
-// row TILE_T, so a tile holds at most 256 rows, at most 2 * TILE_T terms and
-// outputs, and a larger row is always the last row of its tile (the outputs of a
-// tile's rows are one contiguous range of C).
-#ifndef SDL_TILE_T
-#define SDL_TILE_T 1024
+// Rows of at most TILE_T terms go into row tiles of a weight of TILE_BUDGET. A tile row
+// costs TILE_ROW_COST extra units and a larger row TILE_BUDGET, so a tile holds at most
+// 256 rows and fewer than TILE_BUDGET + TILE_T terms and outputs, and a larger row is
+// always the last row of its tile (the outputs of a tile's rows are one contiguous range
+// of C).
+#ifndef SDL_TILE_BUDGET
+#define SDL_TILE_BUDGET 1152
 #endif
-constexpr int TILE_T = SDL_TILE_T;
+constexpr int TILE_T = 1024;
+constexpr int TILE_BUDGET = SDL_TILE_BUDGET;
 constexpr int TILE_THREADS = 256;
+constexpr int TILE_ROW_COST = (TILE_BUDGET + TILE_THREADS - 1) / TILE_THREADS;
 
 // Compiled refill schedule of the tile rows (built once per pattern), entry-major:
 // the terms of a tile in upstream's visiting order (the tile's L entries in order,
@@ -305,7 +308,7 @@ struct TuneConfig
     int cta_threads_2k = 256;   // threads of the CTA kernel for rows up to 2048 terms
     int cta_threads_8k = 512;
     int gmem_threads = 512;
-    // refill: weight (terms plus per-row costs) of a row tile, at most TILE_T, and
+    // refill: weight (terms plus per-row costs) of a row tile, at most TILE_BUDGET, and
     // resident refill CTAs per SM (0: as many as fit)
     int tile_budget = 0; // 0: TILE_T
     int refill_ctas_per_sm = 0;

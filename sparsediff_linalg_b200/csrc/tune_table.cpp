@@ -36,7 +36,7 @@ bool valid(const TuneConfig &c)
     auto pos = [](int v) { return v > 0 && v <= 4096; };
     return (c.warp_max_terms == 128 || c.warp_max_terms == 512) && pos(c.rows_per_cta_warp) &&
            pos(c.cta_threads_2k) && pos(c.cta_threads_8k) && pos(c.gmem_threads) && c.tile_budget >= 0 &&
-           c.tile_budget <= TILE_T && c.tile_max_terms >= 0 && c.tile_max_terms <= TILE_T &&
+           c.tile_budget <= TILE_BUDGET && c.tile_max_terms >= 0 && c.tile_max_terms <= TILE_T &&
            c.refill_ctas_per_sm >= 0 && c.refill_ctas_per_sm <= 64 &&
            (c.refill_threads == 256 || c.refill_threads == 128) && (c.refill_pipe == 0 || c.refill_es == 0);
 }
