@@ -2193,7 +2193,7 @@ void bin_items(const unsigned char *d_cls, int n, int nbins, DevBuf<int> &lists,
     lists.reset(std::max(1, n));
     SDL_CUDA(cudaMemsetAsync(cnt.get(), 0, cnt.bytes(), s));
     SDL_LAUNCH(k_bin_count, grid_for(n, 256, rt.num_sms * 8), 256, 0, s, d_cls, n, nbins, cnt.get());
-    SDL_LAUNCH(k_bin_scatter, std::max(1, (n + BIN_TILE - 1) / BIN_TILE), 256, 0, s, d_cls, n, nbins, cnt.get(),
+    SDL_LAUNCH(k_bin_scatter, (unsigned)std::max(1LL, ((long long)n + BIN_TILE - 1) / BIN_TILE), 256, 0, s, d_cls, n, nbins, cnt.get(),
                cnt.get() + nbins, lists.get());
     SDL_CUDA(cudaMemcpyAsync(count, cnt.get(), nbins * sizeof(int), cudaMemcpyDeviceToHost, s));
     SDL_CUDA(cudaStreamSynchronize(s));

@@ -71,11 +71,12 @@ __device__ __forceinline__ int warp_row_of(const int *p, int lo, int hi, int e)
     const int lane = lane_id();
     while (hi - lo > 1)
     {
-        const int step = (hi - lo + 31) / 32, at = lo + step * lane; // p[lo] <= e: lane 0 holds
+        const int step = (int)(((long long)hi - lo + 31) / 32);
+        const long long at = lo + (long long)step * lane; // p[lo] <= e: lane 0 holds
         const unsigned le = __ballot_sync(FULL_MASK, at < hi && p[at] <= e);
         const int last = 31 - __clz(le);
         lo += step * last;
-        hi = min(hi, lo + step);
+        hi = (int)min((long long)hi, (long long)lo + step);
     }
     return lo;
 }
