@@ -109,7 +109,7 @@ void sdl_product_destroy(sdl_product *P);
 /* No upstream counterpart: autotuner. Re-plans P for its own pattern (structure
    and values are unchanged; only the schedule moves). Candidate symbolic bin
    thresholds (warp-kernel row limit 128 / 512 terms, 4 / 8 / 16 warps per CTA)
-   are timed on the pattern; then candidate tile budgets (TILE_T, 3/4, 1/2 of it)
+   are timed on the pattern; then candidate tile budgets (1152, 768, 512)
    and resident refill CTAs per SM (all that fit, 4, 3), and the small-tile
    refill (128-thread CTAs over tiles and tile rows of at most TILE_T / 2 terms),
    by `reps` refills each with placeholder values, L2 flushed before each; P keeps
@@ -125,7 +125,8 @@ sdl_status sdl_product_tuning(const sdl_product *P, int *warp_max_terms, int *ro
                               int *tile_budget, int *refill_ctas_per_sm, double *refill_us,
                               double *default_refill_us, int *candidates, double *tune_ms);
 /* Re-plans P with a given refill configuration (structure unchanged): tile budget
-   and largest tile row in terms (0: TILE_T = 1024), refill CTA threads (256, or 128:
+   (0: 1152, also the largest) and largest tile row in terms (0: TILE_T = 1024, also the
+   largest), refill CTA threads (256, or 128:
    used when every tile window fits the small-tile refill, i.e. budget and largest
    row at most 512), resident refill CTAs per SM (0: all that fit). The row offsets
    / column indices sdl_product_info returned before are released. Allocates;
