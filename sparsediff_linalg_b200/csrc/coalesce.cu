@@ -99,14 +99,27 @@ __global__ void __launch_bounds__(CS_THREADS) k_cs_count(const unsigned long lon
     }
 }
 
+// A run of row offsets of one value, [first, last] (rows up to INT_MAX, so both ends are
+// inclusive), that k_cs_emit leaves to k_cs_gaps.
+struct CsGap
+{
+    int first, last, value;
+};
+constexpr int CS_GAP = 1 << 16; // longest run that one warp writes, about 9 us
+__host__ __device__ constexpr long long cs_gap_cap(int m) { return 2 * (((long long)m + 1) / CS_GAP); }
+
 // Column and first triplet of every output, and the row offsets: the first output of a
-// row closes the rows between the previous output's row and its own (a warp shares the
-// long gaps), one past the last triplet the rows after it. A warp takes CS_ITEMS times
-// 32 consecutive triplets, so that an output's neighbours are written beside it.
+// row closes the rows between the previous output's row and its own, one past the last
+// triplet the rows after it. Runs of up to 8 rows are written by the lane that finds them,
+// of up to CS_GAP by its warp; longer ones are listed in gaps, cut into pieces of CS_GAP
+// rows, at most cs_gap_cap(m) in all (a run of CS_GAP + 1 rows or more gives at most two
+// pieces per CS_GAP rows). A warp takes CS_ITEMS times 32 consecutive triplets, so that an
+// output's neighbours are written beside it.
 __global__ void __launch_bounds__(CS_THREADS) k_cs_emit(const unsigned long long *__restrict__ keys, int n, int m,
                                                         int col_bits, const int *__restrict__ tile_first,
                                                         int *__restrict__ ostart, int *__restrict__ Ci,
-                                                        int *__restrict__ Cp)
+                                                        int *__restrict__ Cp, CsGap *__restrict__ gaps,
+                                                        int *__restrict__ ngaps)
 {
     __shared__ int part[CS_THREADS / 32];
     const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -138,31 +151,57 @@ __global__ void __launch_bounds__(CS_THREADS) k_cs_emit(const unsigned long long
     {
         const long long q = q0 + 32 * j;
         const int o = o0 + __popc(heads[j] & lanemask_lt());
-        int lo = 0, hi = 0; // Cp[lo .. hi) = o
+        long long lo = 0, hi = 0; // Cp[lo .. hi) = o (hi is up to 2^31)
         if ((heads[j] >> lane) & 1u)
         {
             ostart[o] = (int)q;
             Ci[o] = (int)(key[j] & cmask);
-            lo = q == 0 ? 0 : (int)(prev[j] >> col_bits) + 1;
-            hi = (int)(key[j] >> col_bits) + 1;
+            lo = q == 0 ? 0 : (long long)(prev[j] >> col_bits) + 1;
+            hi = (long long)(key[j] >> col_bits) + 1;
         }
         else if (q == n) // one past the last triplet
         {
             ostart[o] = n;
-            lo = (int)(prev[j] >> col_bits) + 1;
-            hi = m + 1;
+            lo = (long long)(prev[j] >> col_bits) + 1;
+            hi = (long long)m + 1;
         }
         unsigned longs = __ballot_sync(FULL_MASK, hi - lo > 8);
         if (hi - lo <= 8)
-            for (int r = lo; r < hi; ++r) Cp[r] = o;
+            for (long long r = lo; r < hi; ++r) Cp[r] = o;
         for (; longs; longs &= longs - 1)
         {
             const int l = __ffs(longs) - 1;
-            const int x = __shfl_sync(FULL_MASK, lo, l), y = __shfl_sync(FULL_MASK, hi, l);
+            const long long x = __shfl_sync(FULL_MASK, lo, l), y = __shfl_sync(FULL_MASK, hi, l);
             const int v = __shfl_sync(FULL_MASK, o, l);
-            for (int r = x + lane; r < y; r += 32) Cp[r] = v;
+            if (y - x <= CS_GAP)
+            {
+                for (long long r = x + lane; r < y; r += 32) Cp[r] = v;
+                continue;
+            }
+            const int pieces = (int)((y - x + CS_GAP - 1) / CS_GAP);
+            int at = 0;
+            if (lane == 0) at = atomicAdd(ngaps, pieces);
+            at = __shfl_sync(FULL_MASK, at, 0);
+            for (int p = lane; p < pieces; p += 32)
+            {
+                const long long r = x + (long long)p * CS_GAP;
+                gaps[at + p] = CsGap{(int)r, (int)(min(r + CS_GAP, y) - 1), v};
+            }
         }
         o0 += __popc(heads[j]);
+    }
+}
+
+// The long runs of row offsets, a CTA per piece. Written by the warp that found them, runs
+// took the build of 1M triplets in 10 rows out of 500M from 4.7 to 67 ms.
+__global__ void __launch_bounds__(CS_THREADS) k_cs_gaps(const CsGap *__restrict__ gaps, const int *__restrict__ ngaps,
+                                                        int *__restrict__ Cp)
+{
+    for (int g = blockIdx.x; g < *ngaps; g += gridDim.x)
+    {
+        const CsGap G = gaps[g];
+        const int rows = G.last - G.first + 1; // at most CS_GAP
+        for (int k = threadIdx.x; k < rows; k += CS_THREADS) Cp[(long long)G.first + k] = G.value;
     }
 }
 
@@ -473,8 +512,15 @@ int coalesce_build(const int *rows, const int *cols, int n, int m, int ncols, De
     if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "coalesce plan: the sort of the triplets did not finish");
     Ci.reset((size_t)std::max(1, nout));
     ostart.reset((size_t)nout + 1);
+    const long long gap_cap = cs_gap_cap(m);
+    DevBuf<CsGap> gaps((size_t)gap_cap);
+    DevBuf<int> ngaps(gap_cap ? 1 : 0);
+    if (gap_cap) SDL_CUDA(cudaMemsetAsync(ngaps.get(), 0, sizeof(int), s));
     SDL_LAUNCH(k_cs_emit, ntiles, CS_THREADS, 0, s, ka.get(), n, m, col_bits, first.get(), ostart.get(), Ci.get(),
-               Cp.get());
+               Cp.get(), gaps.get(), ngaps.get());
+    if (gap_cap)
+        SDL_LAUNCH(k_cs_gaps, (unsigned)std::min(gap_cap, 148LL * 8), CS_THREADS, 0, s, gaps.get(), ngaps.get(),
+                   Cp.get());
     if (n >= COALESCE_BUCKET_MIN) bucket_build(ostart.get(), perm.get(), n, nout, buckets, s);
     SDL_CUDA(cudaStreamSynchronize(s));
     return nout;

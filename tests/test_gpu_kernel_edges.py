@@ -83,6 +83,38 @@ def test_coalesce_sort_edges_bit_exact(sdl, orc, n, m, ncols, kind):
     assert np.array_equal(bits(Cx.cpu().numpy()), bits(wx))
 
 
+# runs of empty rows at, below and above the lengths that a lane (8 rows), a warp (65536)
+# and a CTA per piece of 65536 write, before the first output, between two and after the last
+@pytest.mark.parametrize("gap", [7, 8, 9, 65535, 65536, 65537, 131072, 131073, 200001])
+def test_coalesce_row_gaps(sdl, gap):
+    import torch
+    from sparsediff_linalg_b200.device import Coalesce
+    rows = np.repeat([gap, 2 * gap, 2 * gap + 1, 3 * gap + 2], [1, 40, 3, 5])
+    m = 4 * gap + 3
+    cols = np.arange(len(rows)) % 17
+    C = Coalesce(T(rows, torch.int32), T(cols, torch.int32), m, 17)
+    want = np.unique(rows.astype(np.int64) * 17 + cols)
+    wp = np.concatenate([[0], np.cumsum(np.bincount(want // 17, minlength=m))])
+    assert np.array_equal(C.Cp.cpu().numpy(), wp) and np.array_equal(C.Ci.cpu().numpy(), want % 17)
+
+
+# the largest row count there is: row offsets up to index 2^31 - 1, none of them left out
+def test_coalesce_largest_row_count(sdl):
+    import torch
+    from sparsediff_linalg_b200.device import Coalesce
+    m = 2**31 - 1
+    rows = [3, 3, 2**30, 2**30 + 9, m - 40, m - 2]
+    C = Coalesce(T(np.array(rows), torch.int32), T(np.arange(6), torch.int32), m, 6)
+    assert C.nnz == 6 and C.Cp.numel() == m + 1
+    at = 0
+    for r, before in [(3, 0), (2**30, 2), (2**30 + 9, 3), (m - 40, 4), (m - 2, 5), (m, 6)]:
+        run = C.Cp[at:r + 1]
+        assert run.numel() == r + 1 - at
+        assert int(run.min()) == before and int(run.max()) == before
+        at = r + 1
+    assert at == m + 1
+
+
 # ---------------------------------------------------------------- bucketed refill
 MIN = 10 << 20  # triplets from which a refill goes through buckets
 
