@@ -873,7 +873,9 @@ struct BuildSmem
     int *row_nr, *row_ls, *row_b, *row_outoff, *row_eoff;
     int *e_incl, *e_s, *e_len, *e_row;
     int *scr;
-    int *misc; // [0]: entries up to the last with a term, [1]: list outputs of a chunk, [2]: their terms
+    // [0]: entries up to the last with a term, [1]: list outputs of a chunk, [2]: their terms,
+    // [3]: set by a term that has no place among the tile's outputs
+    int *misc;
 };
 constexpr int TW_BITS = 12; // an output of a tile
 static_assert(TILE_ACC <= 1 << TW_BITS, "a tile's outputs fit its packed terms");
@@ -957,7 +959,7 @@ __device__ __forceinline__ int tile_terms(const NumArgs &a, const BuildSmem &t, 
                 if (uu >= total) continue;
                 if (w[q] == 0 || t.ci[lo[q]] != j[q] || cursor + uu >= TILE_ACC)
                 {
-                    atomicOr(a.err, 1);
+                    t.misc[3] = 1; // (its word is not written)
                     continue;
                 }
                 t.tw[cursor + uu] = (unsigned)(ec + el[q]) << TW_BITS | (unsigned)lo[q];
@@ -1031,7 +1033,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
     const int r0 = tile_start[tile], nrows = tile_start[tile + 1] - r0;
     const int out0 = a.Cp[r0];
     for (int q = tid; q < TILE_ACC; q += TILE_THREADS) t.cnt[q] = 0;
-    if (tid == 0) t.misc[0] = 0;
+    if (tid == 0) t.misc[0] = t.misc[3] = 0;
     int nr = 0, ne = 0;
     if (tid < nrows)
     {
@@ -1061,10 +1063,18 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
     }
     __syncthreads();
     const int total_out = t.row_outoff[nrows], total_raw = t.row_eoff[nrows];
-    if (total_out > TILE_ACC)
+    // A tile that does not fit, or whose terms do not match C's structure, is left empty:
+    // its words would lie outside their ranges. The host reports it.
+    const auto leave_empty = [&](int code) {
+        if (tid != 0) return;
+        atomicOr(a.err, code);
+        tile_nent[tile] = 0;
+        tiles[tile] = TileDesc{0, 0, 0, 0, 0, -1, 0, 0};
+    };
+    if (total_out > TILE_ACC) // cannot happen with the tile weights
     {
-        if (tid == 0) atomicOr(a.err, 2);
-        return; // cannot happen with the tile weights; the host reports it
+        leave_empty(2);
+        return;
     }
     for (int o = tid; o < total_out; o += TILE_THREADS) t.ci[o] = a.Ci[out0 + o];
     const int b0 = r0 / a.L_m;
@@ -1083,6 +1093,12 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
     });
     atomicMax(&t.misc[0], last_ent);
     __syncthreads();
+    // the operands changed since C's columns and the rows' terms were counted
+    if (t.misc[3] || nterms != term_pref[r0 + nrows] - wb)
+    {
+        leave_empty(1);
+        return;
+    }
     // outputs with three or more terms: list index and first item
     int nlist = 0, nitems = 0;
     for (int oc = 0; oc < total_out; oc += TILE_THREADS)

@@ -259,3 +259,38 @@ def test_row_sort_edges_bit_exact(sdl, orc, n):
     wp, wi, wx = orc.spgemm((Ap, Ai, Ax, len(want), 400), (Bp, Bi, Bx, 400, n))
     assert np.array_equal(P.Cp.cpu().numpy(), wp) and np.array_equal(P.Ci.cpu().numpy(), wi)
     assert np.array_equal(bits(C.cpu().numpy()), bits(wx))
+
+
+# ---------------------------------------------------------------- refill schedule
+# operands changed between the structure of C and its refill plan (columns that some rows of
+# C lack): the plan is refused, the error does not stick, and restored operands get their plan
+def test_schedule_of_changed_operands_is_refused(sdl):
+    import torch
+    from sparsediff_linalg_b200.device import Product
+    from sparsediff_linalg_b200.learned import LearnedFilledProduct, Mlp
+    rng = np.random.default_rng(5)
+    n, nA, nL = 5000, 900, 700
+    rows = [np.unique(rng.integers(0, n, k)) for k in rng.integers(1, 9, nA)]
+    Bp = T(np.concatenate([[0], np.cumsum([len(r) for r in rows])]), torch.int32)
+    good = T(np.concatenate(rows), torch.int32)
+    Bi = good.clone()
+    ent = [np.sort(rng.permutation(nA)[:k]) for k in rng.integers(1, 60, nL)]
+    Ap = T(np.concatenate([[0], np.cumsum([len(e) for e in ent])]), torch.int32)
+    Ai = T(np.concatenate(ent), torch.int32)
+    Ax = torch.randn(Ai.numel(), dtype=torch.float64, device="cuda")
+    Bx = torch.randn(Bi.numel(), dtype=torch.float64, device="cuda")
+    Q = LearnedFilledProduct(Ap, Ai, Bp, Bi, n, Mlp(seed=1), Ax, None, Bx)
+    Bi.copy_((good + 1) % n)
+    torch.cuda.synchronize()
+    with pytest.raises(Exception):
+        Q.complete_plan()
+    assert not Q.plan_ready()
+    Bi.copy_(good)
+    torch.cuda.synchronize()
+    Q.complete_plan()
+    P = Product(Ap, Ai, Bp, Bi, n)
+    cp, cq = (torch.full((P.nnz,), float("nan"), dtype=torch.float64, device="cuda") for _ in range(2))
+    P.fill(Ax, None, Bx, cp)
+    Q.fill(Ax, None, Bx, cq)
+    torch.cuda.synchronize()
+    assert torch.equal(P.Cp, Q.Cp) and torch.equal(cp.view(torch.int64), cq.view(torch.int64))
