@@ -229,6 +229,51 @@ def test_large_row_windows_bit_exact(sdl, orc, kind, nL, nA, n, per_row):
             assert np.array_equal(bits(o.cpu().numpy()), bits(wd))
 
 
+# outputs around the 64 terms that one thread puts in order, and of many more; in the same
+# product rows of over 32 terms per output (lists), tile rows and an empty row
+@pytest.mark.parametrize("n,hot", [(60000, (63, 64, 65, 3500)), (700, (66, 2000))])
+def test_large_row_many_terms_bit_exact(sdl, orc, n, hot):
+    import torch
+    from sparsediff_linalg_b200.device import Batch, Product
+    rng = np.random.default_rng(n + hot[0])
+    nA, few = 24000, 3000
+    # rows of A: a column of all the rows of one L row each (hot), and two others; the last
+    # ones over 50 columns only
+    rows = [np.unique(np.concatenate([[7], rng.integers(0, n, 2)])) for _ in range(nA - few)]
+    rows += [np.unique(rng.integers(0, 50, 3)) for _ in range(few)]
+    cold = [np.unique(rng.integers(8, n, 3)) for _ in range(1500)]  # without the hot column
+    rows += cold
+    Bp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    Bi = np.concatenate(rows).astype(np.int32)
+    ent = [np.concatenate([np.sort(rng.permutation(nA - few)[:k]), np.arange(nA, nA + 1500)]) for k in hot]
+    ent += [np.arange(nA - few, nA), np.array([], np.int64), np.array([5, 77, nA + 3])]
+    ent.append(np.arange(1, 2400))
+    Ap = np.concatenate([[0], np.cumsum([len(e) for e in ent])]).astype(np.int32)
+    Ai = np.concatenate(ent).astype(np.int32)
+    nL, nR = len(ent), len(rows)
+    P, Q = (Product(T(Ap), T(Ai), T(Bp), T(Bi), n) for _ in range(2))
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    batch = Batch([P, Q], stream=s)
+    for rnd in range(2):
+        Ax, Bx = rng.standard_normal(len(Ai)), rng.standard_normal(len(Bi))
+        Ax[::3] = -0.0
+        wp, wi, wx = orc.spgemm((Ap, Ai, Ax, nL, nR), (Bp, Bi, Bx, nR, n))
+        assert np.array_equal(P.Cp.cpu().numpy(), wp) and np.array_equal(P.Ci.cpu().numpy(), wi)
+        C = torch.full((P.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+        dev = [T(Ax), T(Bx)]
+        P.fill(dev[0], None, dev[1], C)
+        assert np.array_equal(bits(C.cpu().numpy()), bits(wx))
+        out = [torch.full((P.nnz,), float("nan"), dtype=torch.float64, device="cuda") for _ in range(2)]
+        for i in range(2):
+            batch.bind(i, dev[0], None, dev[1], out[i])
+        torch.cuda.synchronize()
+        batch.refill(stream=s)
+        torch.cuda.synchronize()
+        for o in out:
+            assert np.array_equal(bits(o.cpu().numpy()), bits(wx))
+
+
 # ---------------------------------------------------------------- symbolic warp sorts
 # rows whose terms fill the sorted sizes (32, 64, 128, 256, 512) exactly, miss or exceed
 # them by one, with columns repeated inside a row or not at all; empty rows between
