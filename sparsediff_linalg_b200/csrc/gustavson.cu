@@ -2321,12 +2321,13 @@ void validate_product(const ProductDesc &d, const TuneConfig &cfg, Product &P, c
 
 // ------------------------------------------------------------ rows beyond the tile budget
 // A row beyond the tile budget is refilled in windows: consecutive outputs with about
-// WIN_TARGET terms together (at most 2^WIN_BITS outputs and WIN_TERMS terms). A CTA
-// computes the window's products in upstream's visiting order -- so an entry's value is
-// read once for its run of terms, and a long row of A contiguously -- into shared memory,
-// and sums every output from there. Rows of more than WIN_MULT terms per output keep
-// output-major lists: at 20 terms per output the refill took 272 us against 506 us, at 48
-// 337 against 339 us.
+// WIN_TARGET terms together (at most 2^WIN_BITS outputs). A CTA computes the window's
+// products in upstream's visiting order -- so an entry's value is read once for its run of
+// terms, and a long row of A contiguously -- into shared memory, and sums every output from
+// there. A window of more than WIN_TERMS terms (a column common to many rows, columns that
+// crowd) is a chain of parts of WIN_TERMS terms: the outputs' sums go on from part to part.
+// Rows of more than WIN_MULT terms per output keep output-major lists: at 20 terms per output
+// the refill took 272 us against 506 us, at 48 337 against 339 us.
 constexpr int WIN_BITS = 11;
 constexpr int WIN_TERMS = 4096;
 constexpr int WIN_TARGET = 3072;
@@ -2442,11 +2443,18 @@ __global__ void k_win_max(const int *__restrict__ begin, int nwin, int *__restri
     if (lane_id() == 0) atomicMax(out, m);
 }
 
-// A CTA per window: its descriptor, and its terms' places output by output: counted out
-// with shared-memory adds, then every output's places put in order (visiting order), by a
-// thread for up to WIN_SORT of them; a warp looks the places of more up among the window's
-// terms. Sorted by one thread whatever their number, outputs of 3500 terms took the build
-// of a 15M-term product from 2.9 to 43 ms.
+// Part `part` of a window (WIN_TERMS terms from part * WIN_TERMS on): where its outputs'
+// entries of win_start begin, and the descriptor of the next part (0: none).
+struct WinPart
+{
+    int window, part, start, next;
+};
+
+// A CTA per descriptor (`parts`; null: every window is one part): the descriptor, and its
+// terms' places output by output: counted out with shared-memory adds, then every output's
+// places put in order (visiting order), by a thread for up to WIN_SORT of them; a warp looks
+// the places of more up among the part's terms. Sorted by one thread whatever their number,
+// outputs of 3500 terms took the build of a 15M-term product from 2.9 to 43 ms.
 constexpr int WIN_SORT = 64;
 __global__ void __launch_bounds__(WIN_THREADS) k_win_build(const int *__restrict__ rows, int nrows,
                                                            const int2 *__restrict__ wins,
@@ -2455,12 +2463,15 @@ __global__ void __launch_bounds__(WIN_THREADS) k_win_build(const int *__restrict
                                                            const uint2 *__restrict__ pairs, const int *__restrict__ Cp,
                                                            long long nA, long long nV, BigWindow *__restrict__ win,
                                                            const int *__restrict__ wout,
+                                                           const WinPart *__restrict__ parts,
                                                            unsigned short *__restrict__ terms,
                                                            unsigned short *__restrict__ start, int *__restrict__ err)
 {
     __shared__ int cur[1 << WIN_BITS], scr[32], row_sh, nmany;
     __shared__ unsigned short list[WIN_TERMS], many[WIN_TERMS / WIN_SORT];
-    const int w = blockIdx.x;
+    const int w0 = blockIdx.x;
+    const WinPart pt = parts ? parts[w0] : WinPart{w0, 0, wout[w0], 0};
+    const int w = pt.window;
     if (threadIdx.x == 0)
     {
         nmany = 0;
@@ -2482,7 +2493,8 @@ __global__ void __launch_bounds__(WIN_THREADS) k_win_build(const int *__restrict
     const int2 wn = wins[it];
     const int first = (w - wn.x) * wn.y; // of the row's outputs
     const int nout = min(wn.y, Cp[row + 1] - Cp[row] - first);
-    const int b = begin[w], n = begin[w + 1] - b;
+    const int b = begin[w] + pt.part * WIN_TERMS, left = begin[w + 1] - b, n = min(left, WIN_TERMS);
+    const bool whole = pt.part == 0 && left <= WIN_TERMS;
     for (int i = threadIdx.x; i < n; i += WIN_THREADS)
     {
         const uint2 q = pairs[b + i];
@@ -2496,10 +2508,12 @@ __global__ void __launch_bounds__(WIN_THREADS) k_win_build(const int *__restrict
     {
         c[k] = cur[threadIdx.x * PER + k];
         sum += c[k];
-        if ((c[k] > 0) != ((int)threadIdx.x * PER + k < nout)) atomicOr(err, 1); // every output has a term
+        // every output of a window has a term
+        const int o = threadIdx.x * PER + k;
+        if (o < nout ? whole && c[k] == 0 : c[k] > 0) atomicOr(err, 1);
     }
     int run = block_incl_scan_int(sum, scr) - sum;
-    const int s0 = wout[w];
+    const int s0 = pt.start;
 #pragma unroll
     for (int k = 0; k < PER; ++k)
     {
@@ -2545,7 +2559,7 @@ __global__ void __launch_bounds__(WIN_THREADS) k_win_build(const int *__restrict
     }
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += WIN_THREADS) terms[b + i] = list[i];
-    if (threadIdx.x == 0) win[w] = BigWindow{b, n, Cp[row] + first, nout, s0, 0};
+    if (threadIdx.x == 0) win[w0] = BigWindow{b, n, Cp[row] + first, nout, s0, pt.next};
 }
 
 // Refill of the windows, a CTA each. What bounds it: the latency of the gathers of V and
@@ -2556,68 +2570,79 @@ __global__ void __launch_bounds__(WIN_THREADS) k_win_build(const int *__restrict
 // (2.32 ms) or 8 (3.8 ms: spills), windows of 3072 terms rather than 1536 (2.73 ms) or
 // 6144 (3.2 ms), the second phase's lists fetched into L2 during the first (2.21 ms
 // without).
-template <bool BATCHED>
-__global__ void __launch_bounds__(WIN_THREADS, 6) k_win_refill(const BigWindow *__restrict__ win,
-                                                            const uint2 *__restrict__ pairs,
-                                                            const unsigned short *__restrict__ terms,
-                                                            const unsigned short *__restrict__ start,
-                                                            const ProdPtrs *__restrict__ vals_dev, ProdPtrs vals,
-                                                            const double *__restrict__ V)
+// CHAINS: the plan has windows in parts, which one CTA takes one after the other. With one
+// column in every row of A, 200 rows of 70000 terms take 270 us (2.48 ms by output-major
+// lists) and 600 rows of 24500 terms 181 us (1.11 ms), at five CTAs per SM for the loop's
+// registers (four: 260 and 203 us; six spill, and take a quarter longer).
+template <bool BATCHED, bool CHAINS>
+__global__ void __launch_bounds__(WIN_THREADS, CHAINS ? 5 : 6) k_win_refill(
+    const BigWindow *__restrict__ win, const uint2 *__restrict__ pairs, const unsigned short *__restrict__ terms,
+    const unsigned short *__restrict__ start, const ProdPtrs *__restrict__ vals_dev, ProdPtrs vals,
+    const double *__restrict__ V)
 {
     extern __shared__ double wsm[];
-    const BigWindow D = win[blockIdx.x];
     ProdPtrs P = vals;
     if (BATCHED) P = *vals_dev;
     const double *Vp = (P.Lx || P.d) ? V : nullptr;
     const double *__restrict__ Ax = P.Ax;
-    const unsigned short *st = start + D.start, *tm = terms + D.pairs;
-    if (threadIdx.x == 0)
-    {
-        prefetch_l2(tm, tm + D.nterms);
-        prefetch_l2(st, st + D.nout + 1);
-    }
     constexpr int U = 4; // terms and outputs of a thread whose loads are in flight together
-    const uint2 *pr = pairs + D.pairs;
-    for (int i0 = threadIdx.x; i0 < D.nterms; i0 += U * WIN_THREADS)
+    for (int k = blockIdx.x;;)
     {
-        uint2 q[U];
+        const BigWindow D = win[k];
+        const unsigned short *st = start + D.start, *tm = terms + D.pairs;
+        if (threadIdx.x == 0)
+        {
+            prefetch_l2(tm, tm + D.nterms);
+            prefetch_l2(st, st + D.nout + 1);
+        }
+        const uint2 *pr = pairs + D.pairs;
+        for (int i0 = threadIdx.x; i0 < D.nterms; i0 += U * WIN_THREADS)
+        {
+            uint2 q[U];
 #pragma unroll
-        for (int j = 0; j < U; ++j)
-            if (i0 + j * WIN_THREADS < D.nterms) q[j] = __ldcs(pr + i0 + j * WIN_THREADS);
-        double v[U], x[U];
+            for (int j = 0; j < U; ++j)
+                if (i0 + j * WIN_THREADS < D.nterms) q[j] = __ldcs(pr + i0 + j * WIN_THREADS);
+            double v[U], x[U];
 #pragma unroll
-        for (int j = 0; j < U; ++j)
-            if (i0 + j * WIN_THREADS < D.nterms)
+            for (int j = 0; j < U; ++j)
+                if (i0 + j * WIN_THREADS < D.nterms)
+                {
+                    v[j] = Vp ? Vp[q[j].y] : 1.0;
+                    x[j] = Ax[q[j].x];
+                }
+#pragma unroll
+            for (int j = 0; j < U; ++j)
+                if (i0 + j * WIN_THREADS < D.nterms) wsm[i0 + j * WIN_THREADS] = __dmul_rn(v[j], x[j]);
+        }
+        __syncthreads();
+        double *C = P.Cx + D.out;
+        for (int o0 = threadIdx.x; o0 < D.nout; o0 += U * WIN_THREADS)
+        {
+            int a[U], e[U], l[U];
+#pragma unroll
+            for (int j = 0; j < U; ++j)
             {
-                v[j] = Vp ? Vp[q[j].y] : 1.0;
-                x[j] = Ax[q[j].x];
+                const int o = o0 + j * WIN_THREADS;
+                a[j] = o < D.nout ? st[o] : 0;
+                e[j] = o < D.nout ? st[o + 1] : 0;
             }
 #pragma unroll
-        for (int j = 0; j < U; ++j)
-            if (i0 + j * WIN_THREADS < D.nterms) wsm[i0 + j * WIN_THREADS] = __dmul_rn(v[j], x[j]);
-    }
-    __syncthreads();
-    double *C = P.Cx + D.out;
-    for (int o0 = threadIdx.x; o0 < D.nout; o0 += U * WIN_THREADS)
-    {
-        int a[U], e[U], l[U];
+            for (int j = 0; j < U; ++j) l[j] = a[j] < e[j] ? tm[a[j]] : 0;
 #pragma unroll
-        for (int j = 0; j < U; ++j)
-        {
-            const int o = o0 + j * WIN_THREADS;
-            a[j] = o < D.nout ? st[o] : 0;
-            e[j] = o < D.nout ? st[o + 1] : 0;
+            for (int j = 0; j < U; ++j)
+            {
+                const int o = o0 + j * WIN_THREADS;
+                if (CHAINS ? o >= D.nout : a[j] >= e[j]) continue;
+                // (a further part goes on from the sum that this thread stored)
+                double acc = CHAINS && k != (int)blockIdx.x ? C[o] : 0.0;
+                if (!CHAINS || a[j] < e[j]) acc = __dadd_rn(acc, wsm[l[j]]);
+                for (int i = a[j] + 1; i < e[j]; ++i) acc = __dadd_rn(acc, wsm[tm[i]]);
+                __stcs(C + o, acc);
+            }
         }
-#pragma unroll
-        for (int j = 0; j < U; ++j) l[j] = a[j] < e[j] ? tm[a[j]] : 0;
-#pragma unroll
-        for (int j = 0; j < U; ++j)
-        {
-            if (a[j] >= e[j]) continue;
-            double acc = __dadd_rn(0.0, wsm[l[j]]);
-            for (int i = a[j] + 1; i < e[j]; ++i) acc = __dadd_rn(acc, wsm[tm[i]]);
-            __stcs(C + o0 + j * WIN_THREADS, acc);
-        }
+        if (!CHAINS || !D.next) break;
+        k = D.next;
+        __syncthreads(); // the part's products are summed
     }
 }
 
@@ -2709,6 +2734,7 @@ template <class E>
 DevBuf<E> to_device(const std::vector<E> &v, cudaStream_t s)
 {
     DevBuf<E> d(v.size());
+    if (v.empty()) return d;
     SDL_CUDA(cudaMemcpyAsync(d.get(), v.data(), v.size() * sizeof(E), cudaMemcpyHostToDevice, s));
     return d;
 }
@@ -2748,9 +2774,8 @@ int bits_for(long long v) // of the values 0 .. v - 1
     return b;
 }
 
-// Windows of the rows B (false: a window holds more than WIN_TERMS terms, or there are
-// too many). The windows of a row have about WIN_TARGET >> halve terms.
-bool build_windows(Product &P, const BigRows &B, int halve, const NumArgs &na, cudaStream_t s)
+// Windows of the rows B (false: there are too many).
+bool build_windows(Product &P, const BigRows &B, const NumArgs &na, cudaStream_t s)
 {
     Runtime &rt = runtime();
     const int nb = B.n();
@@ -2759,7 +2784,7 @@ bool build_windows(Product &P, const BigRows &B, int halve, const NumArgs &na, c
     long long starts = 0, nwin = 0;
     for (int i = 0; i < nb; ++i)
     {
-        const long long want = (long long)(WIN_TARGET >> halve) * B.outs[i] / std::max(1LL, B.terms[i]);
+        const long long want = (long long)WIN_TARGET * B.outs[i] / std::max(1LL, B.terms[i]);
         const int width = (int)std::max(1LL, std::min<long long>(want, 1 << WIN_BITS));
         wins[i] = make_int2((int)nwin, width);
         const long long k = (B.outs[i] + width - 1) / width;
@@ -2796,17 +2821,47 @@ bool build_windows(Product &P, const BigRows &B, int halve, const NumArgs &na, c
     int most = 0;
     SDL_CUDA(cudaMemcpyAsync(&most, largest.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
     SDL_CUDA(cudaStreamSynchronize(s));
+    // Where windows have more than WIN_TERMS terms: their first parts come before the other
+    // windows, the longest first (their sums are the refill's longest chains), their further
+    // parts after them.
+    std::vector<WinPart> parts;
     if (most > WIN_TERMS)
     {
-        P.win_pairs.release();
-        return false;
+        std::vector<int> hb((size_t)W + 1), chained;
+        SDL_CUDA(cudaMemcpyAsync(hb.data(), begin.get(), hb.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+        SDL_CUDA(cudaStreamSynchronize(s));
+        const auto size = [&](int w) { return hb[w + 1] - hb[w]; };
+        for (int w = 0; w < W; ++w)
+            if (size(w) > WIN_TERMS) chained.push_back(w);
+        std::stable_sort(chained.begin(), chained.end(), [&](int x, int y) { return size(x) > size(y); });
+        for (int w : chained) parts.push_back(WinPart{w, 0, wout[w], 0});
+        for (int w = 0; w < W; ++w)
+            if (size(w) <= WIN_TERMS) parts.push_back(WinPart{w, 0, wout[w], 0});
+        const long long starts0 = starts;
+        for (size_t c = 0; c < chained.size(); ++c)
+        {
+            const int w = chained[c];
+            const long long entries = (w + 1 < W ? wout[w + 1] : starts0) - wout[w];
+            size_t last = c;
+            for (int part = 1; (long long)part * WIN_TERMS < size(w); ++part)
+            {
+                if (starts + entries > INT_MAX) return false;
+                parts[last].next = (int)parts.size();
+                last = parts.size();
+                parts.push_back(WinPart{w, part, (int)starts, 0});
+                starts += entries;
+            }
+        }
+        most = WIN_TERMS;
     }
-    P.win.reset(W);
+    const int ndesc = parts.empty() ? W : (int)parts.size();
+    const DevBuf<WinPart> dparts = to_device(parts, s);
+    P.win.reset(ndesc);
     P.win_terms.reset(T);
     P.win_start.reset((size_t)starts);
-    SDL_LAUNCH(k_win_build, W, WIN_THREADS, 0, s, rows.get(), nb, dwins.get(), begin.get(), keys.get(),
+    SDL_LAUNCH(k_win_build, ndesc, WIN_THREADS, 0, s, rows.get(), nb, dwins.get(), begin.get(), keys.get(),
                P.win_pairs.get(), P.Cp.get(), (long long)P.desc.A_nnz, (long long)P.desc.L_nnz * P.desc.blocks,
-               P.win.get(), dwout.get(), P.win_terms.get(), P.win_start.get(), rt.d_error);
+               P.win.get(), dwout.get(), dparts.get(), P.win_terms.get(), P.win_start.get(), rt.d_error);
     if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "product plan: heavy-row windows are inconsistent");
     P.nwin = W;
     P.win_most = most;
@@ -2868,9 +2923,7 @@ void build_big_rows(Product &P, const long long *ub, const NumArgs &na, cudaStre
         (ht[i] <= WIN_MULT * ho[i] ? W : L).add(hr[i], ht[i], ho[i]);
     }
     if (T >= INT_MAX || O >= INT_MAX || T < O) return; // the CTA kernels handle them
-    bool windows = W.n() == 0;
-    for (int halve = 0; halve <= 2 && !windows; ++halve) windows = build_windows(P, W, halve, na, s);
-    if (!windows)
+    if (W.n() && !build_windows(P, W, na, s))
         for (int i = 0; i < W.n(); ++i) L.add(W.rows[i], W.terms[i], W.outs[i]);
     if (L.n()) build_lists(P, L, na, s);
     SDL_CUDA(cudaStreamSynchronize(s));
@@ -3806,12 +3859,11 @@ void big_lists_refill(const Product &P, const ProdPtrs *ptrs, cudaStream_t s, Pr
     if (P.nwin)
     {
         const size_t sm = (size_t)P.win_most * sizeof(double);
-        if (ptrs)
-            SDL_LAUNCH(k_win_refill<true>, P.nwin, WIN_THREADS, sm, s, P.win.get(), P.win_pairs.get(),
-                       P.win_terms.get(), P.win_start.get(), ptrs, vals, V);
-        else
-            SDL_LAUNCH(k_win_refill<false>, P.nwin, WIN_THREADS, sm, s, P.win.get(), P.win_pairs.get(),
-                       P.win_terms.get(), P.win_start.get(), ptrs, vals, V);
+        const bool chains = P.win.n > (size_t)P.nwin;
+        const auto kern = ptrs ? (chains ? k_win_refill<true, true> : k_win_refill<true, false>)
+                               : (chains ? k_win_refill<false, true> : k_win_refill<false, false>);
+        SDL_LAUNCH(kern, P.nwin, WIN_THREADS, sm, s, P.win.get(), P.win_pairs.get(), P.win_terms.get(),
+                   P.win_start.get(), ptrs, vals, V);
     }
     if (P.big_outputs == 0) return;
     const int grid = (P.big_outputs + 255) / 256;

@@ -346,12 +346,14 @@ struct ProductDesc
     int A_m = 0, A_n = 0, A_nnz = 0;
 };
 
-// Outputs [out, out + nout) of C, of one row beyond the tile budget.
+// Outputs [out, out + nout) of C, of one row beyond the tile budget: all of their terms,
+// or one part of them after the other.
 struct BigWindow
 {
     int pairs, nterms; // its pairs
     int out, nout;
-    int start, pad; // its outputs' entries of win_start (nout + 1)
+    int start; // its outputs' entries of win_start (nout + 1)
+    int next;  // the window's next part (0: none), whose sums go on from this one's
 };
 struct Product
 {
@@ -380,7 +382,8 @@ struct Product
     // Windows: a few thousand terms of consecutive outputs of one row, its pairs in
     // upstream's visiting order; per output its terms' places in the window.
     bool big_lists = false;
-    int nwin = 0, win_most = 0; // win_most: terms of the largest window
+    // (The first nwin entries of win are the windows, any others their further parts.)
+    int nwin = 0, win_most = 0; // win_most: terms of the largest window or part
     DevBuf<BigWindow> win;
     DevBuf<uint2> win_pairs;
     DevBuf<unsigned short> win_terms; // the terms' places, output by output

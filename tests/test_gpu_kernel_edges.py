@@ -229,9 +229,12 @@ def test_large_row_windows_bit_exact(sdl, orc, kind, nL, nA, n, per_row):
             assert np.array_equal(bits(o.cpu().numpy()), bits(wd))
 
 
-# outputs around the 64 terms that one thread puts in order, and of many more; in the same
-# product rows of over 32 terms per output (lists), tile rows and an empty row
-@pytest.mark.parametrize("n,hot", [(60000, (63, 64, 65, 3500)), (700, (66, 2000))])
+# outputs around the 64 terms that one thread puts in order, and of many more: windows of more
+# terms than one part holds (4096), where one output's terms end a part exactly, miss or
+# exceed it by one, or take several parts; in the same product rows of over 32 terms per
+# output (lists), tile rows and an empty row
+@pytest.mark.parametrize("n,hot", [(60000, (63, 64, 65, 3500)), (700, (66, 2000)), (60000, (4095, 4096, 4097)),
+                                   (60000, (8192, 8193, 20000)), (700, (5000, 12289))])
 def test_large_row_many_terms_bit_exact(sdl, orc, n, hot):
     import torch
     from sparsediff_linalg_b200.device import Batch, Product
