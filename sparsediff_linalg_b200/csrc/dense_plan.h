@@ -27,6 +27,12 @@ struct BlkTile
     int blk, c0;
 };
 
+// Rows and columns of a source block that a CTA transposes: 32 of each from i0, r0 on.
+struct BlkTrTile
+{
+    int blk, i0, r0;
+};
+
 // Rows [i0, i0 + nrow) of an output block, kept in shared memory while the block's
 // units of output columns (unit_begin .. unit_end, counted over all slabs of the class)
 // are computed.
@@ -53,7 +59,8 @@ struct BlocksCsrPlan
     DevBuf<int> cp, rows, pos;
     DevBuf<double> vals; // S.x gathered in compact order (refill scratch)
     DevBuf<double> BT;   // the source blocks transposed (refill scratch)
-    int tr_x = 0, tr_y = 0; // transpose grid: 32 x 32 tiles of the largest block
+    DevBuf<BlkTrTile> tr; // every output block's source in 32 x 32 tiles
+    int ntr = 0;
     DevBuf<BlkDesc> desc;
     DevBuf<BlkTile> tiles;
     int ntiles = 0;

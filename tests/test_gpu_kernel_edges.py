@@ -56,6 +56,40 @@ def test_blocks_csr_slab_edges_bit_exact(sdl, orc, m0, n0, S_n, dens):
     assert at == P.c_values
 
 
+# blocks whose largest row count and largest column count are not the same block's (64000 x
+# 4000 tiles of 32 x 32 between them, nine blocks: more than a launch can have), beside
+# small ones and one without output columns
+def test_blocks_csr_uneven_shapes_bit_exact(sdl, orc):
+    import torch
+    from sparsediff_linalg_b200.device import BlocksCsr
+    rng = np.random.default_rng(8)
+    S_m, S_n = 2048000, 40
+    at = np.sort(rng.permutation(S_m)[:300])
+    at[:2] = [0, 7]
+    Si = rng.integers(0, S_n, len(at)).astype(np.int32)
+    Sp = np.zeros(S_m + 1, np.int32)
+    Sp[at + 1] = 1
+    Sp = np.cumsum(Sp).astype(np.int32)
+    Sx = rng.standard_normal(len(at))
+    blocks = [(rng.standard_normal((1, S_m)), np.arange(S_m, dtype=np.int32)),
+              (rng.standard_normal((128000, 1)), np.array([7], np.int32)),
+              (rng.standard_normal((5, 3)), np.array([1, 2, 3], np.int32))]
+    blocks += [(rng.standard_normal((9, 40)), np.sort(rng.permutation(at)[:40]).astype(np.int32)) for _ in range(7)]
+    P = BlocksCsr([X.shape[0] for X, _ in blocks], [X.shape[1] for X, _ in blocks], [c for _, c in blocks], Sp, Si,
+                  S_m, S_n)
+    Cv = torch.full((P.c_values,), float("nan"), dtype=torch.float64, device="cuda")
+    P.fill(T(np.concatenate([X.ravel() for X, _ in blocks])), T(Sx), Cv)
+    got = Cv.cpu().numpy()
+    want = orc.blocks_csr(blocks, Sp, Si, Sx, S_n)
+    at = 0
+    for src, mk, nk, perm in P.blocks:
+        cols, Cw = want[src]
+        assert np.array_equal(perm, cols) and Cw.shape == (mk, nk)
+        assert np.array_equal(bits(got[at:at + mk * nk]), bits(Cw.ravel()))
+        at += mk * nk
+    assert at == P.c_values
+
+
 # ---------------------------------------------------------------- sorting triplets
 # sizes around a sort tile (3072 pairs) and a structure tile (2048); matrices whose keys
 # take one digit pass up to seven, one cell only (every key equal), rows in order, and a
