@@ -96,6 +96,11 @@ constexpr int RS_WARPS = 16; // warps of a CTA
 constexpr int RS_COLS = 16;  // output columns of a unit
 constexpr int RS_SHIFT = 3;  // columns a unit may start early, to meet C's 32-byte sectors
 constexpr int RS_REC = 128;  // records a warp stages at once
+// The CTAs share the units out by their cost: a unit's stores and fixed work take about as
+// long as 128 terms (16 blocks of 64 x 256 times 256 x 8000: 38 us at one entry per column,
+// 58 at 12, 130 at 40, 261 at 100). With an even share of the units each, a tenth of the
+// columns at 100 entries and the others at 2 took 238 us, 64 us so (147 by k_blocks_csr).
+constexpr int RS_UNIT_COST = 128;
 constexpr int RS_SLAB_BYTES = 128 * 1024;
 constexpr int RS_N0_MAX = RS_SLAB_BYTES / (32 * 8);
 constexpr int RS_WARP_BYTES = 2 * RS_REC * 16; // two units' records
@@ -193,7 +198,7 @@ __device__ __forceinline__ void rs_unit(const char *Bq, int4 *recs, bool whole, 
 // Slabs of 16 * (Q - 1) + 1 .. 16 * Q rows.
 template <int Q>
 __global__ void __launch_bounds__(RS_WARPS * 32, Q <= 2 ? 2 : 1) k_blocks_csr_slabs(
-    const BlkSlab *__restrict__ slabs, const int *__restrict__ first_slab, long long units, int slab_smem,
+    const BlkSlab *__restrict__ slabs, const BlkShare *__restrict__ shares, int slab_smem,
     const int *__restrict__ cp_all, const int *__restrict__ rows_all,
     const double *__restrict__ vals_all, const double *__restrict__ BT_vals, double *__restrict__ C_vals)
 {
@@ -201,10 +206,10 @@ __global__ void __launch_bounds__(RS_WARPS * 32, Q <= 2 ? 2 : 1) k_blocks_csr_sl
     const int lane = lane_id(), warp = threadIdx.x >> 5;
     double *Bs = reinterpret_cast<double *>(rs_smem);
     int4 *recs = reinterpret_cast<int4 *>(rs_smem + slab_smem + warp * RS_WARP_BYTES);
-    // this CTA's even share of the units, contiguous: it loads few slabs
-    long long u = units * blockIdx.x / gridDim.x;
-    const long long u_end = units * (blockIdx.x + 1) / gridDim.x;
-    for (int si = first_slab[blockIdx.x]; u < u_end; ++si)
+    // this CTA's share of the units, contiguous: it loads few slabs
+    long long u = shares[blockIdx.x].unit;
+    const long long u_end = shares[blockIdx.x + 1].unit;
+    for (int si = shares[blockIdx.x].slab; u < u_end; ++si)
     {
         const BlkSlab sl = slabs[si];
         const BlkDesc &D = sl.D;
@@ -274,8 +279,61 @@ __global__ void __launch_bounds__(RS_WARPS * 32, Q <= 2 ? 2 : 1) k_blocks_csr_sl
     }
 }
 
-using SlabKernel = void (*)(const BlkSlab *, const int *, long long, int, const int *, const int *, const double *,
+using SlabKernel = void (*)(const BlkSlab *, const BlkShare *, int, const int *, const int *, const double *,
                             const double *, double *);
+// The first unit of each CTA, of at most `grid`, and one past the last (cp: the compact CSCs'
+// column offsets). A CTA begins where the cost of the units before reaches its part of the
+// whole. Where that is less than a unit per warp, a second slab would cost it more than its
+// units do: each slab is then shared out among CTAs of its own (16 blocks of 64 x 256 times
+// 256 x 500: 16.6 -> 12.7 us).
+std::vector<BlkShare> share_units(const std::vector<BlkSlab> &slabs, const int *cp, int grid)
+{
+    // cost of the slab's first k units, and of all of them
+    const auto cost = [&](const BlkSlab &S, long long k) {
+        return k * RS_UNIT_COST + cp[S.D.cp_off + std::min<long long>(k * RS_COLS, S.D.n0_C)];
+    };
+    const auto all = [&](const BlkSlab &S) { return cost(S, S.unit_end - S.unit_begin); };
+    // the slab's first unit that `from` or more cost comes before
+    const auto unit_at = [&](const BlkSlab &S, long long from) {
+        long long lo = 0, hi = S.unit_end - S.unit_begin;
+        while (lo < hi)
+        {
+            const long long mid = (lo + hi) / 2;
+            if (cost(S, mid) < from)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        return S.unit_begin + lo;
+    };
+    long long total = 0;
+    for (const BlkSlab &S : slabs) total += all(S);
+    const auto part = [](long long whole, long long k, long long n) { return (long long)((__int128)whole * k / n); };
+    std::vector<BlkShare> out;
+    if ((long long)slabs.size() <= grid && slabs.back().unit_end < (long long)grid * RS_WARPS)
+    {
+        for (size_t si = 0; si < slabs.size(); ++si)
+        {
+            const BlkSlab &S = slabs[si];
+            const long long n = std::max(1LL, std::min(part(grid, all(S), total), S.unit_end - S.unit_begin));
+            for (long long k = 0; k < n; ++k) out.push_back(BlkShare{unit_at(S, part(all(S), k, n)), (int)si, 0});
+        }
+    }
+    else
+    {
+        size_t si = 0;
+        long long before = 0; // cost of the slabs before slab si
+        for (int b = 0; b < grid; ++b)
+        {
+            const long long from = part(total, b, grid);
+            for (; before + all(slabs[si]) <= from; ++si) before += all(slabs[si]);
+            const long long unit = unit_at(slabs[si], from - before);
+            out.push_back(BlkShare{unit, (int)si + (unit == slabs[si].unit_end), 0});
+        }
+    }
+    out.push_back(BlkShare{slabs.back().unit_end, (int)slabs.size(), 0});
+    return out;
+}
 SlabKernel slab_kernel(int q)
 {
     return q == 1 ? k_blocks_csr_slabs<1> : q == 2 ? k_blocks_csr_slabs<2> : q == 3 ? k_blocks_csr_slabs<3> : k_blocks_csr_slabs<4>;
@@ -498,6 +556,7 @@ std::unique_ptr<BlocksCsrPlan> blocks_csr_build(int n_src, const int *m0, const 
     P->tr = upload(tr.data(), tr.size(), s);
     P->desc = upload(descs.data(), std::max<size_t>(1, descs.size()), s);
     P->tiles = upload(tiles.data(), tiles.size(), s);
+    std::vector<BlkShare> shares[SLAB_Q];
     for (int q = 0; q < SLAB_Q; ++q)
         if (!slabs[q].empty())
         {
@@ -516,14 +575,9 @@ std::unique_ptr<BlocksCsrPlan> blocks_csr_build(int n_src, const int *m0, const 
                 1, std::min<long long>((long long)runtime().num_sms * std::max(1, per_sm),
                                        std::max((cls.units + RS_WARPS - 1) / RS_WARPS,
                                                 std::min<long long>(cls.units, runtime().num_sms))));
-            std::vector<int> first((size_t)cls.grid);
-            for (int b = 0, si = 0; b < cls.grid; ++b)
-            {
-                while (slabs[q][si].unit_end <= cls.units * b / cls.grid) ++si;
-                first[b] = si;
-            }
-            cls.first = upload(first.data(), first.size(), s);
-            SDL_CUDA(cudaStreamSynchronize(s)); // `first` leaves
+            shares[q] = share_units(slabs[q], h_cp.data(), cls.grid);
+            cls.grid = (int)shares[q].size() - 1;
+            cls.shares = upload(shares[q].data(), shares[q].size(), s);
         }
     SDL_CUDA(cudaStreamSynchronize(s));
     return P;
@@ -542,7 +596,7 @@ void blocks_csr_fill(const BlocksCsrPlan &P, const double *B_vals, const double 
         const auto &c = P.slab_cls[q];
         if (c.n)
             SDL_LAUNCH(slab_kernel(q + 1), c.grid, RS_WARPS * 32, c.smem + RS_WARPS * RS_WARP_BYTES, s, c.slabs.get(),
-                       c.first.get(), c.units, c.smem, P.cp.get(), P.rows.get(), P.vals.get(), P.BT.get(),
+                       c.shares.get(), c.smem, P.cp.get(), P.rows.get(), P.vals.get(), P.BT.get(),
                        C_vals);
     }
     if (P.ntiles)

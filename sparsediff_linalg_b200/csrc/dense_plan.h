@@ -44,6 +44,13 @@ struct BlkSlab
     long long unit_begin, unit_end;
 };
 
+// Where a CTA's share of the units begins: the unit, and the slab that holds it.
+struct BlkShare
+{
+    long long unit;
+    int slab, pad;
+};
+
 struct BlocksCsrPlan
 {
     int S_m = 0, S_n = 0, S_nnz = 0;
@@ -68,7 +75,7 @@ struct BlocksCsrPlan
     struct SlabClass
     {
         DevBuf<BlkSlab> slabs;
-        DevBuf<int> first; // the slab each CTA starts in
+        DevBuf<BlkShare> shares; // of each CTA, and the end
         int n = 0, smem = 0, grid = 0; // smem: the largest slab's bytes
         long long units = 0;
     };

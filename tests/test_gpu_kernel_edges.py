@@ -90,6 +90,38 @@ def test_blocks_csr_uneven_shapes_bit_exact(sdl, orc):
     assert at == P.c_values
 
 
+# columns of very different entry counts, so that CTAs take shares of very different numbers
+# of units: nearly all entries at the start, in the middle or at the end, several slabs and
+# blocks, and more CTAs than units
+@pytest.mark.parametrize("m0,n0,S_n,heavy", [(64, 300, 9000, slice(0, 700)), (70, 200, 9001, slice(4000, 4020)),
+                                             (130, 500, 5003, slice(4990, 5003)), (16, 100, 40, slice(0, 1))])
+def test_blocks_csr_uneven_columns_bit_exact(sdl, orc, m0, n0, S_n, heavy):
+    import torch
+    from sparsediff_linalg_b200.device import BlocksCsr
+    rng = np.random.default_rng(n0)
+    dens = np.full(S_n, 1.5 / n0)
+    dens[heavy] = 0.9
+    D = rng.random((n0, S_n)) < dens
+    Sp = np.concatenate([[0], np.cumsum(D.sum(1))]).astype(np.int32)
+    Si = np.nonzero(D)[1].astype(np.int32)
+    Sx = rng.standard_normal(len(Si))
+    full, half = np.arange(n0, dtype=np.int32), np.arange(0, n0, 2, dtype=np.int32)
+    blocks = [(rng.standard_normal((m0, len(c))), c) for c in (full, half, full, half)]
+    P = BlocksCsr([X.shape[0] for X, _ in blocks], [X.shape[1] for X, _ in blocks], [c for _, c in blocks], Sp, Si,
+                  n0, S_n)
+    Cv = torch.full((P.c_values,), float("nan"), dtype=torch.float64, device="cuda")
+    P.fill(T(np.concatenate([X.ravel() for X, _ in blocks])), T(Sx), Cv)
+    got = Cv.cpu().numpy()
+    want = orc.blocks_csr(blocks, Sp, Si, Sx, S_n)
+    at = 0
+    for src, mk, nk, perm in P.blocks:
+        cols, Cw = want[src]
+        assert np.array_equal(perm, cols) and Cw.shape == (mk, nk)
+        assert np.array_equal(bits(got[at:at + mk * nk]), bits(Cw.ravel()))
+        at += mk * nk
+    assert at == P.c_values
+
+
 # ---------------------------------------------------------------- sorting triplets
 # sizes around a sort tile (3072 pairs) and a structure tile (2048); matrices whose keys
 # take one digit pass up to seven, one cell only (every key equal), rows in order, and a
