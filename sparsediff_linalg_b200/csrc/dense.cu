@@ -35,11 +35,11 @@ constexpr int BC_THREADS = 256;
 // row-major, so that one column of a block is contiguous). The tiles are listed: a grid of
 // the largest block's tiles for every block was mostly CTAs without work where shapes
 // differ (one block of 2000 x 400 beside 3000 of 8 x 8: the fill 2.13 ms), and overran the
-// launch limits beside a few large blocks.
+// launch limits beside a few large blocks. A thread's four loads are in flight together (2400
+// blocks of 64 x 128: 86 -> 67 us).
 __global__ void __launch_bounds__(BC_THREADS) k_blocks_csr_inputs(
     const int *__restrict__ pos, const double *__restrict__ Sx, long long n, double *__restrict__ vals,
-    int gather_ctas, const BlkDesc *__restrict__ descs, const BlkTrTile *__restrict__ tr, const double *__restrict__ B,
-    double *__restrict__ BT)
+    int gather_ctas, const BlkTrTile *__restrict__ tr, const double *__restrict__ B, double *__restrict__ BT)
 {
     __shared__ double t[32][33];
     if ((int)blockIdx.x < gather_ctas)
@@ -49,21 +49,23 @@ __global__ void __launch_bounds__(BC_THREADS) k_blocks_csr_inputs(
             vals[d] = Sx[pos[d]];
         return;
     }
-    const BlkTrTile q = tr[blockIdx.x - gather_ctas];
-    const BlkDesc D = descs[q.blk];
-    const int i0 = q.i0, r0 = q.r0;
+    const BlkTrTile D = tr[blockIdx.x - gather_ctas];
+    const int i0 = D.i0, r0 = D.r0;
     const double *src = B + D.b_off;
     double *dst = BT + D.b_off;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int y = ty; y < 32; y += BC_THREADS / 32)
+    constexpr int ROWS = 32 / (BC_THREADS / 32); // of a thread
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j)
     {
-        const int i = i0 + y, r = r0 + tx;
+        const int y = ty + j * (32 / ROWS), i = i0 + y, r = r0 + tx;
         if (i < D.m0 && r < D.n0_B) t[y][tx] = src[(long long)i * D.n0_B + r];
     }
     __syncthreads();
-    for (int y = ty; y < 32; y += BC_THREADS / 32)
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j)
     {
-        const int r = r0 + y, i = i0 + tx;
+        const int y = ty + j * (32 / ROWS), r = r0 + y, i = i0 + tx;
         if (r < D.n0_B && i < D.m0) dst[(long long)r * D.m0 + i] = t[tx][y];
     }
 }
@@ -101,6 +103,18 @@ constexpr int RS_REC = 128;  // records a warp stages at once
 // 58 at 12, 130 at 40, 261 at 100). With an even share of the units each, a tenth of the
 // columns at 100 entries and the others at 2 took 238 us, 64 us so (147 by k_blocks_csr).
 constexpr int RS_UNIT_COST = 128;
+// Where a CTA would have several slabs in turn (more than RS_FEW_SLABS per SM in all), a slab's
+// load has to pay: a block stays with k_blocks_csr if its columns and entries are too few for
+// that (rs_pays). The line is fitted to both kernels' times over 600 and 2400 blocks of 16 x
+// 100 to 64 x 256 by 14 to 400 columns of 1 to 20 entries: within 0.6 % of the better one on
+// average. 600 blocks of 64 x 64: in slabs 27 us at 14 columns of 6 (19 us in tiles), 29 at
+// 60 (29), 64 at 400 (95); of 64 x 256: 78 (54), 82 (66), 127 (137).
+constexpr int RS_FEW_SLABS = 1;
+constexpr bool rs_pays(int n0, int q, long long cols, long long entries)
+{
+    const long long load = 4LL * n0 + 300 + 30 * entries / cols;
+    return 4 * cols + entries >= (q == 1 ? load / 2 : load); // (slabs of 16 rows: two CTAs per SM)
+}
 constexpr int RS_SLAB_BYTES = 128 * 1024;
 constexpr int RS_N0_MAX = RS_SLAB_BYTES / (32 * 8);
 constexpr int RS_WARP_BYTES = 2 * RS_REC * 16; // two units' records
@@ -490,6 +504,25 @@ std::unique_ptr<BlocksCsrPlan> blocks_csr_build(int n_src, const int *m0, const 
         std::copy(cc.rows.begin(), cc.rows.end(), h_rows.begin() + cc.d_off);
         std::copy(cc.pos.begin(), cc.pos.end(), h_pos.begin() + cc.d_off);
     }
+    // A slab takes up to 64 rows and RS_SLAB_BYTES, a block's rows shared out evenly.
+    struct SlabCut
+    {
+        long long n; // its slabs
+        int per;     // rows of each
+        bool pays;
+    };
+    const auto slab_cut = [&](int k) {
+        const Csc &cc = cscs[csc_of[k]];
+        if (n0[k] > RS_N0_MAX || cc.col_perm_C.empty() || m0[k] == 0) return SlabCut{0, 0, false};
+        const int qmax = std::max(1, std::min(SLAB_Q, RS_SLAB_BYTES / (16 * 8 * std::max(1, n0[k]))));
+        const long long n = ((long long)m0[k] + 16 * qmax - 1) / (16 * qmax);
+        const int per = (int)((m0[k] + n - 1) / n);
+        return SlabCut{n, per, rs_pays(n0[k], (per + 15) / 16, (long long)cc.col_perm_C.size(), (long long)cc.rows.size())};
+    };
+    long long in_turn = 0; // slabs whose load does not pay
+    for (int k = 0; k < n_src; ++k)
+        if (const SlabCut c = slab_cut(k); !c.pays) in_turn += c.n;
+    const bool small_in_tiles = in_turn > RS_FEW_SLABS * (long long)runtime().num_sms;
     // output blocks and their work tiles
     std::vector<BlkDesc> descs;
     std::vector<BlkTile> tiles;
@@ -512,24 +545,19 @@ std::unique_ptr<BlocksCsrPlan> blocks_csr_build(int n_src, const int *m0, const 
             D.n0_B = n0[k];
             D.n0_C = n0C;
             const int blk = (int)descs.size();
-            if (n0[k] > RS_N0_MAX)
+            const SlabCut cut = slab_cut(k);
+            if (n0[k] > RS_N0_MAX || (small_in_tiles && !cut.pays))
                 for (int c0 = 0; c0 < n0C && m0[k] > 0; c0 += BC_COLS) tiles.push_back(BlkTile{blk, c0});
-            else if (n0C > 0 && m0[k] > 0)
-            {
-                // slabs of at most 64 rows and RS_SLAB_BYTES, rows shared out evenly
-                const int qmax = std::max(1, std::min(SLAB_Q, RS_SLAB_BYTES / (16 * 8 * std::max(1, n0[k]))));
-                const int ns = (m0[k] + 16 * qmax - 1) / (16 * qmax);
-                const int per = (m0[k] + ns - 1) / ns;
-                for (int i0 = 0; i0 < m0[k]; i0 += per)
+            else
+                for (long long i0 = 0; cut.n > 0 && i0 < m0[k]; i0 += cut.per)
                 {
-                    const int nrow = std::min(per, m0[k] - i0), q = (nrow + 15) / 16;
+                    const int nrow = (int)std::min<long long>(cut.per, m0[k] - i0), q = (nrow + 15) / 16;
                     auto &cls = P->slab_cls[q - 1];
                     const long long u0 = cls.units;
                     cls.units += (n0C + RS_SHIFT + RS_COLS - 1) / RS_COLS;
-                    slabs[q - 1].push_back(BlkSlab{D, i0, nrow, u0, cls.units});
+                    slabs[q - 1].push_back(BlkSlab{D, (int)i0, nrow, u0, cls.units});
                     cls.smem = std::max(cls.smem, n0[k] * q * 16 * 8);
                 }
-            }
             descs.push_back(D);
             P->src.push_back(k);
             P->col_perm.push_back(cc.col_perm_C);
@@ -550,7 +578,8 @@ std::unique_ptr<BlocksCsrPlan> blocks_csr_build(int n_src, const int *m0, const 
     std::vector<BlkTrTile> tr;
     for (size_t q = 0; q < descs.size(); ++q)
         for (long long i0 = 0; i0 < descs[q].m0 && descs[q].n0_C > 0; i0 += 32)
-            for (long long r0 = 0; r0 < descs[q].n0_B; r0 += 32) tr.push_back(BlkTrTile{(int)q, (int)i0, (int)r0});
+            for (long long r0 = 0; r0 < descs[q].n0_B; r0 += 32) 
+                tr.push_back(BlkTrTile{descs[q].b_off, descs[q].m0, descs[q].n0_B, (int)i0, (int)r0});
     if (tr.size() > INT_MAX / 2) fail(SDL_ERR_OVERFLOW, "blocks x CSR: too many blocks");
     P->ntr = (int)tr.size();
     P->tr = upload(tr.data(), tr.size(), s);
@@ -590,7 +619,7 @@ void blocks_csr_fill(const BlocksCsrPlan &P, const double *B_vals, const double 
     // (a source feeding two outputs would be transposed twice: they are one to one here)
     const int gather = P.d_total > 0 ? grid_cap(P.d_total, BC_THREADS, runtime().num_sms * 8) : 0;
     SDL_LAUNCH(k_blocks_csr_inputs, gather + P.ntr, BC_THREADS, 0, s, P.pos.get(), S_x, P.d_total, P.vals.get(),
-               gather, P.desc.get(), P.tr.get(), B_vals, P.BT.get());
+               gather, P.tr.get(), B_vals, P.BT.get());
     for (int q = 0; q < SLAB_Q; ++q)
     {
         const auto &c = P.slab_cls[q];

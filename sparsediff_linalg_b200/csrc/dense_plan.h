@@ -27,10 +27,12 @@ struct BlkTile
     int blk, c0;
 };
 
-// Rows and columns of a source block that a CTA transposes: 32 of each from i0, r0 on.
-struct BlkTrTile
+// Rows and columns of a source block (m0 x n0_B from b_off on) that a CTA transposes: 32 of
+// each from i0, r0 on.
+struct alignas(16) BlkTrTile
 {
-    int blk, i0, r0;
+    long long b_off;
+    int m0, n0_B, i0, r0;
 };
 
 // Rows [i0, i0 + nrow) of an output block, kept in shared memory while the block's

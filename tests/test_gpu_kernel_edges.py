@@ -90,6 +90,42 @@ def test_blocks_csr_uneven_shapes_bit_exact(sdl, orc):
     assert at == P.c_values
 
 
+# so many small blocks of few columns that they are not kept in slabs (more than one per SM),
+# one slab fewer, enough columns, and such blocks beside one of more columns and one of more
+# rows
+@pytest.mark.parametrize("nb,n0C,extra", [(148, 20, False), (149, 20, False), (400, 120, False), (350, 1, True)])
+def test_blocks_csr_many_small_blocks_bit_exact(sdl, orc, nb, n0C, extra):
+    import torch
+    from sparsediff_linalg_b200.device import BlocksCsr
+    rng = np.random.default_rng(nb + n0C)
+    S_m, S_n = 60, 200
+    D = np.zeros((S_m, S_n), bool)
+    D[:7, :n0C] = rng.random((7, n0C)) < 0.4
+    D[3, :n0C] = True
+    D[7:, :] = rng.random((S_m - 7, S_n)) < 0.05
+    Sp = np.concatenate([[0], np.cumsum(D.sum(1))]).astype(np.int32)
+    Si = np.nonzero(D)[1].astype(np.int32)
+    Sx = rng.standard_normal(len(Si))
+    small, full = np.arange(7, dtype=np.int32), np.arange(S_m, dtype=np.int32)
+    blocks = [(rng.standard_normal((1 + k % 9, 7)), small) for k in range(nb)]
+    if extra:
+        blocks[200] = (rng.standard_normal((20, S_m)), full)
+        blocks.append((rng.standard_normal((150, 7)), small))
+    P = BlocksCsr([X.shape[0] for X, _ in blocks], [X.shape[1] for X, _ in blocks], [c for _, c in blocks], Sp, Si,
+                  S_m, S_n)
+    Cv = torch.full((P.c_values,), float("nan"), dtype=torch.float64, device="cuda")
+    P.fill(T(np.concatenate([X.ravel() for X, _ in blocks])), T(Sx), Cv)
+    got = Cv.cpu().numpy()
+    want = orc.blocks_csr(blocks, Sp, Si, Sx, S_n)
+    at = 0
+    for src, mk, nk, perm in P.blocks:
+        cols, Cw = want[src]
+        assert np.array_equal(perm, cols) and Cw.shape == (mk, nk)
+        assert np.array_equal(bits(got[at:at + mk * nk]), bits(Cw.ravel()))
+        at += mk * nk
+    assert at == P.c_values
+
+
 # columns of very different entry counts, so that CTAs take shares of very different numbers
 # of units: nearly all entries at the start, in the middle or at the end, several slabs and
 # blocks, and more CTAs than units
