@@ -521,7 +521,8 @@ int coalesce_build(const int *rows, const int *cols, int n, int m, int ncols, De
     if (gap_cap)
         SDL_LAUNCH(k_cs_gaps, (unsigned)std::min(gap_cap, 148LL * 8), CS_THREADS, 0, s, gaps.get(), ngaps.get(),
                    Cp.get());
-    if (n >= COALESCE_BUCKET_MIN) bucket_build(ostart.get(), perm.get(), n, nout, buckets, s);
+    if (n >= COALESCE_BUCKET_MIN || (n >= COALESCE_BUCKET_MIN_HEAVY && n >= (long long)COALESCE_HEAVY * nout))
+        bucket_build(ostart.get(), perm.get(), n, nout, buckets, s);
     SDL_CUDA(cudaStreamSynchronize(s));
     return nout;
 }

@@ -182,16 +182,21 @@ void gather_values(const int *d_src, const double *d_x, double *d_out, int n,
                    cudaStream_t s);
 
 // ---------------------------------------------------------------- coalescing
-// Bucketed refill plan of a coalescing (coalesce.cu), for inputs of at least
-// COALESCE_BUCKET_MIN triplets: the refill first writes every value to its place in buf,
-// where the triplets of each bucket (a range of outputs) lie together, then sums the
-// outputs bucket by bucket. Pass 1 goes by chunks of the input, each in the order of its
-// places: from (which triplet of the chunk) and to (its place). Pass 2: begin, the first
+// Bucketed refill plan of a coalescing (coalesce.cu): the refill first writes every value to
+// its place in buf, where the triplets of each bucket (a range of outputs) lie together, then
+// sums the outputs bucket by bucket. Pass 1 goes by chunks of the input, each in the order of
+// its places: from (which triplet of the chunk) and to (its place). Pass 2: begin, the first
 // output of every bucket; local, of every sorted triplet its place in the bucket. buf is
-// the plan's refill scratch. Below COALESCE_BUCKET_MIN the values fit L2 well enough to
-// be gathered there in one pass (one pass against two: 8.2M triplets 78 and 96 us, 11.2M
-// 126 and 117 us, 21M 336 and 202 us).
+// the plan's refill scratch.
+// From COALESCE_BUCKET_MIN triplets on; below, the values fit L2 well enough to be gathered
+// there in one pass (one pass against two: 8.2M triplets 78 and 96 us, 11.2M 126 and 117 us,
+// 21M 336 and 202 us). From COALESCE_BUCKET_MIN_HEAVY on also with COALESCE_HEAVY triplets
+// per output or more, whose gathers are chains of that length: 4.3M triplets, 100 per output
+// 129 and 66 us, 1000 per output 1025 and 136 us, 10000 per output 10.1 and 1.5 ms. (At 30
+// per output 68 and 64 us, but the plan takes 72 us longer.)
 constexpr int COALESCE_BUCKET_MIN = 10 << 20;
+constexpr int COALESCE_BUCKET_MIN_HEAVY = 4 << 20;
+constexpr int COALESCE_HEAVY = 96;
 struct CoalesceBuckets
 {
     int n = 0, nb = 0, nchunks = 0;

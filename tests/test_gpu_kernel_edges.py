@@ -247,6 +247,30 @@ def test_coalesce_buckets_edges_bit_exact(sdl, n, heavy):
         assert np.array_equal(bits(Cx.cpu().numpy()), bits(wx))
 
 
+# fewer triplets, but many per output: the smallest input that goes through buckets, one
+# triplet or one output to either side of it, and a few outputs that hold them all
+@pytest.mark.parametrize("n,nout", [(4 << 20, (4 << 20) // 96), (4 << 20, (4 << 20) // 96 + 1),
+                                    ((4 << 20) - 1, 1000), ((4 << 20) + 1, 999), (5000011, 7)])
+def test_coalesce_heavy_outputs_bit_exact(sdl, n, nout):
+    import torch
+    from oracle import parallel
+    from sparsediff_linalg_b200.device import Coalesce
+    rng = np.random.default_rng(nout)
+    m, ncols = 3000, 20
+    cell = rng.permutation(m * ncols)[:nout]
+    at = cell[rng.permutation(n) % nout]
+    rows, cols = (at // ncols).astype(np.int32), (at % ncols).astype(np.int32)
+    x = rng.standard_normal(n) * 10.0 ** rng.integers(-6, 7, n)
+    x[::3] = -0.0
+    C = Coalesce(T(rows), T(cols), m, ncols)
+    assert C.nnz == nout
+    Cx = torch.full((C.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+    C.fill(T(x), Cx)
+    wp, wi, wx = parallel.coalesce(rows, cols, x, m, ncols)[:3]
+    assert np.array_equal(C.Cp.cpu().numpy(), wp) and np.array_equal(C.Ci.cpu().numpy(), wi)
+    assert np.array_equal(bits(Cx.cpu().numpy()), bits(wx))
+
+
 # ---------------------------------------------------------------- transpose
 # columns of every sorting class and its edges (64 keys counted in place, 1024 a warp,
 # 8192 a CTA), beside empty and short ones; entries around the 2048-entry tiles; far more
