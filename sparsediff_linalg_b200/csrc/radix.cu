@@ -1,7 +1,10 @@
-// Stable LSD radix sort of pairs, 8 bits per pass, used once per pattern: (32-bit
-// output, 8-byte payload) pairs group the terms of the rows beyond the tile budget by
-// output; (row << bits | column, triplet) pairs order COO triplets. Stability keeps,
-// inside every key, the input order -- upstream's visiting order.
+// Stable LSD radix sort of pairs, 8 bits per pass, used once per pattern: (32-bit key, 8-byte
+// payload) pairs order the terms of the rows beyond the tile budget by window, or by output;
+// (row << bits | column, triplet) pairs order COO triplets. Stability keeps, inside every key,
+// the input order -- upstream's visiting order. The method is that of A. Adinets and
+// D. Merrill, "Onesweep: A Faster Least Significant Digit Radix Sort for GPUs" (2022), with
+// the look-back of D. Merrill and M. Garland, "Single-pass Parallel Prefix Scan with Decoupled
+// Look-back" (2016); the code is this library's own.
 //
 // One kernel reads the keys once for the digit counts of all passes; then each pass is
 // one kernel that reads and writes every pair once. A CTA takes the next tile (a ticket,
@@ -118,21 +121,19 @@ struct TileWord
     static constexpr W MASK = (W(1) << SHIFT) - 1;
 };
 
-// The lanes whose digit is this lane's.
+// The lanes whose digit is this lane's: all but those that differ from it in some bit, which
+// are those whose place in the ballot of that bit does not hold this lane's bit.
 __device__ __forceinline__ unsigned warp_match8(unsigned dg)
 {
-    unsigned grp = FULL_MASK;
+    unsigned differ = 0;
 #pragma unroll
     for (int b = 0; b < 8; ++b)
     {
-        unsigned m; // the lanes whose bit b is this lane's
-        asm volatile("{\n\t.reg .pred p;\n\tand.b32 %0, %1, %2;\n\tsetp.ne.u32 p, %0, 0;\n\t"
-                     "vote.sync.ballot.b32 %0, p, 0xffffffff;\n\t@!p not.b32 %0, %0;\n\t}"
-                     : "=r"(m)
-                     : "r"(dg), "r"(1u << b));
-        grp &= m;
+        const unsigned with = __ballot_sync(FULL_MASK, (dg >> b) & 1u);
+        const unsigned mine = 0u - ((dg >> b) & 1u); // all ones where this lane's bit is set
+        differ |= with ^ mine;
     }
-    return grp;
+    return ~differ;
 }
 
 template <class K, class V>
