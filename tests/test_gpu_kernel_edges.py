@@ -247,6 +247,40 @@ def test_coalesce_buckets_edges_bit_exact(sdl, n, heavy):
         assert np.array_equal(bits(Cx.cpu().numpy()), bits(wx))
 
 
+# the same with a factor per triplet: a scaled sum of two sparse operands with MIN entries
+# together, one fewer and one more; each output is (0 + d1 a) + d2 b, one rounding each
+@pytest.mark.parametrize("extra", [-1, 0, 1])
+def test_scaled_sum_through_buckets_bit_exact(sdl, extra):
+    from sparsediff_linalg_b200 import matrices as M
+    from test_gpu_dense_ops import Lib, csr_of
+    from test_gpu_sums import SIGS
+    L = M.mlib()
+    for name, (res, args) in SIGS.items():
+        getattr(L, name).restype, getattr(L, name).argtypes = res, args
+    lib = Lib(L)
+    rng = np.random.default_rng(900 + extra)
+    m, n = 2900, 4000
+    nnz = [MIN // 2, MIN // 2 + extra]
+    cells = [np.sort(rng.permutation(m * n)[:k]) for k in nnz]
+    vals = [rng.standard_normal(k) for k in nnz]
+    vals[0][::5] = -0.0
+    d = [rng.uniform(-2, 2, m) for _ in range(2)]
+    A, B = (lib.make(("sparse", (np.concatenate([[0], np.cumsum(np.bincount(c // n, minlength=m))]).astype(np.int32),
+                                 (c % n).astype(np.int32), v, m, n))) for c, v in zip(cells, vals))
+    S = L.new_sparse_matrix_alloc(m, n, sum(nnz))
+    L.sum_matrices_alloc(A, B, S)
+    L.sum_scaled_matrices_fill_values(A, B, S, d[0].ctypes.data, d[1].ctypes.data)
+    p, i, x = csr_of(S)
+    lib.free(S, B, A)
+    want, has = np.zeros(m * n), np.zeros(m * n, bool)
+    for c, v, f in zip(cells, vals, d):
+        want[c] = want[c] + f[c // n] * v
+        has[c] = True
+    at = np.flatnonzero(has)
+    assert np.array_equal(p, np.concatenate([[0], np.cumsum(np.bincount(at // n, minlength=m))]))
+    assert np.array_equal(i, at % n) and np.array_equal(bits(x), bits(want[at]))
+
+
 # fewer triplets, but many per output: the smallest input that goes through buckets, one
 # triplet or one output to either side of it, and a few outputs that hold them all
 @pytest.mark.parametrize("n,nout", [(4 << 20, (4 << 20) // 96), (4 << 20, (4 << 20) // 96 + 1),
