@@ -217,6 +217,37 @@ def test_coalesce_largest_row_count(sdl):
     assert at == m + 1
 
 
+# more than 2^30 triplets, where the sort's tile words are 64 bits wide: every cell of 32768
+# columns once, in an order scattered by a multiplication modulo the prime 2^30 + 3, each
+# triplet's value its cell
+def test_coalesce_over_2_30_triplets(sdl):
+    import torch
+    from sparsediff_linalg_b200.device import Coalesce
+    n, ncols = 2**30 + 3, 32768
+    cell = torch.arange(n, dtype=torch.int64, device="cuda")
+    cell.mul_(2654435761).remainder_(n)
+    rows, cols = torch.div(cell, ncols, rounding_mode="floor").to(torch.int32), (cell % ncols).to(torch.int32)
+    x = cell.to(torch.float64)
+    del cell
+    m = n // ncols + 1
+    C = Coalesce(rows, cols, m, ncols)
+    del rows, cols
+    assert C.nnz == n
+    assert torch.equal(C.Cp.cpu(), torch.arange(m + 1, dtype=torch.int64).mul_(ncols).clamp_(max=n).to(torch.int32))
+    out = torch.full((n,), float("nan"), dtype=torch.float64, device="cuda")
+    C.fill(x, out)
+    torch.cuda.synchronize()
+    del x
+    step = 1 << 26
+    for at in range(0, n, step):
+        q = torch.arange(at, min(n, at + step), dtype=torch.int64, device="cuda")
+        assert torch.equal(out[at:at + step], q.to(torch.float64))
+        assert torch.equal(C.Ci[at:at + step], (q % ncols).to(torch.int32))
+    del C, out, q
+    torch.cuda.empty_cache()
+    sdl.sdl_release_cached_memory()
+
+
 # ---------------------------------------------------------------- bucketed refill
 MIN = 10 << 20  # triplets from which a refill goes through buckets
 
@@ -470,6 +501,27 @@ def test_row_sort_edges_bit_exact(sdl, orc, n):
 
 
 # ---------------------------------------------------------------- refill schedule
+# list sections of more words (about 70M) than the schedule's first scratch (64Mi) holds: they
+# are built again in a larger one
+def test_schedule_of_many_list_words_bit_exact(sdl, orc):
+    import torch
+    from sparsediff_linalg_b200.device import Product
+    rng = np.random.default_rng(11)
+    nL, per_l, nA, per_a, n = 66000, 25, 1000, 40, 60
+    Bi = np.concatenate([np.sort(rng.permutation(n)[:per_a]) for _ in range(nA)]).astype(np.int32)
+    Bp = (np.arange(nA + 1) * per_a).astype(np.int32)
+    Ai = np.sort((rng.integers(0, nA, (nL, 1)) + 37 * np.arange(per_l)) % nA, axis=1).astype(np.int32).ravel()
+    Ap = (np.arange(nL + 1) * per_l).astype(np.int32)
+    Ax, Bx = rng.standard_normal(len(Ai)), rng.standard_normal(len(Bi))
+    P = Product(T(Ap), T(Ai), T(Bp), T(Bi), n)
+    wp, wi, wx = orc.spgemm((Ap, Ai, Ax, nL, nA), (Bp, Bi, Bx, nA, n))
+    assert len(Ai) * per_a + len(wi) > 64 << 20  # terms in lists, and their headers
+    assert np.array_equal(P.Cp.cpu().numpy(), wp) and np.array_equal(P.Ci.cpu().numpy(), wi)
+    C = torch.full((P.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+    P.fill(T(Ax), None, T(Bx), C)
+    assert np.array_equal(bits(C.cpu().numpy()), bits(wx))
+
+
 # operands changed between the structure of C and its refill plan (columns that some rows of
 # C lack): the plan is refused, the error does not stick, and restored operands get their plan
 def test_schedule_of_changed_operands_is_refused(sdl):
