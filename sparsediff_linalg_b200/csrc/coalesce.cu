@@ -80,10 +80,11 @@ __device__ __forceinline__ bool cs_opens(const unsigned long long *__restrict__ 
     return q < n && (q == 0 || keys[q] != keys[q - 1]);
 }
 
-// Outputs that each tile's triplets open.
+// Outputs that each tile's triplets open (and no gaps yet).
 __global__ void __launch_bounds__(CS_THREADS) k_cs_count(const unsigned long long *__restrict__ keys, int n,
-                                                         int *__restrict__ tile_outs)
+                                                         int *__restrict__ tile_outs, int *__restrict__ ngaps)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ngaps = 0;
     __shared__ int part[CS_THREADS / 32];
     const long long q0 = (long long)blockIdx.x * CS_TILE + threadIdx.x;
     int c = 0;
@@ -151,31 +152,31 @@ __global__ void __launch_bounds__(CS_THREADS) k_cs_emit(const unsigned long long
     {
         const long long q = q0 + 32 * j;
         const int o = o0 + __popc(heads[j] & lanemask_lt());
-        long long lo = 0, hi = 0; // Cp[lo .. hi) = o (hi is up to 2^31)
+        unsigned lo = 0, hi = 0; // Cp[lo .. hi) = o (hi is up to 2^31)
         if ((heads[j] >> lane) & 1u)
         {
             ostart[o] = (int)q;
             Ci[o] = (int)(key[j] & cmask);
-            lo = q == 0 ? 0 : (long long)(prev[j] >> col_bits) + 1;
-            hi = (long long)(key[j] >> col_bits) + 1;
+            lo = q == 0 ? 0 : (unsigned)(prev[j] >> col_bits) + 1;
+            hi = (unsigned)(key[j] >> col_bits) + 1;
         }
         else if (q == n) // one past the last triplet
         {
             ostart[o] = n;
-            lo = (long long)(prev[j] >> col_bits) + 1;
-            hi = (long long)m + 1;
+            lo = (unsigned)(prev[j] >> col_bits) + 1;
+            hi = (unsigned)m + 1;
         }
         unsigned longs = __ballot_sync(FULL_MASK, hi - lo > 8);
         if (hi - lo <= 8)
-            for (long long r = lo; r < hi; ++r) Cp[r] = o;
+            for (unsigned r = lo; r < hi; ++r) Cp[r] = o;
         for (; longs; longs &= longs - 1)
         {
             const int l = __ffs(longs) - 1;
-            const long long x = __shfl_sync(FULL_MASK, lo, l), y = __shfl_sync(FULL_MASK, hi, l);
+            const unsigned x = __shfl_sync(FULL_MASK, lo, l), y = __shfl_sync(FULL_MASK, hi, l);
             const int v = __shfl_sync(FULL_MASK, o, l);
             if (y - x <= CS_GAP)
             {
-                for (long long r = x + lane; r < y; r += 32) Cp[r] = v;
+                for (unsigned r = x + lane; r < y; r += 32) Cp[r] = v;
                 continue;
             }
             const int pieces = (int)((y - x + CS_GAP - 1) / CS_GAP);
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(CS_THREADS) k_cs_emit(const unsigned long long
             at = __shfl_sync(FULL_MASK, at, 0);
             for (int p = lane; p < pieces; p += 32)
             {
-                const long long r = x + (long long)p * CS_GAP;
+                const unsigned r = x + (unsigned)p * CS_GAP;
                 gaps[at + p] = CsGap{(int)r, (int)(min(r + CS_GAP, y) - 1), v};
             }
         }
@@ -506,20 +507,19 @@ int coalesce_build(const int *rows, const int *cols, int n, int m, int ncols, De
     }
     // tiles of the n triplets and the one position after them
     const int ntiles = (int)((long long)n / CS_TILE + 1);
-    DevBuf<int> outs((size_t)ntiles), first((size_t)ntiles + 1);
-    SDL_LAUNCH(k_cs_count, ntiles, CS_THREADS, 0, s, ka.get(), n, outs.get());
+    DevBuf<int> outs((size_t)ntiles + 1), first((size_t)ntiles + 1);
+    int *ngaps = outs.get() + ntiles;
+    SDL_LAUNCH(k_cs_count, ntiles, CS_THREADS, 0, s, ka.get(), n, outs.get(), ngaps);
     const int nout = exclusive_scan_i32_checked(outs.get(), first.get(), ntiles, s);
     if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "coalesce plan: the sort of the triplets did not finish");
     Ci.reset((size_t)std::max(1, nout));
     ostart.reset((size_t)nout + 1);
     const long long gap_cap = cs_gap_cap(m);
     DevBuf<CsGap> gaps((size_t)gap_cap);
-    DevBuf<int> ngaps(gap_cap ? 1 : 0);
-    if (gap_cap) SDL_CUDA(cudaMemsetAsync(ngaps.get(), 0, sizeof(int), s));
     SDL_LAUNCH(k_cs_emit, ntiles, CS_THREADS, 0, s, ka.get(), n, m, col_bits, first.get(), ostart.get(), Ci.get(),
-               Cp.get(), gaps.get(), ngaps.get());
+               Cp.get(), gaps.get(), ngaps);
     if (gap_cap)
-        SDL_LAUNCH(k_cs_gaps, (unsigned)std::min(gap_cap, 148LL * 8), CS_THREADS, 0, s, gaps.get(), ngaps.get(),
+        SDL_LAUNCH(k_cs_gaps, (unsigned)std::min(gap_cap, 148LL * 8), CS_THREADS, 0, s, gaps.get(), ngaps,
                    Cp.get());
     if (n >= COALESCE_BUCKET_MIN || (n >= COALESCE_BUCKET_MIN_HEAVY && n >= (long long)COALESCE_HEAVY * nout))
         bucket_build(ostart.get(), perm.get(), n, nout, buckets, s);

@@ -1007,7 +1007,7 @@ struct SchedTotals
 __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
     NumArgs a, const unsigned char *__restrict__ rcls, const int *__restrict__ tile_start,
     const long long *__restrict__ term_pref, TileDesc *__restrict__ tiles, int *__restrict__ tile_nent,
-    unsigned *__restrict__ W, unsigned *__restrict__ X, long long x_cap, int2 *__restrict__ ES,
+    unsigned *__restrict__ W, long long w_total, unsigned *__restrict__ X, long long x_cap, int2 *__restrict__ ES,
     SchedTotals *__restrict__ totals)
 {
     extern __shared__ __align__(16) int bsm[];
@@ -1032,6 +1032,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
     const int tile = blockIdx.x;
     const int r0 = tile_start[tile], nrows = tile_start[tile + 1] - r0;
     const int out0 = a.Cp[r0];
+    const long long wb = term_pref[r0];
     for (int q = tid; q < TILE_ACC; q += TILE_THREADS) t.cnt[q] = 0;
     if (tid == 0) t.misc[0] = t.misc[3] = 0;
     int nr = 0, ne = 0;
@@ -1079,7 +1080,6 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
     for (int o = tid; o < total_out; o += TILE_THREADS) t.ci[o] = a.Ci[out0 + o];
     const int b0 = r0 / a.L_m;
     const int vb = b0 * a.L_nnz + a.Lp[r0 - b0 * a.L_m];
-    const long long wb = term_pref[r0];
 
     // terms per output; the ES records of the entries
     int last_ent = 0;
@@ -1093,8 +1093,9 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tile_schedule(
     });
     atomicMax(&t.misc[0], last_ent);
     __syncthreads();
-    // the operands changed since C's columns and the rows' terms were counted
-    if (t.misc[3] || nterms != term_pref[r0 + nrows] - wb)
+    // the operands changed since C's columns and the rows' terms were counted (a tile whose
+    // words end past the next one's first is found by the schedule's check)
+    if (t.misc[3] || wb + nterms > w_total)
     {
         leave_empty(1);
         return;
@@ -2931,7 +2932,7 @@ void build_big_rows(Product &P, const long long *ub, const NumArgs &na, cudaStre
 }
 
 // Checks every index the tile refill will use, once per schedule: per tile, its
-// window and output range, its words inside the word array, and for every term
+// window and output range, its words up to the next tile's, and for every term
 // word that is not a list word its entry, the entry's A position for that term and
 // its value slot, and its output inside the window; per list, its output and items.
 // The refill's term loop then reads without per-term checks.
@@ -2945,7 +2946,8 @@ __global__ void k_validate_schedule(const TileDesc *__restrict__ tiles, int ntil
         const TileDesc D = tiles[t];
         if (D.nterms < 0 || D.nout < 0 || D.nout > TILE_ACC || D.out_begin < 0 ||
             (long long)D.out_begin + D.nout > nnzC || D.word_begin < 0 ||
-            (long long)D.word_begin + D.nterms > word_total || D.vbase < 0 || D.prod != 0)
+            (long long)D.word_begin + D.nterms != (t + 1 < ntiles ? tiles[t + 1].word_begin : word_total) ||
+            D.vbase < 0 || D.prod != 0)
         {
             if (threadIdx.x == 0) atomicOr(err, 4);
             continue;
@@ -3059,7 +3061,7 @@ void build_schedule(const ProductDesc &d, Product &P, const long long *ub, cudaS
         xs.reset((size_t)x_cap);
         SDL_CUDA(cudaMemsetAsync(totals.get(), 0, sizeof(SchedTotals), s));
         SDL_LAUNCH(k_tile_schedule, P.ntiles, TILE_THREADS, build_smem_bytes(), s, na, rcls.get(), tile_start.get(),
-                   tpref.get(), P.tiles.get(), P.tile_nent.get(), P.W.get(), xs.get(), x_cap, P.ES.get(),
+                   tpref.get(), P.tiles.get(), P.tile_nent.get(), P.W.get(), word_total, xs.get(), x_cap, P.ES.get(),
                    totals.get());
         SDL_CUDA(cudaMemcpyAsync(&h, totals.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
         SDL_CUDA(cudaStreamSynchronize(s));

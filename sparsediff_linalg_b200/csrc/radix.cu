@@ -129,9 +129,8 @@ __device__ __forceinline__ unsigned warp_match8(unsigned dg)
 #pragma unroll
     for (int b = 0; b < 8; ++b)
     {
-        const unsigned with = __ballot_sync(FULL_MASK, (dg >> b) & 1u);
-        const unsigned mine = 0u - ((dg >> b) & 1u); // all ones where this lane's bit is set
-        differ |= with ^ mine;
+        const unsigned mine = (unsigned)((int)(dg << (31 - b)) >> 31); // bit b, in every place
+        differ |= __ballot_sync(FULL_MASK, mine) ^ mine;
     }
     return ~differ;
 }
