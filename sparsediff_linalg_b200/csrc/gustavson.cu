@@ -176,9 +176,10 @@ __global__ void k_mask_classes(const unsigned char *__restrict__ mask, int m_out
         if (!mask[r]) cls[r] = 255;
 }
 
-// Numeric class, tile weight and terms in tiles of every output row. A tile row costs its terms,
-// one unit per 16 of its L entries and TILE_ROW_COST units; a larger row
-// costs TILE_BUDGET, so it always ends its tile. Rows with more than TILE_MAX_LROW L
+// Numeric class, tile weight (in half units) and terms in tiles of every output row. A tile
+// row costs its terms, one unit per 16 of its L entries and TILE_ROW_COST units -- or half a
+// unit less if it has few terms, so that 256 of those fit a tile; a larger row costs
+// TILE_BUDGET, so it always ends its tile. Rows with more than TILE_MAX_LROW L
 // entries never join a tile (the 18-bit entry index of a term word stays in range).
 constexpr int TILE_MAX_LROW = 131072;
 __global__ void k_num_classify(const long long *__restrict__ ub, const int *__restrict__ Cp,
@@ -205,8 +206,8 @@ __global__ void k_num_classify(const long long *__restrict__ ub, const int *__re
         else
             c = NUM_GMEM;
         cls[r] = (unsigned char)c;
-        const long long lw = (lenL + 15) / 16 + TILE_ROW_COST;
-        weight[r] = c == NUM_TILE ? u + lw : (c == 255 ? lw : TILE_BUDGET);
+        const long long lw = 2 * ((lenL + 15) / 16) + (u < TILE_FEW ? TILE_ROW_COST2_FEW : 2 * TILE_ROW_COST);
+        weight[r] = c == NUM_TILE ? 2 * u + lw : (c == 255 ? lw : 2 * TILE_BUDGET);
         tterms[r] = c == NUM_TILE ? u : 0;
     }
 }
@@ -3007,7 +3008,7 @@ void build_schedule(const ProductDesc &d, Product &P, const long long *ub, cudaS
     const long long word_total = exclusive_scan_i64(tterms.get(), tpref.get(), m_out, s);
     DevBuf<int> flag(m_out), tile_of((size_t)m_out + 1);
     const int budget = P.cfg.tile_budget > 0 ? std::max(TILE_T / 8, std::min(TILE_BUDGET, P.cfg.tile_budget)) : TILE_BUDGET;
-    SDL_LAUNCH(k_tile_flags, grid_for(m_out, 256, rt.num_sms * 8), 256, 0, s, wpref.get(), m_out, budget,
+    SDL_LAUNCH(k_tile_flags, grid_for(m_out, 256, rt.num_sms * 8), 256, 0, s, wpref.get(), m_out, 2 * budget,
                flag.get());
     P.ntiles = exclusive_scan_i32_checked(flag.get(), tile_of.get(), m_out, s);
     DevBuf<int> tile_start((size_t)P.ntiles + 1);

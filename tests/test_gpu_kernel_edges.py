@@ -501,6 +501,31 @@ def test_row_sort_edges_bit_exact(sdl, orc, n):
 
 
 # ---------------------------------------------------------------- refill schedule
+# tiles at their limit of 256 rows: rows without terms, of one term, of 7 and 8 terms (the
+# edge of the cheaper row), alone and mixed, with tile budgets down to the smallest
+@pytest.mark.parametrize("lens", [(0,), (1,), (0, 1), (7,), (8,), (7, 8, 0, 1, 300)])
+@pytest.mark.parametrize("budget", [0, 128, 500, 1152])
+def test_tiles_of_short_rows_bit_exact(sdl, orc, lens, budget):
+    import torch
+    from sparsediff_linalg_b200.device import Product
+    rng = np.random.default_rng(len(lens) * 7 + budget)
+    nL, nA, n = 5000, 800, 900
+    rows = rng.choice(lens, nL)
+    rows[[17, 4000]] = 3
+    Ap = np.concatenate([[0], np.cumsum(rows)]).astype(np.int32)
+    Ai = np.concatenate([np.sort(rng.permutation(nA)[:k]) for k in rows]).astype(np.int32)
+    Bp, Bi = np.arange(nA + 1, dtype=np.int32), rng.integers(0, n, nA).astype(np.int32)
+    Ax, Bx = rng.standard_normal(len(Ai)), rng.standard_normal(nA)
+    P = Product(T(Ap), T(Ai), T(Bp), T(Bi), n)
+    if budget:
+        P.replan(tile_budget=budget)
+    C = torch.full((P.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+    P.fill(T(Ax), None, T(Bx), C)
+    wp, wi, wx = orc.spgemm((Ap, Ai, Ax, nL, nA), (Bp, Bi, Bx, nA, n))
+    assert np.array_equal(P.Cp.cpu().numpy(), wp) and np.array_equal(P.Ci.cpu().numpy(), wi)
+    assert np.array_equal(bits(C.cpu().numpy()), bits(wx))
+
+
 # list sections of more words (about 70M) than the schedule's first scratch (64Mi) holds: they
 # are built again in a larger one
 def test_schedule_of_many_list_words_bit_exact(sdl, orc):
