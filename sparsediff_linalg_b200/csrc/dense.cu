@@ -93,7 +93,10 @@ __global__ void __launch_bounds__(BC_THREADS) k_blocks_csr_inputs(
 // registers it took 1.15 ms, with 32 rows a pass 1.11-1.16 ms.
 // Blocks of more than RS_N0_MAX columns stay with k_blocks_csr: slabs of only 16 rows
 // spread a record's read too thin (8 blocks of 64 x 1000 with 40 per column: 711 against
-// 601 us; with slabs of 32 rows, n0 = 512 and 6 per column, 96 against 143 us).
+// 601 us; with slabs of 32 rows, n0 = 512 and 6 per column, 96 against 143 us). Up to there
+// the slabs hold their lead at every density (16 blocks of 64 x 256 times 256 x 8000, us in
+// slabs and in tiles: 36 and 36 at 1 per column, 58 and 85 at 12, 130 and 202 at 40, 636 and
+// 1011 at 250), also where a unit's records are staged in parts or read from global memory.
 constexpr int RS_WARPS = 16; // warps of a CTA
 constexpr int RS_COLS = 16;  // output columns of a unit
 constexpr int RS_SHIFT = 3;  // columns a unit may start early, to meet C's 32-byte sectors

@@ -15,11 +15,12 @@
 // all counts up to it once known). The tile is reordered by digit in shared memory, so
 // the pairs of one digit leave for consecutive positions.
 //
-// What bounds it: instruction issue (about 150 instructions per 32 pairs, a third of
-// them the ballots, at 32 warps per SM) before the 2 x 12 bytes per pair and pass through
-// HBM. 10M (64-bit, 32-bit) pairs take 93 us a pass; with a histogram kernel, a scan of
-// all tiles' digit counts and a scatter that read the keys twice more, a pass took 210 us.
-// match_any in place of the ballots: 130 us.
+// What bounds it: latency at 32 warps per SM (64 registers) more than any unit: per pass of
+// 10M (64-bit, 32-bit) pairs, 92 us, 55 % of the issue slots (170 instructions per 32 pairs),
+// 55 % of the shared-memory pipe and 26 % of HBM are used, and a warp waits 13.8 cycles per
+// instruction, for loads (2.8), fixed latencies (2.3), shared memory (2.1) and barriers (1.5).
+// With a histogram kernel, a scan of all tiles' digit counts and a scatter that read the keys
+// twice more, a pass took 210 us; match_any in place of the ballots: 130 us.
 #include <algorithm>
 #include <mutex>
 #include <set>

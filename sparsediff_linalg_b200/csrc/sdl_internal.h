@@ -84,6 +84,8 @@ int take_device_error(cudaStream_t s);
 
 // ---------------------------------------------------------------- memory
 void *dev_alloc(size_t bytes); // from the block cache or cudaMalloc, counted; throws on failure
+// Into the block cache (after a device synchronisation) or cudaFree; inside a FreeScope when
+// that ends.
 void dev_free(void *p);
 // While one exists, the device blocks that this thread frees are held back and freed
 // together when the outermost one ends, after one device synchronisation.
@@ -93,7 +95,7 @@ struct FreeScope
     ~FreeScope();
     FreeScope(const FreeScope &) = delete;
     FreeScope &operator=(const FreeScope &) = delete;
-};         // into the block cache (after a device synchronisation) or cudaFree
+};
 void release_cached_device_memory(); // frees the current device's cached blocks
 extern std::atomic<unsigned long long> g_dev_allocs;
 
@@ -319,11 +321,11 @@ struct TuneConfig
     int gmem_threads = 512;
     // refill: weight (terms plus per-row costs) of a row tile, at most TILE_BUDGET, and
     // resident refill CTAs per SM (0: as many as fit)
-    int tile_budget = 0; // 0: TILE_T
+    int tile_budget = 0; // 0: TILE_BUDGET
     int refill_ctas_per_sm = 0;
     // rows with more terms leave the tiles for the larger-row kernels (0: TILE_T);
-    // refill CTA threads: 256, or 128 for plans whose tiles have at most TILE_T
-    // outputs (tile budget and tile_max_terms at most TILE_T / 2)
+    // refill CTA threads: 256, or 128 for plans whose tiles have at most
+    // (TILE_BUDGET + TILE_T) / 2 outputs (tile budget and tile_max_terms at most TILE_T / 2)
     int tile_max_terms = 0;
     int refill_threads = 256;
     // the pipelined refill (tile data staged ahead by asynchronous copies) for plans
