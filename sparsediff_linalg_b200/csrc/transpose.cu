@@ -146,24 +146,36 @@ constexpr int RANK_TILE = 2048, RANK_TILE_SPARSE = 256;
 constexpr int RANK_THREADS = 256;
 
 // First segment that starts in each tile of `tile` keys (nseg past the last), and the
-// segments beyond SEG_SHORT keys, listed per class.
+// segments beyond SEG_SHORT keys, listed per class (one add per warp and class).
 __global__ void k_seg_tiles(const int *__restrict__ off, int nseg, int tile, int ntiles, int *__restrict__ first,
                             int *__restrict__ counts, int *__restrict__ lists)
 {
-    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s <= nseg;
-         s += (long long)gridDim.x * blockDim.x)
+    const int lane = lane_id();
+    for (long long s0 = blockIdx.x * (long long)blockDim.x + threadIdx.x - lane; s0 <= nseg;
+         s0 += (long long)gridDim.x * blockDim.x)
     {
-        const int o = off[s];
-        const int b0 = s ? off[s - 1] / tile + 1 : 0;
-        const int b1 = s < nseg ? o / tile : ntiles;
-        for (int b = b0; b <= b1; ++b) first[b] = (int)s;
-        if (s == nseg) break;
-        const int len = off[s + 1] - o;
-        if (len > SEG_SHORT)
+        const long long s = s0 + lane;
+        int cls = SEG_NCLS;
+        if (s <= nseg)
         {
-            const int c = len <= 1024 ? SEG_W1K : len <= 8192 ? SEG_C8K : SEG_BIG;
+            const int o = off[s];
+            const int b0 = s ? off[s - 1] / tile + 1 : 0;
+            const int b1 = s < nseg ? o / tile : ntiles;
+            for (int b = b0; b <= b1; ++b) first[b] = (int)s;
+            const int len = s < nseg ? off[s + 1] - o : 0;
+            if (len > SEG_SHORT) cls = len <= 1024 ? SEG_W1K : len <= 8192 ? SEG_C8K : SEG_BIG;
+        }
+        if (!__any_sync(FULL_MASK, cls < SEG_NCLS)) continue;
+#pragma unroll
+        for (int c = 0; c < SEG_NCLS; ++c)
+        {
+            const unsigned of = __ballot_sync(FULL_MASK, cls == c);
+            if (!of) continue;
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&counts[c], __popc(of));
+            at = __shfl_sync(FULL_MASK, at, 0) + __popc(of & lanemask_lt());
             // a class's segments are at most nkeys / 65 together: its list starts there
-            lists[c * (long long)(off[nseg] / (SEG_SHORT + 1)) + atomicAdd(&counts[c], 1)] = (int)s;
+            if (cls == c) lists[c * (long long)(off[nseg] / (SEG_SHORT + 1)) + at] = (int)s;
         }
     }
 }
@@ -218,9 +230,12 @@ __global__ void __launch_bounds__(RANK_THREADS) k_seg_rank(const unsigned long l
     }
 }
 
-// <= 1024 keys: one warp per segment, shared-memory bitonic.
+// <= 1024 keys: one warp per segment, shared-memory bitonic. Like the other
+// sorts it writes the two halves of the keys in their order (another kernel that took them from
+// the sorted keys: columns of 66 entries, 30M in all, 3.02 -> 2.42 ms).
 __global__ void k_segsort_w1k(const int *__restrict__ list, int count, const int *__restrict__ off,
-                              unsigned long long *__restrict__ keys)
+                              const unsigned long long *__restrict__ keys, int *__restrict__ lo_out,
+                              int *__restrict__ hi_out)
 {
     extern __shared__ unsigned long long smk[];
     const int lane = lane_id();
@@ -235,14 +250,19 @@ __global__ void k_segsort_w1k(const int *__restrict__ list, int count, const int
         for (int q = lane; q < P; q += 32) buf[q] = q < len ? keys[b + q] : ~0ull;
         __syncwarp();
         warp_bitonic_sort(buf, P);
-        for (int q = lane; q < len; q += 32) keys[b + q] = buf[q];
+        for (int q = lane; q < len; q += 32)
+        {
+            lo_out[b + q] = (int)(buf[q] & 0xffffffffu);
+            hi_out[b + q] = (int)(buf[q] >> 32);
+        }
         __syncwarp();
     }
 }
 
 // <= 8192 keys: one CTA per segment.
 __global__ void k_segsort_c8k(const int *__restrict__ list, int count, const int *__restrict__ off,
-                              unsigned long long *__restrict__ keys)
+                              const unsigned long long *__restrict__ keys, int *__restrict__ lo_out,
+                              int *__restrict__ hi_out)
 {
     extern __shared__ unsigned long long smk[];
     for (int w = blockIdx.x; w < count; w += gridDim.x)
@@ -253,7 +273,11 @@ __global__ void k_segsort_c8k(const int *__restrict__ list, int count, const int
         for (int q = threadIdx.x; q < P; q += blockDim.x) smk[q] = q < len ? keys[b + q] : ~0ull;
         __syncthreads();
         block_bitonic_sort(smk, P);
-        for (int q = threadIdx.x; q < len; q += blockDim.x) keys[b + q] = smk[q];
+        for (int q = threadIdx.x; q < len; q += blockDim.x)
+        {
+            lo_out[b + q] = (int)(smk[q] & 0xffffffffu);
+            hi_out[b + q] = (int)(smk[q] >> 32);
+        }
         __syncthreads();
     }
 }
@@ -261,10 +285,12 @@ __global__ void k_segsort_c8k(const int *__restrict__ list, int count, const int
 constexpr int BIG_CHUNK = 8192;
 
 // Big segments: sort BIG_CHUNK-sized chunks in shared memory, then merge runs
-// pairwise (merge path per thread) between keys and scratch until one run is left.
+// pairwise (merge path per thread) between keys and scratch until one run is left, and write
+// its halves.
 __global__ void k_segsort_big(const int *__restrict__ list, int count, const int *__restrict__ off,
                               unsigned long long *__restrict__ keys,
-                              unsigned long long *__restrict__ scratch)
+                              unsigned long long *__restrict__ scratch, int *__restrict__ lo_out,
+                              int *__restrict__ hi_out)
 {
     extern __shared__ unsigned long long smk[];
     for (int w = blockIdx.x; w < count; w += gridDim.x)
@@ -317,25 +343,13 @@ __global__ void k_segsort_big(const int *__restrict__ list, int count, const int
             __syncthreads();
             in_src = !in_src;
         }
-        if (!in_src)
+        const unsigned long long *sorted = in_src ? src : dst;
+        for (int q = threadIdx.x; q < len; q += blockDim.x)
         {
-            for (int q = threadIdx.x; q < len; q += blockDim.x) src[q] = dst[q];
-            __syncthreads();
+            lo_out[b + q] = (int)(sorted[q] & 0xffffffffu);
+            hi_out[b + q] = (int)(sorted[q] >> 32);
         }
     }
-}
-
-// The two halves of the sorted keys of the listed segments, a CTA per segment.
-__global__ void k_unpack_segs(const int *__restrict__ list, int count, const int *__restrict__ off,
-                              const unsigned long long *__restrict__ keys, int *__restrict__ lo_out,
-                              int *__restrict__ hi_out)
-{
-    for (int w = blockIdx.x; w < count; w += gridDim.x)
-        for (int q = off[list[w]] + threadIdx.x; q < off[list[w] + 1]; q += blockDim.x)
-        {
-            lo_out[q] = (int)(keys[q] & 0xffffffffu);
-            hi_out[q] = (int)(keys[q] >> 32);
-        }
 }
 
 // Sorts every segment [off[s], off[s+1]) of keys ascending (keys unique per segment) and
@@ -362,7 +376,7 @@ void segment_sort(unsigned long long *d_keys, const int *d_off, int nseg, int nk
         int g = std::min((h[SEG_W1K] + 3) / 4, cap);
         size_t sm = 4 * 1024 * sizeof(unsigned long long);
         SDL_CUDA(cudaFuncSetAttribute(k_segsort_w1k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        SDL_LAUNCH(k_segsort_w1k, g, 128, sm, s, lists.get(), h[SEG_W1K], d_off, d_keys);
+        SDL_LAUNCH(k_segsort_w1k, g, 128, sm, s, lists.get(), h[SEG_W1K], d_off, d_keys, lo_out, hi_out);
     }
     if (h[SEG_C8K] || h[SEG_BIG])
     {
@@ -373,21 +387,17 @@ void segment_sort(unsigned long long *d_keys, const int *d_off, int nseg, int nk
         {
             int g = std::min(h[SEG_C8K], cap);
             SDL_LAUNCH(k_segsort_c8k, g, 512, sm, s, lists.get() + SEG_C8K * (size_t)stride, h[SEG_C8K], d_off,
-                       d_keys);
+                       d_keys, lo_out, hi_out);
         }
         if (h[SEG_BIG])
         {
             DevBuf<unsigned long long> scratch(nkeys);
             int g = std::min(h[SEG_BIG], rt.num_sms);
             SDL_LAUNCH(k_segsort_big, g, 1024, sm, s, lists.get() + SEG_BIG * (size_t)stride, h[SEG_BIG], d_off,
-                       d_keys, scratch.get());
+                       d_keys, scratch.get(), lo_out, hi_out);
             SDL_CUDA(cudaStreamSynchronize(s)); // scratch is freed on return
         }
     }
-    for (int c = 0; c < SEG_NCLS; ++c)
-        if (h[c])
-            SDL_LAUNCH(k_unpack_segs, std::min(h[c], cap), 256, 0, s, lists.get() + c * (size_t)stride, h[c], d_off,
-                       d_keys, lo_out, hi_out);
     SDL_CUDA(cudaStreamSynchronize(s)); // the lists are freed on return
 }
 
