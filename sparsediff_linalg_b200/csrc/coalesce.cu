@@ -206,6 +206,30 @@ __global__ void __launch_bounds__(CS_THREADS) k_cs_gaps(const CsGap *__restrict_
     }
 }
 
+// What a one-pass refill of the plan would meet: the most triplets of an output, and how many
+// of the sampled neighbours in sorted order (a tile in CS_SAMPLE) lie more than CS_NEAR
+// triplets apart in the input.
+constexpr int CS_SAMPLE = 16;
+constexpr int CS_NEAR = 32; // 256 bytes of values
+__global__ void __launch_bounds__(CS_THREADS) k_cs_spread(const int *__restrict__ ostart, int nout,
+                                                          const int *__restrict__ perm, int n,
+                                                          int *__restrict__ longest, int *__restrict__ far)
+{
+    int most = 0, f = 0;
+    for (long long o = blockIdx.x * (long long)CS_THREADS + threadIdx.x; o < nout; o += (long long)gridDim.x * CS_THREADS)
+        most = max(most, ostart[o + 1] - ostart[o]);
+    for (long long t = (long long)blockIdx.x * CS_SAMPLE * CS_TILE; t < n; t += (long long)gridDim.x * CS_SAMPLE * CS_TILE)
+        for (long long q = t + threadIdx.x; q < min(t + CS_TILE, (long long)n); q += CS_THREADS)
+            if (q > 0) f += abs(perm[q] - perm[q - 1]) > CS_NEAR;
+    most = __reduce_max_sync(FULL_MASK, most);
+    f = __reduce_add_sync(FULL_MASK, f);
+    if (lane_id() == 0)
+    {
+        atomicMax(longest, most);
+        if (f) atomicAdd(far, f);
+    }
+}
+
 // ------------------------------------------------------------------ bucketed refill
 // For large inputs the one-pass refill gathers every triplet value at random from an
 // array larger than L2, so DRAM moves whole sectors for 8 useful bytes. The bucketed
@@ -473,6 +497,22 @@ void bucket_build(const int *ostart, const int *perm, int n, int nout, CoalesceB
     SDL_LAUNCH(k_cb_order, B.nchunks, CB_CHUNK_THREADS, CB_ORDER_SMEM, s, B.to.get(), n, shift, B.from.get());
 }
 
+// Whether the plan's refill goes through buckets (the rule beside COALESCE_BUCKET_MIN).
+bool takes_buckets(const int *ostart, const int *perm, int n, int nout, cudaStream_t s)
+{
+    if (n < COALESCE_BUCKET_MIN_HEAVY) return false;
+    if (n >= (long long)COALESCE_HEAVY * nout) return true;
+    if (n < COALESCE_BUCKET_MIN) return false;
+    DevBuf<int> stats(2);
+    SDL_CUDA(cudaMemsetAsync(stats.get(), 0, stats.bytes(), s));
+    const int grid = 148 * 8;
+    SDL_LAUNCH(k_cs_spread, grid, CS_THREADS, 0, s, ostart, nout, perm, n, stats.get(), stats.get() + 1);
+    int h[2] = {0, 0}; // longest, far
+    SDL_CUDA(cudaMemcpyAsync(h, stats.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+    SDL_CUDA(cudaStreamSynchronize(s));
+    return h[0] >= COALESCE_HEAVY || h[1] > COALESCE_FAR * (n / CS_SAMPLE);
+}
+
 } // namespace
 
 int coalesce_build(const int *rows, const int *cols, int n, int m, int ncols, DevBuf<int> &Cp, DevBuf<int> &Ci,
@@ -521,8 +561,7 @@ int coalesce_build(const int *rows, const int *cols, int n, int m, int ncols, De
     if (gap_cap)
         SDL_LAUNCH(k_cs_gaps, (unsigned)std::min(gap_cap, 148LL * 8), CS_THREADS, 0, s, gaps.get(), ngaps,
                    Cp.get());
-    if (n >= COALESCE_BUCKET_MIN || (n >= COALESCE_BUCKET_MIN_HEAVY && n >= (long long)COALESCE_HEAVY * nout))
-        bucket_build(ostart.get(), perm.get(), n, nout, buckets, s);
+    if (takes_buckets(ostart.get(), perm.get(), n, nout, s)) bucket_build(ostart.get(), perm.get(), n, nout, buckets, s);
     SDL_CUDA(cudaStreamSynchronize(s));
     return nout;
 }

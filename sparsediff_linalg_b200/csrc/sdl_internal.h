@@ -196,9 +196,17 @@ void gather_values(const int *d_src, const double *d_x, double *d_out, int n,
 // per output or more, whose gathers are chains of that length: 4.3M triplets, 100 per output
 // 129 and 66 us, 1000 per output 1025 and 136 us, 10000 per output 10.1 and 1.5 ms. (At 30
 // per output 68 and 64 us, but the plan takes 72 us longer.)
+// Not where the triplets of neighbouring outputs are neighbours in the input (sorted input,
+// elements assembled along the rows): if at most COALESCE_FAR of the neighbours in sorted
+// order are far apart in the input and no output has COALESCE_HEAVY triplets, one pass reads
+// whole sectors. 30M triplets, one pass against two: sorted 139 and 269 us, 4 x 4 elements
+// along the rows 164 and 286 us, runs of 8 in random order 176 and 263 us, all at random 532
+// and 271 us; 12M: 61 and 128, 76 and 138, 70 and 122, 127 and 128 us. The line is where the
+// two meet at 30M if the time goes with the share of far neighbours.
 constexpr int COALESCE_BUCKET_MIN = 10 << 20;
 constexpr int COALESCE_BUCKET_MIN_HEAVY = 4 << 20;
 constexpr int COALESCE_HEAVY = 96;
+constexpr double COALESCE_FAR = 0.3;
 struct CoalesceBuckets
 {
     int n = 0, nb = 0, nchunks = 0;

@@ -278,6 +278,37 @@ def test_coalesce_buckets_edges_bit_exact(sdl, n, heavy):
         assert np.array_equal(bits(Cx.cpu().numpy()), bits(wx))
 
 
+# inputs of that size whose neighbours in sorted order are neighbours in the input, which are
+# gathered in one pass: sorted, 4 x 4 elements one after the other, sorted with an output of
+# so many triplets (96) that it keeps buckets or one fewer; and shuffled for half of them
+@pytest.mark.parametrize("kind", ["sorted", "elements", "heavy95", "heavy96", "half"])
+def test_coalesce_ordered_input_bit_exact(sdl, kind):
+    import torch
+    from oracle import parallel
+    from sparsediff_linalg_b200.device import Coalesce
+    rng = np.random.default_rng(len(kind))
+    n, m, ncols = MIN + 48, 700000, 700000
+    if kind == "elements":
+        at = rng.integers(0, m - 4, n // 16)[:, None]
+        rows, cols = (at + np.repeat(np.arange(4), 4)).ravel(), (at + np.tile(np.arange(4), 4)).ravel()
+    else:
+        key = np.sort(rng.integers(0, m * ncols, n))
+        if kind.startswith("heavy"):
+            key[5000000:5000000 + int(kind[5:])] = key[5000000]
+        if kind == "half":
+            key[:n // 2] = rng.permutation(key[:n // 2])
+        rows, cols = key // ncols, key % ncols
+    rows, cols = rows.astype(np.int32), cols.astype(np.int32)
+    x = rng.standard_normal(len(rows))
+    x[::3] = -0.0
+    C = Coalesce(T(rows), T(cols), m, ncols)
+    Cx = torch.full((C.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+    C.fill(T(x), Cx)
+    wp, wi, wx = parallel.coalesce(rows, cols, x, m, ncols)[:3]
+    assert np.array_equal(C.Cp.cpu().numpy(), wp) and np.array_equal(C.Ci.cpu().numpy(), wi)
+    assert np.array_equal(bits(Cx.cpu().numpy()), bits(wx))
+
+
 # the same with a factor per triplet: a scaled sum of two sparse operands with MIN entries
 # together, one fewer and one more; each output is (0 + d1 a) + d2 b, one rounding each
 @pytest.mark.parametrize("extra", [-1, 0, 1])
