@@ -2448,6 +2448,26 @@ __global__ void k_win_max(const int *__restrict__ begin, int nwin, int *__restri
     if (lane_id() == 0) atomicMax(out, m);
 }
 
+// Terms of the listed windows' largest outputs, a CTA per window.
+__global__ void __launch_bounds__(WIN_THREADS) k_win_peak(const int *__restrict__ list, const int *__restrict__ begin,
+                                                          const unsigned *__restrict__ keys, int *__restrict__ peak)
+{
+    __shared__ int cnt[1 << WIN_BITS], most;
+    for (int o = threadIdx.x; o < 1 << WIN_BITS; o += WIN_THREADS) cnt[o] = 0;
+    if (threadIdx.x == 0) most = 0;
+    __syncthreads();
+    const int w = list[blockIdx.x];
+    for (int i = begin[w] + threadIdx.x; i < begin[w + 1]; i += WIN_THREADS)
+        atomicAdd(&cnt[keys[i] & ((1 << WIN_BITS) - 1)], 1);
+    __syncthreads();
+    int m = 0;
+    for (int o = threadIdx.x; o < 1 << WIN_BITS; o += WIN_THREADS) m = max(m, cnt[o]);
+    m = __reduce_max_sync(FULL_MASK, m);
+    if (lane_id() == 0) atomicMax(&most, m);
+    __syncthreads();
+    if (threadIdx.x == 0) peak[blockIdx.x] = most;
+}
+
 // Part `part` of a window (WIN_TERMS terms from part * WIN_TERMS on): where its outputs'
 // entries of win_start begin, and the descriptor of the next part (0: none).
 struct WinPart
@@ -2779,9 +2799,25 @@ int bits_for(long long v) // of the values 0 .. v - 1
     return b;
 }
 
-// Windows of the rows B (false: there are too many).
-bool build_windows(Product &P, const BigRows &B, const NumArgs &na, cudaStream_t s)
+// Windows of the rows B; row i's have about WIN_TARGET >> narrow[i] terms. Where columns crowd
+// (banded rows: the outputs near the middle have most of the terms), narrower windows are
+// better than windows in parts, a second of which has few terms and as many outputs. If such
+// windows hold over a sixteenth of the terms, `narrow` is set, once, and the windows are to be
+// built again -- for all rows: the largest window sets the shared memory of every CTA, and so
+// what is left for L1 (197 us instead of 158 with the other rows' windows as they were). 3000 rows of 10000 terms over 394 outputs 164 us in parts, 125
+// us narrower (build 2.3 and 3.0 ms), of 12000 terms over 2200 outputs 204 and 150 us. A
+// window whose largest output has a sixteenth of its terms or more is no reason: with columns
+// by Zipf's law 324 and 290 us were not worth the build (2.0 and 3.0 ms).
+enum class Windows
 {
+    BUILT,
+    AGAIN,
+    TOO_MANY
+};
+Windows build_windows(Product &P, const BigRows &B, std::vector<int> &narrow, const NumArgs &na, cudaStream_t s)
+{
+    const bool first_try = narrow.empty();
+    if (first_try) narrow.assign(B.n(), 0);
     Runtime &rt = runtime();
     const int nb = B.n();
     std::vector<int2> wins(nb);
@@ -2789,11 +2825,11 @@ bool build_windows(Product &P, const BigRows &B, const NumArgs &na, cudaStream_t
     long long starts = 0, nwin = 0;
     for (int i = 0; i < nb; ++i)
     {
-        const long long want = (long long)WIN_TARGET * B.outs[i] / std::max(1LL, B.terms[i]);
+        const long long want = (long long)(WIN_TARGET >> narrow[i]) * B.outs[i] / std::max(1LL, B.terms[i]);
         const int width = (int)std::max(1LL, std::min<long long>(want, 1 << WIN_BITS));
         wins[i] = make_int2((int)nwin, width);
         const long long k = (B.outs[i] + width - 1) / width;
-        if (nwin + k >= 1LL << (32 - WIN_BITS)) return false;
+        if (nwin + k >= 1LL << (32 - WIN_BITS)) return Windows::TOO_MANY;
         nwin += k;
         for (long long q = 0; q < k; ++q)
         {
@@ -2801,7 +2837,7 @@ bool build_windows(Product &P, const BigRows &B, const NumArgs &na, cudaStream_t
             starts += std::min<long long>(width, B.outs[i] - q * width) + 1;
         }
     }
-    if (starts > INT_MAX) return false;
+    if (starts > INT_MAX) return Windows::TOO_MANY;
     const int T = (int)B.T, W = (int)nwin;
     const DevBuf<int> rows = to_device(B.rows, s), dwout = to_device(wout, s);
     const DevBuf<int2> dwins = to_device(wins, s);
@@ -2838,6 +2874,32 @@ bool build_windows(Product &P, const BigRows &B, const NumArgs &na, cudaStream_t
         const auto size = [&](int w) { return hb[w + 1] - hb[w]; };
         for (int w = 0; w < W; ++w)
             if (size(w) > WIN_TERMS) chained.push_back(w);
+        if (first_try)
+        {
+            const DevBuf<int> list = to_device(chained, s);
+            DevBuf<int> dpeak(chained.size());
+            SDL_LAUNCH(k_win_peak, (unsigned)chained.size(), WIN_THREADS, 0, s, list.get(), begin.get(), keys.get(),
+                       dpeak.get());
+            std::vector<int> peak(chained.size());
+            SDL_CUDA(cudaMemcpyAsync(peak.data(), dpeak.get(), dpeak.bytes(), cudaMemcpyDeviceToHost, s));
+            SDL_CUDA(cudaStreamSynchronize(s));
+            long long crowded = 0;
+            int row = 0; // (the windows are in the rows' order)
+            for (size_t c = 0; c < chained.size(); ++c)
+            {
+                const int w = chained[c];
+                while (row + 1 < nb && wins[row + 1].x <= w) ++row;
+                if (16LL * peak[c] > size(w)) continue;
+                crowded += size(w);
+                narrow[row] = std::max(narrow[row], size(w) > 3 * WIN_TERMS / 2 ? 2 : 1);
+            }
+            if (16 * crowded > T)
+            {
+                for (int &h : narrow) h = std::max(h, 1);
+                P.win_pairs.release();
+                return Windows::AGAIN;
+            }
+        }
         std::stable_sort(chained.begin(), chained.end(), [&](int x, int y) { return size(x) > size(y); });
         for (int w : chained) parts.push_back(WinPart{w, 0, wout[w], 0});
         for (int w = 0; w < W; ++w)
@@ -2850,7 +2912,7 @@ bool build_windows(Product &P, const BigRows &B, const NumArgs &na, cudaStream_t
             size_t last = c;
             for (int part = 1; (long long)part * WIN_TERMS < size(w); ++part)
             {
-                if (starts + entries > INT_MAX) return false;
+                if (starts + entries > INT_MAX) return Windows::TOO_MANY;
                 parts[last].next = (int)parts.size();
                 last = parts.size();
                 parts.push_back(WinPart{w, part, (int)starts, 0});
@@ -2870,7 +2932,7 @@ bool build_windows(Product &P, const BigRows &B, const NumArgs &na, cudaStream_t
     if (take_device_error(s)) fail(SDL_ERR_INTERNAL, "product plan: heavy-row windows are inconsistent");
     P.nwin = W;
     P.win_most = most;
-    return true;
+    return Windows::BUILT;
 }
 
 // Output-major term lists of the rows B (a stable sort by output, k_big_starts).
@@ -2928,7 +2990,10 @@ void build_big_rows(Product &P, const long long *ub, const NumArgs &na, cudaStre
         (ht[i] <= WIN_MULT * ho[i] ? W : L).add(hr[i], ht[i], ho[i]);
     }
     if (T >= INT_MAX || O >= INT_MAX || T < O) return; // the CTA kernels handle them
-    if (W.n() && !build_windows(P, W, na, s))
+    std::vector<int> narrow;
+    Windows built = W.n() ? build_windows(P, W, narrow, na, s) : Windows::BUILT;
+    if (built == Windows::AGAIN) built = build_windows(P, W, narrow, na, s);
+    if (built != Windows::BUILT)
         for (int i = 0; i < W.n(); ++i) L.add(W.rows[i], W.terms[i], W.outs[i]);
     if (L.n()) build_lists(P, L, na, s);
     SDL_CUDA(cudaStreamSynchronize(s));

@@ -279,7 +279,7 @@ def test_coalesce_buckets_edges_bit_exact(sdl, n, heavy):
 
 
 # inputs of that size whose neighbours in sorted order are neighbours in the input, which are
-# gathered in one pass: sorted, 4 x 4 elements one after the other, sorted with an output of
+# gathered in one pass: sorted, 4 x 4 elements along the rows, sorted with an output of
 # so many triplets (96) that it keeps buckets or one fewer; and shuffled for half of them
 @pytest.mark.parametrize("kind", ["sorted", "elements", "heavy95", "heavy96", "half"])
 def test_coalesce_ordered_input_bit_exact(sdl, kind):
@@ -289,7 +289,7 @@ def test_coalesce_ordered_input_bit_exact(sdl, kind):
     rng = np.random.default_rng(len(kind))
     n, m, ncols = MIN + 48, 700000, 700000
     if kind == "elements":
-        at = rng.integers(0, m - 4, n // 16)[:, None]
+        at = np.sort(rng.integers(0, m - 4, n // 16))[:, None]
         rows, cols = (at + np.repeat(np.arange(4), 4)).ravel(), (at + np.tile(np.arange(4), 4)).ravel()
     else:
         key = np.sort(rng.integers(0, m * ncols, n))
@@ -497,6 +497,37 @@ def test_large_row_many_terms_bit_exact(sdl, orc, n, hot):
         torch.cuda.synchronize()
         for o in out:
             assert np.array_equal(bits(o.cpu().numpy()), bits(wx))
+
+
+# banded rows, whose middle outputs have most of the terms, so that windows are built again
+# narrower (half, a quarter); alone, and beside a row with an output of 6000 terms, whose
+# window stays one in parts
+@pytest.mark.parametrize("per_l,per_a,step,hot", [(100, 100, 3, False), (200, 100, 9, False), (100, 100, 3, True),
+                                                  (60, 60, 1, True)])
+def test_large_row_banded_windows_bit_exact(sdl, orc, per_l, per_a, step, hot):
+    import torch
+    from sparsediff_linalg_b200.device import Product
+    rng = np.random.default_rng(per_l + hot)
+    nL, nA = 60, 7000
+    n = nA * step + per_a * step + 1
+    base = np.arange(nA)[:, None] * step + rng.integers(0, 2, (nA, 1))
+    rows = base + step * np.arange(per_a)[None]
+    if hot:
+        rows[:, 0] = 0
+    Bp, Bi = (np.arange(nA + 1) * per_a).astype(np.int32), rows.astype(np.int32).ravel()
+    ent = [at + np.arange(per_l) for at in np.linspace(10, nA - per_l, nL).astype(int)]
+    if hot:
+        ent[7] = np.arange(500, 6500)
+    Ap = np.concatenate([[0], np.cumsum([len(e) for e in ent])]).astype(np.int32)
+    Ai = np.concatenate(ent).astype(np.int32)
+    Ax, Bx = rng.standard_normal(len(Ai)), rng.standard_normal(len(Bi))
+    Ax[::3] = -0.0
+    P = Product(T(Ap), T(Ai), T(Bp), T(Bi), n)
+    C = torch.full((P.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+    P.fill(T(Ax), None, T(Bx), C)
+    wp, wi, wx = orc.spgemm((Ap, Ai, Ax, nL, nA), (Bp, Bi, Bx, nA, n))
+    assert np.array_equal(P.Cp.cpu().numpy(), wp) and np.array_equal(P.Ci.cpu().numpy(), wi)
+    assert np.array_equal(bits(C.cpu().numpy()), bits(wx))
 
 
 # ---------------------------------------------------------------- symbolic warp sorts
