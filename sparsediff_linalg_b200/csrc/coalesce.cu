@@ -206,27 +206,43 @@ __global__ void __launch_bounds__(CS_THREADS) k_cs_gaps(const CsGap *__restrict_
     }
 }
 
-// What a one-pass refill of the plan would meet: the most triplets of an output, and how many
-// of the sampled neighbours in sorted order (a tile in CS_SAMPLE) lie more than CS_NEAR
-// triplets apart in the input.
+// What a one-pass refill of the plan would meet: the most triplets of an output, and the
+// 128-byte lines of values that the CS_TILE neighbours of a tile in sorted order read, summed
+// over one tile in CS_SAMPLE. (Per 32 neighbours the lines of interleaved sorted streams, six
+// sorted matrices to be added up, count several times.)
 constexpr int CS_SAMPLE = 16;
-constexpr int CS_NEAR = 32; // 256 bytes of values
 __global__ void __launch_bounds__(CS_THREADS) k_cs_spread(const int *__restrict__ ostart, int nout,
                                                           const int *__restrict__ perm, int n,
-                                                          int *__restrict__ longest, int *__restrict__ far)
+                                                          int *__restrict__ longest, int *__restrict__ lines)
 {
-    int most = 0, f = 0;
+    static_assert(2 * CS_TILE == 1 << 12, "the places that the top 12 bits of a hash name");
+    __shared__ int seen[2 * CS_TILE];
+    int most = 0, mlines = 0;
     for (long long o = blockIdx.x * (long long)CS_THREADS + threadIdx.x; o < nout; o += (long long)gridDim.x * CS_THREADS)
         most = max(most, ostart[o + 1] - ostart[o]);
     for (long long t = (long long)blockIdx.x * CS_SAMPLE * CS_TILE; t < n; t += (long long)gridDim.x * CS_SAMPLE * CS_TILE)
-        for (long long q = t + threadIdx.x; q < min(t + CS_TILE, (long long)n); q += CS_THREADS)
-            if (q > 0) f += abs(perm[q] - perm[q - 1]) > CS_NEAR;
+    {
+        __syncthreads();
+        for (int k = threadIdx.x; k < 2 * CS_TILE; k += CS_THREADS) seen[k] = -1;
+        __syncthreads();
+        for (int i = threadIdx.x; i < CS_TILE && t + i < n; i += CS_THREADS)
+        {
+            const int line = perm[t + i] >> 4;
+            // (the table has twice as many places as there are lines, so a probe ends)
+            for (unsigned h = (unsigned)line * 2654435761u;; h += 1u << 20)
+            {
+                const int old = atomicCAS(&seen[h >> 20], -1, line);
+                mlines += old == -1;
+                if (old == -1 || old == line) break;
+            }
+        }
+    }
     most = __reduce_max_sync(FULL_MASK, most);
-    f = __reduce_add_sync(FULL_MASK, f);
+    mlines = __reduce_add_sync(FULL_MASK, mlines);
     if (lane_id() == 0)
     {
         atomicMax(longest, most);
-        if (f) atomicAdd(far, f);
+        if (mlines) atomicAdd(lines, mlines);
     }
 }
 
@@ -507,10 +523,10 @@ bool takes_buckets(const int *ostart, const int *perm, int n, int nout, cudaStre
     SDL_CUDA(cudaMemsetAsync(stats.get(), 0, stats.bytes(), s));
     const int grid = 148 * 8;
     SDL_LAUNCH(k_cs_spread, grid, CS_THREADS, 0, s, ostart, nout, perm, n, stats.get(), stats.get() + 1);
-    int h[2] = {0, 0}; // longest, far
+    int h[2] = {0, 0}; // longest, lines
     SDL_CUDA(cudaMemcpyAsync(h, stats.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
     SDL_CUDA(cudaStreamSynchronize(s));
-    return h[0] >= COALESCE_HEAVY || h[1] > COALESCE_FAR * (n / CS_SAMPLE);
+    return h[0] >= COALESCE_HEAVY || h[1] > coalesce_lines(n) * (n / CS_SAMPLE);
 }
 
 } // namespace

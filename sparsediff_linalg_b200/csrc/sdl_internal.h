@@ -197,16 +197,17 @@ void gather_values(const int *d_src, const double *d_x, double *d_out, int n,
 // 129 and 66 us, 1000 per output 1025 and 136 us, 10000 per output 10.1 and 1.5 ms. (At 30
 // per output 68 and 64 us, but the plan takes 72 us longer.)
 // Not where the triplets of neighbouring outputs are neighbours in the input (sorted input,
-// elements assembled along the rows): if at most COALESCE_FAR of the neighbours in sorted
-// order are far apart in the input and no output has COALESCE_HEAVY triplets, one pass reads
-// whole sectors. 30M triplets, one pass against two: sorted 139 and 269 us, 4 x 4 elements
-// along the rows 164 and 286 us, runs of 8 in random order 176 and 263 us, all at random 532
-// and 271 us; 12M: 61 and 128, 76 and 138, 70 and 122, 127 and 128 us. The line is where the
-// two meet at 30M if the time goes with the share of far neighbours.
+// sums of sorted matrices, elements one after the other): if neighbours in sorted order read
+// at most coalesce_lines(n) 128-byte lines per value and no output has COALESCE_HEAVY
+// triplets, one pass takes less. One pass against two, by runs in random order (1 / lines per
+// value): 12M triplets, sorted 61 and 130 us, runs of 8 70 and 122, of 4 82 and 122, of 2 100
+// and 126, all at random 127 and 128 us; 30M: 139 and 269, 176 and 263, 242 and 265, 346 and
+// 271, 532 and 271 us; 48M: 225 and 421, 293 and 409, 430 and 413, 625 and 425, 993 and 425
+// us. The line goes through where the two meet at 30M and 48M.
 constexpr int COALESCE_BUCKET_MIN = 10 << 20;
 constexpr int COALESCE_BUCKET_MIN_HEAVY = 4 << 20;
 constexpr int COALESCE_HEAVY = 96;
-constexpr double COALESCE_FAR = 0.3;
+constexpr double coalesce_lines(int n) { return 0.13 + 5e6 / n; }
 struct CoalesceBuckets
 {
     int n = 0, nb = 0, nchunks = 0;
