@@ -310,9 +310,10 @@ def test_coalesce_ordered_input_bit_exact(sdl, kind):
 
 
 # the same with a factor per triplet: a scaled sum of two sparse operands with MIN entries
-# together, one fewer and one more; each output is (0 + d1 a) + d2 b, one rounding each
-@pytest.mark.parametrize("extra", [-1, 0, 1])
-def test_scaled_sum_through_buckets_bit_exact(sdl, extra):
+# together, one fewer and one more; each output is (0 + d1 a) + d2 b, one rounding each. Few
+# long rows in random order, since rows in order are gathered in one pass (the last case)
+@pytest.mark.parametrize("extra,shuffled", [(-1, True), (0, True), (1, True), (1, False)])
+def test_scaled_sum_through_buckets_bit_exact(sdl, extra, shuffled):
     from sparsediff_linalg_b200 import matrices as M
     from test_gpu_dense_ops import Lib, csr_of
     from test_gpu_sums import SIGS
@@ -321,9 +322,10 @@ def test_scaled_sum_through_buckets_bit_exact(sdl, extra):
         getattr(L, name).restype, getattr(L, name).argtypes = res, args
     lib = Lib(L)
     rng = np.random.default_rng(900 + extra)
-    m, n = 2900, 4000
+    m, n = 16, 725000
     nnz = [MIN // 2, MIN // 2 + extra]
-    cells = [np.sort(rng.permutation(m * n)[:k]) for k in nnz]
+    cells = [rng.permutation(m * n)[:k] for k in nnz]
+    cells = [c[np.argsort(c // n, kind="stable")] if shuffled else np.sort(c) for c in cells]
     vals = [rng.standard_normal(k) for k in nnz]
     vals[0][::5] = -0.0
     d = [rng.uniform(-2, 2, m) for _ in range(2)]
